@@ -1,0 +1,59 @@
+// The persistent group kernels of batched sweeps: one per (kind, system),
+// instantiated by batch.cu (LLE maps), batch_bif.cu and batch_basins.cu.
+#pragma once
+
+#include "../../include/chaos_gb300.h"
+#include "batch.h"
+#include "engine.cuh"
+
+namespace chaos {
+
+constexpr int kBatchBlock = 128;
+
+using GroupKernel = void (*)(const JobDesc*, const Chunk*, int, int*);
+GroupKernel bif_group_kernel(int system);
+GroupKernel basins_group_kernel(int system);
+
+template <int S> struct FieldOf;
+template <> struct FieldOf<SYS_LORENZ_RK4> { using F = Lorenz; };
+template <> struct FieldOf<SYS_ROSSLER_RK4> { using F = Rossler; };
+template <> struct FieldOf<SYS_CHEN_RK4> { using F = Chen; };
+
+// Persistent kernel of one (kind, system) group: pulls chunks [0, count) of
+// the group's range from its counter until none is left. One kernel per
+// group keeps each code path's register allocation as small as the
+// single-sweep kernel's (a kernel that switched over every kind and system
+// would be sized for the largest of them).
+template <template <int> class Work, int S>
+__global__ void __launch_bounds__(kBatchBlock) group_kernel(const JobDesc* __restrict__ jobs,
+                                                            const Chunk* __restrict__ chunks, int count,
+                                                            int* counter) {
+    __shared__ int slot;
+    for (;;) {
+        if (threadIdx.x == 0) slot = atomicAdd(counter, 1);
+        __syncthreads();
+        const int c = slot;
+        __syncthreads();
+        if (c >= count) return;
+        const Chunk ch = chunks[c];
+        const JobDesc& J = jobs[ch.job];
+        Work<S>::run(J, ch.begin, ch.count);
+    }
+}
+
+// The group kernel of a work that every built-in system has.
+template <template <int> class Work> GroupKernel group_kernel_of(int system) {
+    switch (system) {
+        case SYS_LORENZ_RK4: return group_kernel<Work, SYS_LORENZ_RK4>;
+        case SYS_ROSSLER_RK4: return group_kernel<Work, SYS_ROSSLER_RK4>;
+        case SYS_CHEN_RK4: return group_kernel<Work, SYS_CHEN_RK4>;
+        case SYS_CHAMELEON: return group_kernel<Work, SYS_CHAMELEON>;
+        case SYS_ROSSLER_CD: return group_kernel<Work, SYS_ROSSLER_CD>;
+        case SYS_SIN3: return group_kernel<Work, SYS_SIN3>;
+        case SYS_SIN2: return group_kernel<Work, SYS_SIN2>;
+        case SYS_MEMRISTOR: return group_kernel<Work, SYS_MEMRISTOR>;
+        default: return nullptr;
+    }
+}
+
+}  // namespace chaos

@@ -13,6 +13,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "launch.h"
 #include "order_keys.h"
 #include "peaks.h"
@@ -79,9 +81,12 @@ template <> __device__ __forceinline__ bool basins_diverged<double>(double v, co
     if (b > 0x7fefffffffffffffull) return true;  // NaN or +-inf
     return P.checkMax && max_exceeded(b, P);
 }
+// As one compare: a limit that is negative or below the largest float decides
+// alone, a NaN limit (never exceeded) leaves the largest float.
 template <> __device__ __forceinline__ bool basins_diverged<float>(float v, const SweepParams& P) {
-    const float av = fabsf(v);
-    return !(av <= 3.4028234663852886e38f) || (P.checkMax && av > P.maxValueF);
+    constexpr float kMax = 3.4028234663852886e38f;
+    const float lim = P.checkMax ? fminf(P.maxValueF, kMax) : kMax;
+    return !(fabsf(v) <= lim);
 }
 
 // The sample tests and the streaming peak detector (PeakStream) live in
@@ -95,6 +100,37 @@ template <int NX, class T> __device__ __forceinline__ T pick(const T* x, int wv)
     for (int j = 1; j < NX; ++j)
         if (j == wv) v = x[j];
     return v;
+}
+
+// The recorded component of a sweep: known at compile time (W >= 0), or at run
+// time. The FP32 sweeps of the RK4 systems and of Chameleon run their loops
+// with the component known: picking it costs two selects a sample and
+// trajectory otherwise, which the packed loops' ALU pipe feels (700,001
+// Rossler points 18.6 -> 17.7 ms, 1,000 Lorenz points 0.90 -> 0.84 ms).
+template <int W> struct Component {
+    static constexpr int kIndex = W;
+    int wv;
+    template <int NX, class T> __device__ __forceinline__ T of(const T* x) const {
+        if constexpr (W >= 0) return x[W < NX ? W : 0];
+        else return pick<NX>(x, wv);
+    }
+};
+template <int S, class T> struct KnownComponent {
+    static constexpr bool value = std::is_same<T, float>::value && (S <= SYS_CHEN_RK4 || S == SYS_CHAMELEON);
+};
+// f(component) for the component wv of a sweep: one copy of f per component of
+// a system with KnownComponent (three components), else one for all. The
+// single-sweep kernels choose on the host, a kernel per component (three
+// copies in one kernel share its registers and its schedule: 1,000 Lorenz
+// points took 1.17 ms in that form), a batch's kernels on the device, chunk by chunk.
+template <bool Known, class Fn> __host__ __device__ __forceinline__ void with_component(int wv, Fn&& f) {
+    if constexpr (Known) {
+        if (wv == 0) f(Component<0>{0});
+        else if (wv == 1) f(Component<1>{1});
+        else f(Component<2>{2});
+    } else {
+        f(Component<-1>{wv});
+    }
 }
 
 // Loads state and parameters of point p of a sweep (mutated parameters or
@@ -139,99 +175,216 @@ template <int NX, class T> __device__ __forceinline__ bool basins_fixed(const T*
     return sqrt(fabs((double)s)) < 1e-9;
 }
 
-// Samples per block of the recorded loops' block form: the steps of a block
-// run back to back, then the gate judges its samples together.
-constexpr int kRecordBlock = 4;
 // Steps per block of the bifurcation transients' block form.
 constexpr int kTransientBlock = 8;
 
-// The block form runs for the float detector (the branching form behind its
-// gate) on the built-in systems; a user system keeps the one-step loop (its
-// equations are not stepped past a divergence).
-template <int S, class T, bool Sel> struct RecordBlocks {
-    static constexpr bool value = PeakStream<T, Sel>::Gate && S != SYS_USER;
+// The FP32 recorded loops judge their samples in windows (PeakWindow,
+// peaks.h). A thread runs L trajectories (1, or 2 in packed lanes); what it
+// needs once a window lives in shared memory, so that the step loop keeps its
+// registers: the samples of the window and the two before it, the detectors
+// and a basins point's sums. A thread's samples are one column whose length
+// is odd in units of a bank row's step (L words), so a warp's stores of one
+// sample are free of bank conflicts.
+// 32 samples a window for one trajectory, 24 for two: the longer, the rarer
+// the judging (700,001 Rossler points 18.3 ms with 16 in two lanes, 18.1 with
+// 24), but 24 already leave room for only six blocks of 128 threads per SM.
+template <int L> struct Window {
+    static constexpr int K = L == 1 ? 32 : 24;  // samples
+    static constexpr int kColumn = (K + 3) * L;  // floats of a thread's column: 2 + K samples, 1 unused
+    static constexpr size_t kDetectors = sizeof(int4) * L, kSums = sizeof(float4) * L;
+    static constexpr size_t bytes(int block) { return (kDetectors + kSums + kColumn * sizeof(float)) * block; }
+
+    int4* det;     // [L][blockDim.x]
+    float4* sum;   // [L][blockDim.x]
+    float* col;    // this thread's column
+    __device__ __forceinline__ Window() {
+        extern __shared__ int4 window_smem[];
+        det = window_smem + threadIdx.x;
+        sum = reinterpret_cast<float4*>(window_smem + L * blockDim.x) + threadIdx.x;
+        col = reinterpret_cast<float*>(window_smem + 2 * L * blockDim.x) + kColumn * threadIdx.x;
+    }
+    __device__ __forceinline__ float& at(int l, int j) const { return col[(j + 2) * L + l]; }  // -2 <= j < K
+    __device__ __forceinline__ void put(int j, float v) const { col[j + 2] = v; }
+    __device__ __forceinline__ void put(int j, float2 v) const { reinterpret_cast<float2*>(col)[j + 2] = v; }
+    __device__ __forceinline__ PeakWindow detector(int l) const {
+        const int4 d = det[l * blockDim.x];
+        return PeakWindow{d.x, d.y, d.z, d.w};
+    }
+    __device__ __forceinline__ void keep(int l, const PeakWindow& d) const {
+        det[l * blockDim.x] = make_int4(d.nc, d.i0, d.n, d.tprev);
+    }
+
+    // Judges the candidates of one window that starts at sample index k: the
+    // lanes' candidates one after the other in one loop, so that a warp goes
+    // round as often as its busiest thread has candidates. open: bit l set
+    // while lane l's detector is on a plateau. on_peak(l, detector, val, t)
+    // sees the detector before the peak is counted.
+    template <class OnPeak>
+    __device__ __forceinline__ void judge(int k, unsigned c0, unsigned c1, int m0, int m1, unsigned& open,
+                                          OnPeak&& on_peak) const {
+        auto run = [&](int l, int j, int m) {  // j < 0: a plateau from the window before
+            PeakWindow d = detector(l);
+            auto a = [&](int i) { return at(l, i); };
+            auto peak = [&](float val, int t) {
+                on_peak(l, d, val, t);
+                d.tprev = t;
+                ++d.n;
+            };
+            if (j < 0) d.walk(k, 0, m, a, peak);
+            else d.judge(k, j, m, a, peak);
+            open = (open & ~(1u << l)) | (d.i0 >= 0 ? 1u << l : 0u);
+            keep(l, d);
+        };
+        if (open != 0u) {
+            if (open & 1u) run(0, -1, m0);
+            if (L == 2 && (open & 2u)) run(1, -1, m1);
+        }
+        while ((c0 | c1) != 0u) {
+            const int l = L == 2 && c0 == 0u ? 1 : 0, m = l ? m1 : m0;
+            unsigned c = l ? c1 : c0;
+            const int j = PeakWindow::next(c, m);
+            if (l) c1 = c;
+            else c0 = c;
+            run(l, j, m);
+        }
+    }
 };
+
+// The recorded loop of one FP32 trajectory: B samples x[wv], one before each
+// advance(); diverged(v) ends the point (returned as 0, otherwise 1); xp
+// receives the state before the last advance of a point that did not diverge,
+// last the last sample and n the detected peaks. on_peak(l, detector, val, t)
+// for every detected peak, in order.
+//
+// What bounds it is issue slots (large sweeps) or one warp's chain (small
+// ones), so a sample costs two compares, a predicated bit and a shared store
+// beside its step, and the peak rules run once a window for the whole warp.
+// Judging blocks of 4 samples instead (a gate of two compares and two selects
+// a sample) sent nearly every block of a chaotic sweep through the
+// transitions sample by sample, since one of 32 orbits always had a peak in
+// it. Measured against that, 20,000 steps: 1,000 Lorenz points (then with the
+// detector as selects) 1.83 -> 0.88 ms, 700,001 Rossler points 19.9 -> 18.1 ms;
+// 1024^2 Lorenz basins 37.4 -> 33.9 ms.
+template <int NX, int W, class Advance, class Diverged, class OnPeak>
+__device__ __forceinline__ int record_windows(int B, float* x, float* xp, Component<W> wc, const Window<1>& w, float& last,
+                                              int& n, Advance&& advance, Diverged&& diverged, OnPeak&& on_peak) {
+    constexpr int K = Window<1>::K;
+    PeakWindow d;
+    d.init();
+    w.keep(0, d);
+    w.put(-2, 0.f);
+    w.put(-1, 0.f);
+    float v = wc.template of<NX>(x), p = 0.f;  // the recorded sample, carried from one step to the next
+    unsigned up = 0, open = 0;
+    int i = 0;
+    bool dv = false;
+    for (; i + K < B; i += K) {
+        unsigned mask = 0;
+#pragma unroll 1
+        for (int q = 0; q < K; q += 4) {
+            mask <<= 4;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                if (v > p) mask |= 8u >> r;
+                p = v;
+                w.put(q + r, v);
+                advance();
+                v = wc.template of<NX>(x);
+                dv |= diverged(v);
+            }
+        }
+        int m = K;
+        if (__builtin_expect(dv, 0)) {  // the samples up to the one before the divergent one count
+            for (m = 1; m < K && !diverged(w.at(0, m));) ++m;
+            mask >>= K - m;
+            p = w.at(0, m - 1);
+        }
+        const unsigned cand = PeakWindow::candidates(mask, up, m);
+        if ((cand | open) != 0u) w.judge(i, cand, 0u, m, 0, open, on_peak);
+        if (dv) break;
+        up = mask & 1u;
+        w.put(-2, w.at(0, K - 2));
+        w.put(-1, p);
+    }
+    if (!dv) {
+        unsigned mask = 0;
+        int m = 0;
+        for (; i + m < B && !dv;) {
+#pragma unroll
+            for (int j = 0; j < NX; ++j) xp[j] = x[j];
+            mask = (mask << 1) | (v > p ? 1u : 0u);
+            p = v;
+            w.put(m++, v);
+            advance();
+            v = wc.template of<NX>(x);
+            dv = diverged(v);
+        }
+        if (m > 0) {
+            const unsigned cand = PeakWindow::candidates(mask, up, m);
+            if ((cand | open) != 0u) w.judge(i, cand, 0u, m, 0, open, on_peak);
+        }
+    }
+    last = p;
+    n = w.detector(0).n;
+    return dv ? 0 : 1;
+}
 
 // The recorded part of a bifurcation point, from its state x after a
 // transient that ended bounded and not fixed: nB samples through the
 // streaming peak detector (intervals in units hI), divergence and fixed-point
 // tests; writes flags/counts/first and the first `cap` kept peaks/intervals
-// of row o.
-//
-// Block form: kRecordBlock steps without a branch, their divergence tests
-// or-ed together, then the samples through PeakStream::push_block. A block in
-// which the orbit diverged pushes its samples up to the divergent one, as the
-// one-step loop does, and ends the loop (the steps after the divergent one
-// change nothing that is reported). The last step, whose starting state the
-// fixed-point test keeps, always runs in the one-step loop.
-template <int S, class T, bool Sel = false>
+// of row o. FP32 judges windows of samples (record_windows; the steps a
+// window runs past a divergent one change nothing that is reported; the
+// launch brings Window<1>::bytes of shared memory), FP64 one sample at a time.
+template <int S, class T, int W>
 __device__ __forceinline__ void bif_record(const SweepParams& P, const BifOut& O, T* x, const T* a,
-                                           const StepCtx<T>& c, int nB, double hI, long long o) {
+                                           const StepCtx<T>& c, int nB, double hI, long long o, Component<W> wc) {
     constexpr int NX = Traits<S>::NX;
     T xp[NX];
-    const int wv = P.wv;
     int flag = 1;
-    PeakStream<T, Sel> ps;
-    ps.init();
-    const double first = (double)pick<NX>(x, wv);
+    int n = 0;  // detected peaks
+    const double first = (double)wc.template of<NX>(x);
     double* pk = O.peaks ? O.peaks + o * (long long)O.cap : nullptr;
     double* iv = O.intervals ? O.intervals + o * (long long)O.cap : nullptr;
-    auto on_peak = [&](T val, int t) {
-        if (ps.n >= 1) {
-            const int q = ps.n - 1;
+    auto write_peak = [&](int found, int tprev, T val, int t) {
+        if (found >= 1) {
+            const int q = found - 1;
             if (q < O.cap) {
                 if (pk) pk[q] = (double)val;
-                if (iv) iv[q] = __dmul_rn((double)(t - ps.tprev), hI);
+                if (iv) iv[q] = __dmul_rn((double)(t - tprev), hI);
             }
         }
-        ps.tprev = t;
-        ++ps.n;
     };
-    T v = pick<NX>(x, wv);  // the recorded sample, carried from one step to the next
 #pragma unroll
     for (int j = 0; j < NX; ++j) xp[j] = x[j];
-    int i = 0;
-    if constexpr (RecordBlocks<S, T, Sel>::value) {
-        constexpr int K = kRecordBlock;
-        for (; i + K < nB; i += K) {
-            T s[K + 1];
-            s[0] = v;
-            bool dv = false;
-#pragma unroll
-            for (int j = 1; j <= K; ++j) {
-                step<S>(x, a, c);
-                s[j] = pick<NX>(x, wv);
-                dv |= bif_diverged(s[j], P);
-            }
-            if (__builtin_expect(!dv, 1)) {
-                ps.template push_block<K>(s, on_peak);
-                v = s[K];
-                continue;
-            }
-#pragma unroll
-            for (int j = 0; j < K; ++j) {
-                T val;
-                int t;
-                if (ps.push(s[j], val, t)) on_peak(val, t);
-                if (bif_diverged(s[j + 1], P)) break;
-            }
-            flag = 0;
-            break;
-        }
-    }
-    if (flag == 1)
-        for (; i < nB; ++i) {
+    if constexpr (std::is_same<T, float>::value) {
+        float last;
+        flag = record_windows<NX>(
+            nB, x, xp, wc, Window<1>(), last, n, [&] { step<S>(x, a, c); },
+            [&](float v) { return bif_diverged(v, P); },
+            [&](int, const PeakWindow& d, float val, int t) { write_peak(d.n, d.tprev, val, t); });
+    } else {
+        PeakStream<T> ps;
+        ps.init();
+        T v = wc.template of<NX>(x);  // the recorded sample, carried from one step to the next
+        for (int i = 0; i < nB; ++i) {
 #pragma unroll
             for (int j = 0; j < NX; ++j) xp[j] = x[j];
             T val;
             int t;
-            if (ps.push(v, val, t)) on_peak(val, t);
+            if (ps.push(v, val, t)) {
+                write_peak(ps.n, ps.tprev, val, t);
+                ps.tprev = t;
+                ++ps.n;
+            }
             step<S>(x, a, c);
-            v = pick<NX>(x, wv);
+            v = wc.template of<NX>(x);
             if (bif_diverged(v, P)) { flag = 0; break; }
         }
+        n = ps.n;
+    }
     if (flag == 1 && nB > 0 && bif_fixed<NX>(x, xp)) flag = -1;
-    const int kept = ps.n > 1 ? ps.n - 1 : 0;
+    const int kept = n > 1 ? n - 1 : 0;
     O.flags[o] = flag;
     O.counts[o] = flag == 1 ? kept : (flag == -1 ? -1 : 0);
     if (O.first) O.first[o] = first;
@@ -241,8 +394,9 @@ __device__ __forceinline__ void bif_record(const SweepParams& P, const BifOut& O
 // Bifurcation point (reference kernels calculateTransTimeCUDA +
 // calculateDiscreteModelCUDA + peakFinderCUDA, bifurcationCUDA.cu:258-371),
 // fused. Writes flags/counts/first and the first `cap` kept peaks/intervals.
-template <int S, class T, bool Sel = false>
-__device__ __forceinline__ void bif_point(const SweepParams& P, const BifOut& O, long long p, long long o) {
+template <int S, class T, int W>
+__device__ __forceinline__ void bif_point(const SweepParams& P, const BifOut& O, long long p, long long o,
+                                             Component<W> wc) {
     constexpr int NX = Traits<S>::NX, NA = Traits<S>::NA;
     T x[NX], a[NA], xp[NX];
     load_point<S, T>(P, p, x, a);
@@ -255,25 +409,24 @@ __device__ __forceinline__ void bif_point(const SweepParams& P, const BifOut& O,
         hI = __dmul_rn(hp, (double)P.bPre);
     }
     const StepCtx<T> c((T)hp);
-    const int wv = P.wv;
     int flag = 1;
     if (nS > 0) {
         // the state before the last step is kept for the fixed-point test:
         // the last step is peeled off the loop, so the others copy nothing
         int s = 0;
-        if constexpr (S != SYS_USER && !Sel) {
+        if constexpr (S != SYS_USER) {
             // blocks of kTransientBlock steps, one divergence branch a block:
             // a point's flags do not depend on the step at which it diverged
-            // (the steps after it on an unbounded state report nothing). The
-            // select form (small sweeps, one latency-bound orbit a warp)
-            // keeps the one-step loop and its registers.
+            // (the steps after it on an unbounded state report nothing).
+            // Lorenz in FP32, one warp per scheduler: 69 cycles a step
+            // against 91 with a branch after every step.
             constexpr int K = kTransientBlock;
             for (; s + K <= nS - 1; s += K) {
                 bool dv = false;
 #pragma unroll
                 for (int j = 0; j < K; ++j) {
                     step<S>(x, a, c);
-                    dv |= bif_diverged(pick<NX>(x, wv), P);
+                    dv |= bif_diverged(wc.template of<NX>(x), P);
                 }
                 if (dv) { flag = 0; break; }
             }
@@ -281,18 +434,18 @@ __device__ __forceinline__ void bif_point(const SweepParams& P, const BifOut& O,
         if (flag == 1)
             for (; s < nS - 1; ++s) {
                 step<S>(x, a, c);
-                if (bif_diverged(pick<NX>(x, wv), P)) { flag = 0; break; }
+                if (bif_diverged(wc.template of<NX>(x), P)) { flag = 0; break; }
             }
         if (flag == 1) {
 #pragma unroll
             for (int j = 0; j < NX; ++j) xp[j] = x[j];
             step<S>(x, a, c);
-            if (bif_diverged(pick<NX>(x, wv), P)) flag = 0;
+            if (bif_diverged(wc.template of<NX>(x), P)) flag = 0;
             else if (bif_fixed<NX>(x, xp)) flag = -1;
         }
     }
     if (flag == 1) {
-        bif_record<S, T, Sel>(P, O, x, a, c, nB, hI, o);
+        bif_record<S, T>(P, O, x, a, c, nB, hI, o, wc);
     } else {  // a transient that ended diverged or fixed is reported as diverged
         O.flags[o] = 0;
         O.counts[o] = 0;
@@ -412,13 +565,26 @@ template <> struct PeakSums<double> {
 template <> struct PeakSums<float> {
     float hi = 0.f, lo = 0.f;
     int span = 0;
-    __device__ __forceinline__ void add(float val, int dt, double) {
+    __device__ __forceinline__ void add(float val, int dt) {
         const float s = hi + val;  // TwoSum(hi, val) = s + err exactly
         const float bv = s - hi;
         const float err = (hi - (s - bv)) + (val - bv);
         hi = s;
         lo = lo + err;
         span += dt;
+    }
+    __device__ __forceinline__ void store(float4* to) const { *to = make_float4(hi, lo, __int_as_float(span), 0.f); }
+    __device__ __forceinline__ void load(const float4* from) {
+        const float4 v = *from;
+        hi = v.x;
+        lo = v.y;
+        span = __float_as_int(v.z);
+    }
+    static __device__ __forceinline__ void add_stored(float4* at, float val, int dt) {
+        PeakSums s;
+        s.load(at);
+        s.add(val, dt);
+        s.store(at);
     }
     __device__ __forceinline__ double peaks() const { return (double)hi + (double)lo; }
     __device__ __forceinline__ double intervals(double hI) const { return __dmul_rn((double)span, hI); }
@@ -430,75 +596,54 @@ template <> struct PeakSums<float> {
 // sweep has preScaller == 1 (one step per sample, no inner loop).
 // The recorded part of a basins point, from its state x after the transient:
 // peak detector, divergence and fixed-point tests, features into row o.
-template <int S, class T, bool PRE1, bool Sel = false>
+template <int S, class T, bool PRE1, int W>
 __device__ __forceinline__ void basins_record(const SweepParams& P, const BasinsOut& O, T* x, const T* a,
-                                              const StepCtx<T>& c, long long o) {
+                                              const StepCtx<T>& c, long long o, Component<W> wc) {
     constexpr int NX = Traits<S>::NX;
     T xp[NX];
-    const int wv = P.wv;
 #pragma unroll
     for (int j = 0; j < NX; ++j) xp[j] = x[j];
-    PeakStream<T, Sel> ps;
-    ps.init();
-    int flag = 1;
+    int flag = 1, n = 0;  // n: detected peaks
     PeakSums<T> sums;
     T lastT = T(0);  // widened once after the loop (a per-step FP64 convert costs FP64-pipe time)
-    auto on_peak = [&](T val, int t) {
-        if (ps.n >= 1) sums.add(val, t - ps.tprev, P.hInterval);
-        ps.tprev = t;
-        ++ps.n;
+    auto advance = [&] {
+        if (PRE1) step<S>(x, a, c);
+        else
+            for (int r = 0; r < P.preScaller; ++r) step<S>(x, a, c);
     };
-    T v = pick<NX>(x, wv);  // the recorded sample, carried from one step to the next
-    int i = 0;
-    if constexpr (RecordBlocks<S, T, Sel>::value) {  // the block form of bif_record
-        constexpr int K = kRecordBlock;
-        for (; i + K < P.B; i += K) {
-            T s[K + 1];
-            s[0] = v;
-            bool dv = false;
-#pragma unroll
-            for (int j = 1; j <= K; ++j) {
-                if (PRE1) step<S>(x, a, c);
-                else
-                    for (int r = 0; r < P.preScaller; ++r) step<S>(x, a, c);
-                s[j] = pick<NX>(x, wv);
-                dv |= basins_diverged(s[j], P);
-            }
-            if (__builtin_expect(!dv, 1)) {
-                ps.template push_block<K>(s, on_peak);
-                lastT = s[K - 1];
-                v = s[K];
-                continue;
-            }
-#pragma unroll
-            for (int j = 0; j < K; ++j) {
-                lastT = s[j];
-                T val;
-                int t;
-                if (ps.push(s[j], val, t)) on_peak(val, t);
-                if (basins_diverged(s[j + 1], P)) break;
-            }
-            flag = 0;
-            break;
-        }
-    }
-    if (flag == 1)
-        for (; i < P.B; ++i) {
+    if constexpr (std::is_same<T, float>::value) {  // as bif_record; the sums in shared memory
+        const Window<1> w;
+        sums.store(w.sum);
+        flag = record_windows<NX>(
+            P.B, x, xp, wc, w, lastT, n, advance, [&](float v) { return basins_diverged(v, P); },
+            [&](int, const PeakWindow& d, float val, int t) {
+                if (d.n >= 1) PeakSums<float>::add_stored(w.sum, val, t - d.tprev);
+            });
+        sums.load(w.sum);
+    } else {
+        PeakStream<T> ps;
+        ps.init();
+        T v = wc.template of<NX>(x);  // the recorded sample, carried from one step to the next
+        for (int i = 0; i < P.B; ++i) {
 #pragma unroll
             for (int j = 0; j < NX; ++j) xp[j] = x[j];
             lastT = v;
             T val;
             int t;
-            if (ps.push(v, val, t)) on_peak(val, t);
-            if (PRE1) step<S>(x, a, c);
-            else
-                for (int r = 0; r < P.preScaller; ++r) step<S>(x, a, c);
-            v = pick<NX>(x, wv);
+            if (ps.push(v, val, t)) {
+                if (ps.n >= 1) sums.add(val, t - ps.tprev, P.hInterval);
+                ps.tprev = t;
+                ++ps.n;
+            }
+            advance();
+            v = wc.template of<NX>(x);
             if (basins_diverged(v, P)) { flag = 0; break; }
         }
+        n = ps.n;
+    }
     if (flag == 1 && P.B > 0 && basins_fixed<NX>(x, xp)) flag = -1;
     const double last = (double)lastT;
-    const int kept = ps.n > 1 ? ps.n - 1 : 0;
+    const int kept = n > 1 ? n - 1 : 0;
     double ap, ai;
     if (flag == 0) { ap = 999.0; ai = 999.0; }
     else if (flag == -1) { ap = last; ai = -1.0; }
@@ -516,14 +661,15 @@ __device__ __forceinline__ void basins_record(const SweepParams& P, const Basins
     }
 }
 
-template <int S, class T, bool PRE1 = false, bool Sel = false>
-__device__ __forceinline__ void basins_point(const SweepParams& P, const BasinsOut& O, long long p, long long o) {
+template <int S, class T, bool PRE1, int W>
+__device__ __forceinline__ void basins_point(const SweepParams& P, const BasinsOut& O, long long p, long long o,
+                                             Component<W> wc) {
     constexpr int NX = Traits<S>::NX, NA = Traits<S>::NA;
     T x[NX], a[NA];
     load_point<S, T>(P, p, x, a);
     const StepCtx<T> c((T)P.h);
     for (int s = 0; s < P.S; ++s) step<S>(x, a, c);
-    basins_record<S, T, PRE1, Sel>(P, O, x, a, c, o);
+    basins_record<S, T, PRE1>(P, O, x, a, c, o, wc);
 }
 
 // ---------------------------------------------------------------------------
@@ -971,14 +1117,6 @@ __device__ __forceinline__ void lle_pair_twin(const LleParams& L, long long p, l
 // ends when neither lane is recording.
 __device__ __forceinline__ float lane(const P2& v, int l) { return l ? v.v.y : v.v.x; }
 
-template <int NX> __device__ __forceinline__ P2 pick2(const P2* x, int wv) {
-    P2 v = x[0];
-#pragma unroll
-    for (int j = 1; j < NX; ++j)
-        if (j == wv) v = x[j];
-    return v;
-}
-
 // sqrtf(fabsf(sum (x - xp)^2)) < 1e-9 per lane, as bif_fixed<NX, float>
 template <int NX> __device__ __forceinline__ bool bif_fixed_lane(const P2* x, const P2* xp, int l) {
     float s = 0.f;
@@ -1015,10 +1153,10 @@ __device__ __forceinline__ void load_pair(const SweepParams& P, long long p0, lo
 // step peeled off for the fixed-point test; flag[l] (1 on entry for a lane in
 // use, 0 otherwise) ends 1, 0 (diverged) or -1 (fixed), as bif_point's.
 // Blocks of kTransientBlock steps with one test a block, as in bif_point.
-template <class F>
-__device__ __forceinline__ void bif_pair_transient(const SweepParams& P, P2* x, const P2* a, int* flag) {
+template <class F, int W>
+__device__ __forceinline__ void bif_pair_transient(const SweepParams& P, P2* x, const P2* a, int* flag,
+                                                   Component<W> wc) {
     P2 xp[3];
-    const int wv = P.wv;
     if (P.S > 0) {
         const RK4H<P2> c((float)P.h);
         int s = 0;
@@ -1029,7 +1167,7 @@ __device__ __forceinline__ void bif_pair_transient(const SweepParams& P, P2* x, 
 #pragma unroll
                 for (int j = 0; j < K; ++j) {
                     rk4_step<F>(x, a, c);
-                    const P2 v = pick2<3>(x, wv);
+                    const P2 v = wc.template of<3>(x);
                     d0 |= bif_diverged(v.v.x, P);
                     d1 |= bif_diverged(v.v.y, P);
                 }
@@ -1041,7 +1179,7 @@ __device__ __forceinline__ void bif_pair_transient(const SweepParams& P, P2* x, 
         if (flag[0] == 1 || flag[1] == 1)
             for (; s < P.S - 1; ++s) {  // the last step peeled off, as in bif_point
                 rk4_step<F>(x, a, c);
-                const P2 v = pick2<3>(x, wv);
+                const P2 v = wc.template of<3>(x);
                 if (flag[0] == 1 && bif_diverged(v.v.x, P)) flag[0] = 0;
                 if (flag[1] == 1 && bif_diverged(v.v.y, P)) flag[1] = 0;
                 if (flag[0] != 1 && flag[1] != 1) break;
@@ -1050,7 +1188,7 @@ __device__ __forceinline__ void bif_pair_transient(const SweepParams& P, P2* x, 
 #pragma unroll
             for (int j = 0; j < 3; ++j) xp[j] = x[j];
             rk4_step<F>(x, a, c);
-            const P2 v = pick2<3>(x, wv);
+            const P2 v = wc.template of<3>(x);
             if (flag[0] == 1 && bif_diverged(v.v.x, P)) flag[0] = 0;
             if (flag[1] == 1 && bif_diverged(v.v.y, P)) flag[1] = 0;
 #pragma unroll
@@ -1060,202 +1198,188 @@ __device__ __forceinline__ void bif_pair_transient(const SweepParams& P, P2* x, 
     }
 }
 
-template <class F>
+// The recorded loop of two trajectories in packed lanes, per lane exactly
+// record_windows: rec[l] says whether lane l records, flag[l] becomes 0 when
+// it diverges (the pair goes on while the other lane records), xp the state
+// before the last advance (of a lane that did not diverge).
+template <int W, class Advance, class Diverged, class OnPeak>
+__device__ __forceinline__ void record_pair_windows(int B, P2* x, P2* xp, Component<W> wc, const Window<2>& w, bool* rec,
+                                                    int* flag, float* last, Advance&& advance, Diverged&& diverged,
+                                                    OnPeak&& on_peak) {
+    constexpr int K = Window<2>::K;
+    PeakWindow d;
+    d.init();
+    w.keep(0, d);
+    w.keep(1, d);
+    w.put(-2, make_float2(0.f, 0.f));
+    w.put(-1, make_float2(0.f, 0.f));
+    P2 v = wc.template of<3>(x), p(0.0);
+    unsigned up0 = 0, up1 = 0, open = 0;
+    int i = 0;
+    for (; i + K < B; i += K) {
+        unsigned mask0 = 0, mask1 = 0;
+        bool dv0 = false, dv1 = false;
+#pragma unroll 1
+        for (int q = 0; q < K; q += 4) {
+            mask0 <<= 4;
+            mask1 <<= 4;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                if (v.v.x > p.v.x) mask0 |= 8u >> r;
+                if (v.v.y > p.v.y) mask1 |= 8u >> r;
+                p = v;
+                w.put(q + r, v.v);
+                advance();
+                v = wc.template of<3>(x);
+                dv0 |= diverged(v.v.x);
+                dv1 |= diverged(v.v.y);
+            }
+        }
+        int m0 = K, m1 = K;
+        if (__builtin_expect(rec[0] && dv0, 0)) {
+            for (m0 = 1; m0 < K && !diverged(w.at(0, m0));) ++m0;
+            mask0 >>= K - m0;
+        }
+        if (__builtin_expect(rec[1] && dv1, 0)) {
+            for (m1 = 1; m1 < K && !diverged(w.at(1, m1));) ++m1;
+            mask1 >>= K - m1;
+        }
+        const unsigned c0 = rec[0] ? PeakWindow::candidates(mask0, up0, m0) : 0u;
+        const unsigned c1 = rec[1] ? PeakWindow::candidates(mask1, up1, m1) : 0u;
+        if ((c0 | c1 | open) != 0u) w.judge(i, c0, c1, m0, m1, open, on_peak);
+        if (rec[0]) last[0] = w.at(0, m0 - 1);
+        if (rec[1]) last[1] = w.at(1, m1 - 1);
+        if (rec[0] && dv0) {
+            rec[0] = false;
+            flag[0] = 0;
+            open &= ~1u;
+        }
+        if (rec[1] && dv1) {
+            rec[1] = false;
+            flag[1] = 0;
+            open &= ~2u;
+        }
+        if (!rec[0] && !rec[1]) return;
+        up0 = mask0 & 1u;
+        up1 = mask1 & 1u;
+        w.put(-2, make_float2(w.at(0, K - 2), w.at(1, K - 2)));
+        w.put(-1, p.v);
+    }
+    unsigned mask0 = 0, mask1 = 0;
+    int m0 = 0, m1 = 0, m = 0;  // samples each lane judges, and those of the tail
+    for (; i + m < B && (rec[0] || rec[1]);) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) xp[j] = x[j];
+        if (rec[0]) {
+            mask0 = (mask0 << 1) | (v.v.x > p.v.x ? 1u : 0u);
+            ++m0;
+            last[0] = v.v.x;
+        }
+        if (rec[1]) {
+            mask1 = (mask1 << 1) | (v.v.y > p.v.y ? 1u : 0u);
+            ++m1;
+            last[1] = v.v.y;
+        }
+        p = v;
+        w.put(m++, v.v);
+        advance();
+        v = wc.template of<3>(x);
+        if (rec[0] && diverged(v.v.x)) { rec[0] = false; flag[0] = 0; }
+        if (rec[1] && diverged(v.v.y)) { rec[1] = false; flag[1] = 0; }
+    }
+    const unsigned c0 = m0 > 0 ? PeakWindow::candidates(mask0, up0, m0) : 0u;
+    const unsigned c1 = m1 > 0 ? PeakWindow::candidates(mask1, up1, m1) : 0u;
+    if ((c0 | c1 | open) != 0u) w.judge(i, c0, c1, m0, m1, open, on_peak);
+}
+
+template <class F, int W>
 __device__ __forceinline__ void bif_pair_point(const SweepParams& P, const BifOut& O, long long p0, long long p1,
-                                               long long o0, long long o1, bool two) {
+                                                  long long o0, long long o1, bool two, Component<W> wc) {
     P2 x[3], a[3], xp[3];
     load_pair<F>(P, p0, p1, x, a);
     const RK4H<P2> c((float)P.h);
-    const int wv = P.wv;
     int flag[2] = {1, two ? 1 : 0};
-    bif_pair_transient<F>(P, x, a, flag);
+    bif_pair_transient<F>(P, x, a, flag, wc);
     bool rec[2];
     double first[2] = {0.0, 0.0};  // stays 0 for a lane that does not record (as the scalar path)
-    PeakStream<float> ps[2];
+    int n[2] = {0, 0};  // detected peaks
 #pragma unroll
     for (int l = 0; l < 2; ++l) {
         rec[l] = flag[l] == 1;
         if (!rec[l]) flag[l] = 0;
-        ps[l].init();
     }
     const long long oo[2] = {o0, o1};
     if (rec[0] || rec[1]) {
         {
-            const P2 v = pick2<3>(x, wv);
+            const P2 v = wc.template of<3>(x);
             if (rec[0]) first[0] = (double)v.v.x;
             if (rec[1]) first[1] = (double)v.v.y;
         }
-        P2 v = pick2<3>(x, wv);  // carried from one step to the next
-        auto on_peak = [&](int l, float val, int t) {
-            if (ps[l].n >= 1) {
-                const int q = ps[l].n - 1;
-                if (q < O.cap) {
-                    if (O.peaks) O.peaks[oo[l] * O.cap + q] = (double)val;
-                    if (O.intervals)
-                        O.intervals[oo[l] * O.cap + q] = __dmul_rn((double)(t - ps[l].tprev), P.hInterval);
-                }
-            }
-            ps[l].tprev = t;
-            ++ps[l].n;
-        };
-        int i = 0;
-        {  // the block form of bif_record, per lane (a lane that stopped skips its detector)
-            constexpr int K = kRecordBlock;
-            for (; i + K < P.B; i += K) {
-                float s[2][K + 1];
-                s[0][0] = v.v.x;
-                s[1][0] = v.v.y;
-                bool dv[2] = {false, false};
-#pragma unroll
-                for (int j = 1; j <= K; ++j) {
-                    rk4_step<F>(x, a, c);
-                    const P2 w = pick2<3>(x, wv);
-                    s[0][j] = w.v.x;
-                    s[1][j] = w.v.y;
-                    dv[0] |= bif_diverged(w.v.x, P);
-                    dv[1] |= bif_diverged(w.v.y, P);
-                }
-#pragma unroll
-                for (int l = 0; l < 2; ++l) {
-                    if (!rec[l]) continue;
-                    if (__builtin_expect(!dv[l], 1)) {
-                        ps[l].template push_block<K>(s[l], [&](float val, int t) { on_peak(l, val, t); });
-                        continue;
-                    }
-#pragma unroll
-                    for (int j = 0; j < K; ++j) {
-                        float val;
-                        int t;
-                        if (ps[l].push(s[l][j], val, t)) on_peak(l, val, t);
-                        if (bif_diverged(s[l][j + 1], P)) break;
-                    }
-                    rec[l] = false;
-                    flag[l] = 0;
-                }
-                v = P2(s[0][K], s[1][K]);
-                if (!rec[0] && !rec[1]) break;
-            }
-        }
-        for (; i < P.B && (rec[0] || rec[1]); ++i) {
-#pragma unroll
-            for (int j = 0; j < 3; ++j) xp[j] = x[j];
-#pragma unroll
-            for (int l = 0; l < 2; ++l) {
-                float val;
-                int t;
-                const bool hit = ps[l].push(lane(v, l), val, t);  // a lane that stopped keeps stepping its detector
-                if (rec[l] && hit) on_peak(l, val, t);
-            }
-            rk4_step<F>(x, a, c);
-            v = pick2<3>(x, wv);
-            if (rec[0] && bif_diverged(v.v.x, P)) { rec[0] = false; flag[0] = 0; }
-            if (rec[1] && bif_diverged(v.v.y, P)) { rec[1] = false; flag[1] = 0; }
-            if (!rec[0] && !rec[1]) break;
-        }
+        const Window<2> w;
+        float last[2];
+        record_pair_windows(P.B, x, xp, wc, w, rec, flag, last, [&] { rk4_step<F>(x, a, c); },
+                            [&](float v) { return bif_diverged(v, P); },
+                            [&](int l, const PeakWindow& d, float val, int t) {
+                                const int q = d.n - 1;
+                                if (q >= 0 && q < O.cap) {
+                                    const long long at = (l ? o1 : o0) * O.cap + q;
+                                    if (O.peaks) O.peaks[at] = (double)val;
+                                    if (O.intervals) O.intervals[at] = __dmul_rn((double)(t - d.tprev), P.hInterval);
+                                }
+                            });
+        n[0] = w.detector(0).n;
+        n[1] = w.detector(1).n;
 #pragma unroll
         for (int l = 0; l < 2; ++l)
             if (rec[l] && P.B > 0 && bif_fixed_lane<3>(x, xp, l)) flag[l] = -1;
     }
 #pragma unroll
     for (int l = 0; l < (two ? 2 : 1); ++l) {
-        const int kept = ps[l].n > 1 ? ps[l].n - 1 : 0;
+        const int kept = n[l] > 1 ? n[l] - 1 : 0;
         O.flags[oo[l]] = flag[l];
         O.counts[oo[l]] = flag[l] == 1 ? kept : (flag[l] == -1 ? -1 : 0);
         if (O.first) O.first[oo[l]] = first[l];
     }
 }
 
-template <class F, bool PRE1 = false>
+template <class F, bool PRE1, int W>
 __device__ __forceinline__ void basins_pair_point(const SweepParams& P, const BasinsOut& O, long long p0,
-                                                  long long p1, long long o0, long long o1, bool two) {
+                                                     long long p1, long long o0, long long o1, bool two,
+                                                     Component<W> wc) {
     P2 x[3], a[3], xp[3];
     load_pair<F>(P, p0, p1, x, a);
     const RK4H<P2> c((float)P.h);
-    const int wv = P.wv;
     for (int s = 0; s < P.S; ++s) rk4_step<F>(x, a, c);
 #pragma unroll
     for (int j = 0; j < 3; ++j) xp[j] = x[j];
-    PeakStream<float> ps[2];
     int flag[2] = {1, two ? 1 : 0};
     bool rec[2] = {true, two};
     PeakSums<float> sums[2];
     float lastF[2] = {0.f, 0.f};  // widened after the loop
-    ps[0].init();
-    ps[1].init();
-    P2 v = pick2<3>(x, wv);  // carried from one step to the next
-    auto on_peak = [&](int l, float val, int t) {
-        if (ps[l].n >= 1) sums[l].add(val, t - ps[l].tprev, P.hInterval);
-        ps[l].tprev = t;
-        ++ps[l].n;
-    };
-    int i = 0;
-    {  // the block form of basins_record, per lane
-        constexpr int K = kRecordBlock;
-        for (; i + K < P.B; i += K) {
-            float s[2][K + 1];
-            s[0][0] = v.v.x;
-            s[1][0] = v.v.y;
-            bool dv[2] = {false, false};
-#pragma unroll
-            for (int j = 1; j <= K; ++j) {
-                if (PRE1) rk4_step<F>(x, a, c);
-                else
-                    for (int r = 0; r < P.preScaller; ++r) rk4_step<F>(x, a, c);
-                const P2 w = pick2<3>(x, wv);
-                s[0][j] = w.v.x;
-                s[1][j] = w.v.y;
-                dv[0] |= basins_diverged(w.v.x, P);
-                dv[1] |= basins_diverged(w.v.y, P);
-            }
-#pragma unroll
-            for (int l = 0; l < 2; ++l) {
-                if (!rec[l]) continue;
-                if (__builtin_expect(!dv[l], 1)) {
-                    ps[l].template push_block<K>(s[l], [&](float val, int t) { on_peak(l, val, t); });
-                    lastF[l] = s[l][K - 1];
-                    continue;
-                }
-#pragma unroll
-                for (int j = 0; j < K; ++j) {
-                    lastF[l] = s[l][j];
-                    float val;
-                    int t;
-                    if (ps[l].push(s[l][j], val, t)) on_peak(l, val, t);
-                    if (basins_diverged(s[l][j + 1], P)) break;
-                }
-                rec[l] = false;
-                flag[l] = 0;
-            }
-            v = P2(s[0][K], s[1][K]);
-            if (!rec[0] && !rec[1]) break;
-        }
-    }
-    for (; i < P.B && (rec[0] || rec[1]); ++i) {
-#pragma unroll
-        for (int j = 0; j < 3; ++j) xp[j] = x[j];
-#pragma unroll
-        for (int l = 0; l < 2; ++l) {
-            if (!rec[l]) continue;
-            lastF[l] = lane(v, l);
-            float val;
-            int t;
-            if (ps[l].push(lane(v, l), val, t)) on_peak(l, val, t);
-        }
-        if (PRE1) rk4_step<F>(x, a, c);
-        else
-            for (int r = 0; r < P.preScaller; ++r) rk4_step<F>(x, a, c);
-        v = pick2<3>(x, wv);
-        if (rec[0] && basins_diverged(v.v.x, P)) { rec[0] = false; flag[0] = 0; }
-        if (rec[1] && basins_diverged(v.v.y, P)) { rec[1] = false; flag[1] = 0; }
-        if (!rec[0] && !rec[1]) break;
-    }
+    const Window<2> w;
+    sums[0].store(w.sum);
+    sums[1].store(w.sum + blockDim.x);
+    record_pair_windows(
+        P.B, x, xp, wc, w, rec, flag, lastF,
+        [&] {
+            if (PRE1) rk4_step<F>(x, a, c);
+            else
+                for (int r = 0; r < P.preScaller; ++r) rk4_step<F>(x, a, c);
+        },
+        [&](float v) { return basins_diverged(v, P); },
+        [&](int l, const PeakWindow& d, float val, int t) {
+            if (d.n >= 1) PeakSums<float>::add_stored(w.sum + l * blockDim.x, val, t - d.tprev);
+        });
+    const int n[2] = {w.detector(0).n, w.detector(1).n};
+    sums[0].load(w.sum);
+    sums[1].load(w.sum + blockDim.x);
     const long long oo[2] = {o0, o1};
     FeatureKeys fk;
 #pragma unroll
     for (int l = 0; l < (two ? 2 : 1); ++l) {
         if (rec[l] && P.B > 0 && basins_fixed_lane<3>(x, xp, l)) flag[l] = -1;
         const double last = (double)lastF[l];
-        const int kept = ps[l].n > 1 ? ps[l].n - 1 : 0;
+        const int kept = n[l] > 1 ? n[l] - 1 : 0;
         double ap, ai;
         if (flag[l] == 0) { ap = 999.0; ai = 999.0; }
         else if (flag[l] == -1) { ap = last; ai = -1.0; }
@@ -1269,68 +1393,6 @@ __device__ __forceinline__ void basins_pair_point(const SweepParams& P, const Ba
         fk.add(flag[l], flag[l] == 1 ? kept : 0, ap, ai, last);
     }
     if (O.mm) fk.flush(O.mm);
-}
-
-// Two basins points per thread, hybrid: the transient (no tests, 80 % of the
-// steps of a typical map) runs packed, two trajectories per FP32x2
-// instruction; the recorded part then runs lane by lane with the scalar loop,
-// whose per-sample peak detector and divergence test a packed loop would have
-// to run for both lanes anyway. Bit-identical to basins_point.
-template <class F> struct SysOf;
-template <> struct SysOf<Lorenz> { static constexpr int S = SYS_LORENZ_RK4; };
-template <> struct SysOf<Rossler> { static constexpr int S = SYS_ROSSLER_RK4; };
-template <> struct SysOf<Chen> { static constexpr int S = SYS_CHEN_RK4; };
-
-template <class F, bool PRE1 = false>
-__device__ __forceinline__ void basins_hybrid_point(const SweepParams& P, const BasinsOut& O, long long p0,
-                                                    long long p1, long long o0, long long o1, bool two) {
-    P2 x[3], a[3];
-    load_pair<F>(P, p0, p1, x, a);
-    {
-        const RK4H<P2> c((float)P.h);
-        for (int s = 0; s < P.S; ++s) rk4_step<F>(x, a, c);
-    }
-    const StepCtx<float> cs((float)P.h);
-#pragma unroll 1
-    for (int l = 0; l < (two ? 2 : 1); ++l) {
-        float xs[3], as[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            xs[k] = lane(x[k], l);
-            as[k] = lane(a[k], l);
-        }
-        basins_record<SysOf<F>::S, float, PRE1>(P, O, xs, as, cs, l ? o1 : o0);
-    }
-}
-
-// Two bifurcation points per thread, hybrid: the transient packed (per-lane
-// divergence and fixed-point tests, as bif_pair_point), the recorded part lane
-// by lane with the scalar loop (bif_record). Bit-identical to bif_point.
-template <class F>
-__device__ __forceinline__ void bif_hybrid_point(const SweepParams& P, const BifOut& O, long long p0, long long p1,
-                                                 long long o0, long long o1, bool two) {
-    P2 x[3], a[3];
-    load_pair<F>(P, p0, p1, x, a);
-    int flag[2] = {1, two ? 1 : 0};
-    bif_pair_transient<F>(P, x, a, flag);
-    const StepCtx<float> cs((float)P.h);
-#pragma unroll 1
-    for (int l = 0; l < (two ? 2 : 1); ++l) {
-        const long long o = l ? o1 : o0;
-        if (flag[l] != 1) {  // diverged or fixed in the transient: reported as diverged
-            O.flags[o] = 0;
-            O.counts[o] = 0;
-            if (O.first) O.first[o] = 0.0;
-            continue;
-        }
-        float xs[3], as[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            xs[k] = lane(x[k], l);
-            as[k] = lane(a[k], l);
-        }
-        bif_record<SysOf<F>::S, float>(P, O, xs, as, cs, P.B, P.hInterval, o);
-    }
 }
 
 // ---------------------------------------------------------------------------

@@ -7,34 +7,27 @@
 #include <cstdlib>
 
 #include "engine.cuh"
+#include "sweep_launch.h"
 
 namespace chaos {
 
 namespace {
-constexpr int kBlock = 128;     // default block
-constexpr int kMaxBlock = 256;  // largest block a tuned launch may use
+constexpr int kBlock = kSweepBlock;
 
-// Sel: the peak detector as selects (sweeps of at most 8 warps per SM, where
-// each warp waits on its own trajectory) or in the block form.
-template <int S, bool Sel>
+// The sweep kernels take Window<trajectories per thread>::bytes(block)
+// of dynamic shared memory.
+template <int S, int W>
 __global__ void __launch_bounds__(kMaxBlock) bif_kernel_f32(SweepParams P, BifOut O) {
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= P.nPoints) return;
-    bif_point<S, float, Sel>(P, O, P.pBegin + o, o);
+    bif_point<S, float>(P, O, P.pBegin + o, o, Component<W>{P.wv});
 }
 
 template <int S>
 __global__ void __launch_bounds__(kBlock) bif_list_kernel_f32(SweepParams P, BifOut O, const int* list, int count) {
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
-    bif_point<S, float, true>(P, O, list[k], k);
-}
-
-template <int S, bool PRE1, bool Sel>
-__global__ void __launch_bounds__(kMaxBlock) basins_kernel_f32(SweepParams P, BasinsOut O) {
-    const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= P.nPoints) return;
-    basins_point<S, float, PRE1, Sel>(P, O, P.pBegin + o, o);
+    bif_point<S, float>(P, O, list[k], k, Component<-1>{P.wv});
 }
 
 // MINB = resident blocks per SM the register allocation is shaped for:
@@ -74,37 +67,16 @@ __global__ void __launch_bounds__(kBlock) spectrum_kernel_f32(LleParams L, doubl
     spectrum_point_twin<F>(L, L.pBegin + o, out);
 }
 
-// Bifurcation / basins, two points per thread in packed FP32x2 lanes (RK4 systems).
-template <class F>
-__global__ void __launch_bounds__(kMaxBlock) bif_pair_kernel_f32(SweepParams P, BifOut O) {
+// Bifurcation / basins, two points per thread in packed FP32x2 lanes (RK4
+// systems). Bound by the FMA pipe; registers capped at 64 (four blocks of 256,
+// eight of 128 per SM), where the step loop still spills nothing: 1024^2
+// Lorenz basins 34.3 -> 34.1 ms against the 77 it takes unbounded.
+template <class F, int W>
+__global__ void __launch_bounds__(kMaxBlock, 4) bif_pair_kernel_f32(SweepParams P, BifOut O) {
     const long long o = 2 * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
     if (o >= P.nPoints) return;
     const bool two = o + 1 < P.nPoints;
-    bif_pair_point<F>(P, O, P.pBegin + o, P.pBegin + (two ? o + 1 : o), o, two ? o + 1 : o, two);
-}
-
-template <class F, bool PRE1>
-__global__ void __launch_bounds__(kMaxBlock) basins_pair_kernel_f32(SweepParams P, BasinsOut O) {
-    const long long o = 2 * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
-    if (o >= P.nPoints) return;
-    const bool two = o + 1 < P.nPoints;
-    basins_pair_point<F, PRE1>(P, O, P.pBegin + o, P.pBegin + (two ? o + 1 : o), o, two ? o + 1 : o, two);
-}
-
-template <class F>
-__global__ void __launch_bounds__(kMaxBlock) bif_hybrid_kernel_f32(SweepParams P, BifOut O) {
-    const long long o = 2 * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
-    if (o >= P.nPoints) return;
-    const bool two = o + 1 < P.nPoints;
-    bif_hybrid_point<F>(P, O, P.pBegin + o, P.pBegin + (two ? o + 1 : o), o, two ? o + 1 : o, two);
-}
-
-template <class F, bool PRE1>
-__global__ void __launch_bounds__(kMaxBlock) basins_hybrid_kernel_f32(SweepParams P, BasinsOut O) {
-    const long long o = 2 * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
-    if (o >= P.nPoints) return;
-    const bool two = o + 1 < P.nPoints;
-    basins_hybrid_point<F, PRE1>(P, O, P.pBegin + o, P.pBegin + (two ? o + 1 : o), o, two ? o + 1 : o, two);
+    bif_pair_point<F>(P, O, P.pBegin + o, P.pBegin + (two ? o + 1 : o), o, two ? o + 1 : o, two, Component<W>{P.wv});
 }
 
 inline unsigned grid_for(long long n) { return (unsigned)((n + kBlock - 1) / kBlock); }
@@ -133,32 +105,18 @@ int lle_occupancy_variant(int system) {
 
 bool lle_variant_forced() { return g_lle_variant.load(std::memory_order_relaxed) != 0 || lle_env_variant() != 0; }
 
-#define CHAOS_SYSTEM_SWITCH(sys, CALL) \
-    switch (sys) {                     \
-        case SYS_LORENZ_RK4: CALL(SYS_LORENZ_RK4); break; \
-        case SYS_ROSSLER_RK4: CALL(SYS_ROSSLER_RK4); break; \
-        case SYS_CHEN_RK4: CALL(SYS_CHEN_RK4); break; \
-        case SYS_CHAMELEON: CALL(SYS_CHAMELEON); break; \
-        case SYS_ROSSLER_CD: CALL(SYS_ROSSLER_CD); break; \
-        case SYS_SIN3: CALL(SYS_SIN3); break; \
-        case SYS_SIN2: CALL(SYS_SIN2); break; \
-        case SYS_MEMRISTOR: CALL(SYS_MEMRISTOR); break; \
-        default: return cudaErrorInvalidValue; \
-    }
 }  // namespace
 
 std::atomic<int> g_sweep_pairs{-1};
 
-// Paired (two points per thread) FP32 sweeps for the RK4 systems. Mode 1
-// (default): sweeps of at least 4 x SMs x 1024 points run as pairs -- 1-D
-// bifurcations as hybrid pairs (packed transient, recorded part lane by lane),
-// basins maps fully packed -- and smaller ones one point per thread (pairs
-// halve the threads of a latency-bound sweep). Measured on GB300 with the
-// recorded loops' block form: a 1.6 M-point Lorenz 1-D bifurcation 53.4 ms
-// hybrid, 57.5 ms fully packed (Rossler 45.5 / 45.3 ms); the 2048^2 Lorenz
-// basins map 145.9 ms fully packed, 147.7 ms hybrid, and at 1024^2 the
-// packed form ahead by 1.3 / 1.7 / 2.0 % on Lorenz / Rossler / Chen.
-// 2: always fully packed; 0: never; 3: always hybrid. Set with
+// Paired (two points per thread, packed FP32x2 lanes) FP32 sweeps for the RK4
+// systems. Mode 1 (default): sweeps of at least 2048 points per SM run as
+// pairs, smaller ones one point per thread: pairs issue half the instructions
+// but halve the warps that hide each other's latency. Measured on GB300, one
+// point per thread against pairs: 1-D Rossler, 20,000 steps, 240,000 points
+// 7.38 / 7.42 ms, 320,000 9.56 / 9.40 ms, 700,001 20.0 / 18.1 ms; Lorenz
+// basins, 25,000 steps, 500^2 9.09 / 9.18 ms, 600^2 13.2 / 12.9 ms, 1024^2
+// 35.4 / 33.9 ms. 2 (or 3): always pairs; 0: never. Set with
 // chaos_set_tuning or CHAOS_SWEEP_PAIRS.
 int sweep_pairs() {
     const int v = g_sweep_pairs.load(std::memory_order_relaxed);
@@ -176,14 +134,10 @@ int set_sweep_pairs(int v) {
     return 0;
 }
 
-inline unsigned grid_of(long long threads, int block) { return (unsigned)((threads + block - 1) / block); }
-
 // Launch shapes the self-timing tuner (tune.cu) found, per kind (0 1-D
 // bifurcation, 1 basins, 2 LLE map) and RK4 system: 0 = none (the built-in
 // rules below), else form * 1024 + block with form 1 (one point per thread)
-// or 2 (two points per thread in packed FP32x2 lanes); for basins also form 3
-// (two points per thread, packed transient, recorded part lane by lane); for
-// the LLE map also form 12 / 16 (one point per thread, registers shaped for
+// or 2 (two points per thread in packed FP32x2 lanes); for the LLE map also form 12 / 16 (one point per thread, registers shaped for
 // 12 / 16 resident blocks per SM, block 128).
 std::atomic<int> g_shape[3][3];
 
@@ -196,35 +150,14 @@ long long pair_threshold() {
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        return 4LL * std::max(sms, 1) * 1024;
+        return 2048LL * std::max(sms, 1);
     }();
     return threshold;
 }
 
-// Sweeps of at most 8 warps per SM (SMs x 256 points) run the peak detector
-// as selects: there every warp waits on its own dependent chain, and the
-// selects overlap the detector with the next step; larger sweeps run the
-// block form. Measured on GB300 (1-D Lorenz, 20,000 steps): 1,000 points
-// 1.84 ms selects / 2.02 ms blocks, 5,000 1.94 / 2.00, 20,000 2.26 / 2.43,
-// 50,000 2.87 / 2.80; the reference's 300^2 Chameleon sweep 50.6 / 46.5 ms.
-long long select_form_threads() {
-    static long long threads = [] {
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        return (long long)std::max(sms, 1) * 256;
-    }();
-    return threads;
-}
-
-struct Launch {
-    int form;  // 1 one point per thread, 2 packed pairs, 3 hybrid pairs
-    int block;
-};
-
 // Pairs halve the threads: worth it when the sweep fills the GPU several
 // times over, not for small (latency-bound) sweeps. An explicit sweep-pairs
-// mode (0 / 2 / 3) wins; then a tuned shape; then the measured rule.
+// mode (0 / 2) wins; then a tuned shape; then the measured rule.
 Launch sweep_launch(const SweepParams& P, bool basins) {
     if (P.system > SYS_CHEN_RK4 || P.sweepStep) return {1, kBlock};  // a pair shares one step size
     const int mode = sweep_pairs();
@@ -232,36 +165,30 @@ Launch sweep_launch(const SweepParams& P, bool basins) {
     const int block = shape ? shape % 1024 : kBlock;
     const bool big = P.nPoints >= pair_threshold();
     if (mode == 0) return {1, block};
-    if (mode == 2) return {2, block};
-    if (mode == 3) return {3, block};
+    if (mode >= 2) return {2, block};
     if (shape) {
         const int form = shape / 1024;
-        return {form >= 2 && !big ? 1 : form, block};
+        return {big ? form : 1, block};
     }
-    return {big ? (basins ? 2 : 3) : 1, kBlock};
+    return {big ? 2 : 1, kBlock};
 }
 
 template <class F> void launch_bif_pairs(const SweepParams& P, const BifOut& O, int block, cudaStream_t st) {
-    bif_pair_kernel_f32<F><<<grid_of((P.nPoints + 1) / 2, block), block, 0, st>>>(P, O);
+    with_component<true>(P.wv, [&](auto wc) {
+        auto* k = bif_pair_kernel_f32<F, decltype(wc)::kIndex>;
+        const size_t shm = Window<2>::bytes(block);
+        if (shm > 48 * 1024)  // blocks of 256 (the tuner's)
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+        k<<<grid_of((P.nPoints + 1) / 2, block), block, shm, st>>>(P, O);
+    });
     note_launch();
 }
 
-template <class F> void launch_basins_pairs(const SweepParams& P, const BasinsOut& O, int block, cudaStream_t st) {
-    const unsigned g = grid_of((P.nPoints + 1) / 2, block);
-    if (P.preScaller == 1) basins_pair_kernel_f32<F, true><<<g, block, 0, st>>>(P, O);
-    else basins_pair_kernel_f32<F, false><<<g, block, 0, st>>>(P, O);
-    note_launch();
-}
-
-template <class F> void launch_bif_hybrid(const SweepParams& P, const BifOut& O, int block, cudaStream_t st) {
-    bif_hybrid_kernel_f32<F><<<grid_of((P.nPoints + 1) / 2, block), block, 0, st>>>(P, O);
-    note_launch();
-}
-
-template <class F> void launch_basins_hybrid(const SweepParams& P, const BasinsOut& O, int block, cudaStream_t st) {
-    const unsigned g = grid_of((P.nPoints + 1) / 2, block);
-    if (P.preScaller == 1) basins_hybrid_kernel_f32<F, true><<<g, block, 0, st>>>(P, O);
-    else basins_hybrid_kernel_f32<F, false><<<g, block, 0, st>>>(P, O);
+template <int S> void launch_bif_points(const SweepParams& P, const BifOut& O, int block, cudaStream_t st) {
+    with_component<KnownComponent<S, float>::value>(P.wv, [&](auto wc) {
+        bif_kernel_f32<S, decltype(wc)::kIndex>
+            <<<grid_of(P.nPoints, block), block, Window<1>::bytes(block), st>>>(P, O);
+    });
     note_launch();
 }
 
@@ -274,17 +201,7 @@ cudaError_t launch_bif_f32(const SweepParams& P, const BifOut& O, cudaStream_t s
         else launch_bif_pairs<Chen>(P, O, l.block, st);
         return cudaGetLastError();
     }
-    if (l.form == 3) {
-        if (P.system == SYS_LORENZ_RK4) launch_bif_hybrid<Lorenz>(P, O, l.block, st);
-        else if (P.system == SYS_ROSSLER_RK4) launch_bif_hybrid<Rossler>(P, O, l.block, st);
-        else launch_bif_hybrid<Chen>(P, O, l.block, st);
-        return cudaGetLastError();
-    }
-    const bool sel = P.nPoints <= select_form_threads();
-#define CALL(S)                                                                           \
-    (sel ? bif_kernel_f32<S, true><<<grid_of(P.nPoints, l.block), l.block, 0, st>>>(P, O) \
-         : bif_kernel_f32<S, false><<<grid_of(P.nPoints, l.block), l.block, 0, st>>>(P, O), \
-     note_launch())
+#define CALL(S) launch_bif_points<S>(P, O, l.block, st)
     CHAOS_SYSTEM_SWITCH(P.system, CALL)
 #undef CALL
     return cudaGetLastError();
@@ -292,35 +209,8 @@ cudaError_t launch_bif_f32(const SweepParams& P, const BifOut& O, cudaStream_t s
 
 cudaError_t launch_bif_list_f32(const SweepParams& P, const BifOut& O, const int* list, int count, cudaStream_t st) {
     if (count <= 0) return cudaSuccess;
-#define CALL(S) (bif_list_kernel_f32<S><<<grid_for(count), kBlock, 0, st>>>(P, O, list, count), note_launch())
-    CHAOS_SYSTEM_SWITCH(P.system, CALL)
-#undef CALL
-    return cudaGetLastError();
-}
-
-cudaError_t launch_basins_f32(const SweepParams& P, const BasinsOut& O, cudaStream_t st) {
-    if (P.nPoints <= 0) return cudaSuccess;
-    const Launch l = sweep_launch(P, true);
-    if (l.form == 2) {
-        if (P.system == SYS_LORENZ_RK4) launch_basins_pairs<Lorenz>(P, O, l.block, st);
-        else if (P.system == SYS_ROSSLER_RK4) launch_basins_pairs<Rossler>(P, O, l.block, st);
-        else launch_basins_pairs<Chen>(P, O, l.block, st);
-        return cudaGetLastError();
-    }
-    if (l.form == 3) {
-        if (P.system == SYS_LORENZ_RK4) launch_basins_hybrid<Lorenz>(P, O, l.block, st);
-        else if (P.system == SYS_ROSSLER_RK4) launch_basins_hybrid<Rossler>(P, O, l.block, st);
-        else launch_basins_hybrid<Chen>(P, O, l.block, st);
-        return cudaGetLastError();
-    }
-    const unsigned g = grid_of(P.nPoints, l.block);
-    const bool sel = P.nPoints <= select_form_threads();  // the detector as selects, as in the 1-D sweeps
-#define CALL(S)                                                                               \
-    (P.preScaller == 1 ? (sel ? basins_kernel_f32<S, true, true><<<g, l.block, 0, st>>>(P, O)    \
-                              : basins_kernel_f32<S, true, false><<<g, l.block, 0, st>>>(P, O))  \
-                       : (sel ? basins_kernel_f32<S, false, true><<<g, l.block, 0, st>>>(P, O)   \
-                              : basins_kernel_f32<S, false, false><<<g, l.block, 0, st>>>(P, O)), \
-     note_launch())
+#define CALL(S) \
+    (bif_list_kernel_f32<S><<<grid_for(count), kBlock, Window<1>::bytes(kBlock), st>>>(P, O, list, count), note_launch())
     CHAOS_SYSTEM_SWITCH(P.system, CALL)
 #undef CALL
     return cudaGetLastError();

@@ -20,7 +20,7 @@ __global__ void __launch_bounds__(kBlock) bif_kernel(SweepParams P, BifOut O) {
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= P.nPoints) return;
     if constexpr (Legacy) bif_point_legacy<S>(P, O, P.pBegin + o, o);
-    else bif_point<S, double>(P, O, P.pBegin + o, o);
+    else bif_point<S, double>(P, O, P.pBegin + o, o, Component<-1>{P.wv});
 }
 
 // Bifurcation points list[0, count), result row k for list[k].
@@ -29,14 +29,14 @@ __global__ void __launch_bounds__(kBlock) bif_list_kernel(SweepParams P, BifOut 
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     if constexpr (Legacy) bif_point_legacy<S>(P, O, list[k], k);
-    else bif_point<S, double>(P, O, list[k], k);
+    else bif_point<S, double>(P, O, list[k], k, Component<-1>{P.wv});
 }
 
 template <int S>
 __global__ void __launch_bounds__(kBlock) basins_kernel(SweepParams P, BasinsOut O) {
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= P.nPoints) return;
-    basins_point<S, double>(P, O, P.pBegin + o, o);
+    basins_point<S, double, false>(P, O, P.pBegin + o, o, Component<-1>{P.wv});
 }
 
 template <int S>

@@ -25,12 +25,12 @@ __global__ void __launch_bounds__(kBlock) bif_kernel_user(SweepParams P, BifOut 
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= P.nPoints) return;
     if (P.legacyLoop) bif_point_legacy<SYS_USER>(P, O, P.pBegin + o, o);
-    else bif_point<SYS_USER, double>(P, O, P.pBegin + o, o);
+    else bif_point<SYS_USER, double>(P, O, P.pBegin + o, o, Component<-1>{P.wv});
 }
 __global__ void __launch_bounds__(kBlock) basins_kernel_user(SweepParams P, BasinsOut O) {
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= P.nPoints) return;
-    basins_point<SYS_USER, double>(P, O, P.pBegin + o, o);
+    basins_point<SYS_USER, double, false>(P, O, P.pBegin + o, o, Component<-1>{P.wv});
 }
 __global__ void __launch_bounds__(kBlock) lle_kernel_user(LleParams L, double* out) {
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;

@@ -90,13 +90,7 @@ template <class T, bool Sel = false> struct PeakStream {
     //
     // Sel: the same transitions as selects, without branches (a candidate
     // that opens a plateau and a running plateau are one state; "up" and
-    // "below" exclude each other, "ge" excludes "up"). A warp whose threads
-    // each run one latency-bound trajectory (small sweeps) then overlaps the
-    // detector with the next step's arithmetic instead of waiting on its
-    // branches: 1000 Lorenz points 2.50 -> 1.87 ms, 20,000 points 2.87 ->
-    // 2.28 ms against the branching form. Larger sweeps run the branching
-    // form behind its gate in blocks of samples (push_block), which issues
-    // fewer instructions.
+    // "below" exclude each other, "ge" excludes "up").
     CHAOS_HD bool push(T v, T& val, int& t) {
         if constexpr (Gate) {
             const T d = v - p1;
@@ -150,38 +144,71 @@ template <class T, bool Sel = false> struct PeakStream {
         if constexpr (Gate) thr = plateau ? kInfT() : (rise ? T(0) : -kInfT());
         return hit;
     }
+};
 
-    // Pushes the K samples s[0..K-1] (Gate form); on_peak(val, t) for every
-    // peak detected, in order. The gate runs over the whole block first: when
-    // no sample of it would leave the common path (the threshold of each
-    // sample follows from the previous one's difference), the block costs
-    // four operations a sample and one branch; otherwise every sample goes
-    // through push, exactly as one at a time.
-    template <int K, class OnPeak> CHAOS_HD void push_block(const T* s, OnPeak&& on_peak) {
-        static_assert(Gate, "push_block is the float detector's block form");
-        T th = thr, p = p1;
-        bool slow = false;
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-            const T d = s[j] - p;
-            slow |= !(d > th);
-            th = d > T(1e-13f) ? T(0) : -kInfT();
-            p = s[j];
+// The windowed form of the float detector: the samples of a window are judged
+// together once it is full. Per sample it keeps one bit, "above its
+// predecessor", and the sample itself in the caller's buffer; only a sample
+// that is not above a predecessor that was can end a rise, so the exact rules
+// (PeakStream's, one transition for one) run for the few candidates
+// (candidates()) and for a plateau left open by the window before. The
+// samples of a window are finite, or belong to a point whose result they do
+// not reach.
+struct PeakWindow {
+    int nc;     // candidate k-1 is judged when k > nc
+    int i0;     // an open plateau: index of the candidate that opened it; -1: none
+    int n;      // peaks detected so far (the dropped first one included)
+    int tprev;  // time index of the previous detected peak
+
+    CHAOS_HD void init() { nc = 1; i0 = -1; n = 0; tprev = 0; }
+
+    // Candidates of a window of m (1..32) samples, bit m-1-j for sample j:
+    // mask holds the samples' "above its predecessor" bits in the same order,
+    // up the bit of the last sample of the window before (0 at the start).
+    static CHAOS_HD unsigned candidates(unsigned mask, unsigned up, int m) {
+        return ((mask >> 1) | (up << (m - 1))) & ~mask & (m < 32 ? (1u << m) - 1u : 0xffffffffu);
+    }
+
+    // Takes the earliest candidate out of cand; its position in the window.
+    static CHAOS_HD int next(unsigned& cand, int m) {
+#if defined(__CUDA_ARCH__)
+        const int b = 31 - __clz(cand);
+#else
+        const int b = 31 - __builtin_clz(cand);
+#endif
+        cand ^= 1u << b;
+        return m - 1 - b;
+    }
+
+    // Walks the open plateau along the samples j .. m-1 of the window that
+    // starts at index k; at(j) reads sample j, -2 <= j < m (-2 and -1 are the
+    // last two of the window before, 0 at the start). on_peak(val, t) for a
+    // detected peak.
+    template <class At, class OnPeak> CHAOS_HD void walk(int k, int j, int m, At&& at, OnPeak&& on_peak) {
+        for (; j < m; ++j) {
+            const float p = at(j - 1), d = at(j) - p;
+            if (d > 0.f || d < -1e-13f) {
+                if (d < -1e-13f) on_peak(p, (i0 + k + j - 1) >> 1);
+                nc = k + j + 1;
+                i0 = -1;
+                return;
+            }
         }
-        if (__builtin_expect(!slow, 1)) {
-            thr = th;
-            p1 = p;
-            k += K;
-            return;
-        }
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-            T val;
-            int t;
-            if (push(s[j], val, t)) on_peak(val, t);
+    }
+
+    // Judges the candidate whose drop is sample j.
+    template <class At, class OnPeak> CHAOS_HD void judge(int k, int j, int m, At&& at, OnPeak&& on_peak) {
+        if (k + j <= nc) return;
+        const float p = at(j - 1);
+        if (!(p - at(j - 2) > 1e-13f)) return;
+        if (at(j) - p < -1e-13f) {
+            on_peak(p, k + j - 1);
+            nc = k + j + 1;
+        } else {
+            i0 = k + j - 1;
+            walk(k, j + 1, m, at, on_peak);
         }
     }
 };
-
 
 }  // namespace chaos

@@ -548,10 +548,8 @@ int chaos_trajectory(const chaos_exec* ex, int system, long long nTraj, const do
 #define CHAOS_TUNE_LLE_F32_VARIANT 1
 /* CHAOS_TUNE_SWEEP_PAIRS: FP32 bifurcation / basins sweeps of the RK4 systems
    run two points per thread in packed FP32x2 lanes: 1 (default) for sweeps
-   of at least 4 x SMs x 1024 points -- 1-D bifurcations as hybrid pairs
-   (packed transient, recorded part lane by lane), basins maps fully packed --
-   2 always fully packed, 0 never (one point per thread), 3 always hybrid.
-   Results are identical in every mode. */
+   of at least 2048 points per SM, 2 always, 0 never (one point per thread);
+   3 is accepted and means 2. Results are identical in every mode. */
 #define CHAOS_TUNE_SWEEP_PAIRS 2
 /* CHAOS_TUNE_GRID_FMA: 0 (default) swept values start + n*scale with the
    multiply and the add rounded apart, as the reference's getValueByIdx is
@@ -607,8 +605,8 @@ int chaos_get_tuning(int knob);
  * depend on shapes. An explicit CHAOS_TUNE_SWEEP_PAIRS (0 / 2 / 3) or
  * CHAOS_TUNE_LLE_F32_VARIANT still wins. table (may be NULL) receives nTable
  * rows (9 fill all) of 6 doubles: kind (0 1-D bifurcation, 1 basins, 2 LLE
- * map), system, form (0 rule; 1 / 2 trajectories per thread; 3 basins hybrid
- * pairs; 12 / 16 LLE register shapes), block, best ms, the built-in rule's ms.
+ * map), system, form (0 rule; 1 / 2 trajectories per thread; 12 / 16 LLE
+ * register shapes), block, best ms, the built-in rule's ms.
  */
 int chaos_autotune(const chaos_exec* ex, double* table, int nTable);
 
