@@ -13,10 +13,17 @@ namespace chaos {
 
 namespace {
 constexpr int kBlock = 128;
+// Blocks of the sweep kernels: one warp. A warp's FP64 instruction occupies
+// its pipe for about 64 cycles and one SM issues one every 16 to 18, so an SM
+// with w warps takes time proportional to w from four on, and what counts is
+// that no SM gets a warp more than another. Measured (25,000 Lorenz steps, a
+// 150^2 basins map, 704 warps on 152 SMs): blocks of four warps 81.4 ms (two
+// blocks on some SMs), of one warp 60.7 ms; a 100^2 Rossler LLE map 85.7 -> 75.5 ms.
+constexpr int kSweep = 32;
 
 // Legacy: the legacy library's per-point loop (P.legacyLoop != 0).
 template <int S, bool Legacy>
-__global__ void __launch_bounds__(kBlock) bif_kernel(SweepParams P, BifOut O) {
+__global__ void __launch_bounds__(kSweep) bif_kernel(SweepParams P, BifOut O) {
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= P.nPoints) return;
     if constexpr (Legacy) bif_point_legacy<S>(P, O, P.pBegin + o, o);
@@ -25,7 +32,7 @@ __global__ void __launch_bounds__(kBlock) bif_kernel(SweepParams P, BifOut O) {
 
 // Bifurcation points list[0, count), result row k for list[k].
 template <int S, bool Legacy>
-__global__ void __launch_bounds__(kBlock) bif_list_kernel(SweepParams P, BifOut O, const int* list, int count) {
+__global__ void __launch_bounds__(kSweep) bif_list_kernel(SweepParams P, BifOut O, const int* list, int count) {
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     if constexpr (Legacy) bif_point_legacy<S>(P, O, list[k], k);
@@ -33,14 +40,14 @@ __global__ void __launch_bounds__(kBlock) bif_list_kernel(SweepParams P, BifOut 
 }
 
 template <int S>
-__global__ void __launch_bounds__(kBlock) basins_kernel(SweepParams P, BasinsOut O) {
+__global__ void __launch_bounds__(kSweep) basins_kernel(SweepParams P, BasinsOut O) {
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= P.nPoints) return;
     basins_point<S, double, false>(P, O, P.pBegin + o, o, Component<-1>{P.wv});
 }
 
 template <int S>
-__global__ void __launch_bounds__(kBlock) lle_kernel(LleParams L, double* out) {
+__global__ void __launch_bounds__(kSweep) lle_kernel(LleParams L, double* out) {
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= L.nPoints) return;
     out[o] = lle_point_full<S, double>(L, L.pBegin + o);
@@ -48,7 +55,7 @@ __global__ void __launch_bounds__(kBlock) lle_kernel(LleParams L, double* out) {
 
 // The legacy library's LLE kernels' scheme (L.legacyLoop).
 template <int S>
-__global__ void __launch_bounds__(kBlock) lle_legacy_kernel(LleParams L, double* out) {
+__global__ void __launch_bounds__(kSweep) lle_legacy_kernel(LleParams L, double* out) {
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= L.nPoints) return;
     out[o] = lle_point_legacy<S>(L, L.pBegin + o);
@@ -56,7 +63,7 @@ __global__ void __launch_bounds__(kBlock) lle_legacy_kernel(LleParams L, double*
 
 // The LLE map with the reference's cuRAND twin start (L.twin == 2).
 template <int S>
-__global__ void __launch_bounds__(kBlock) lle_reftwin_kernel(LleParams L, double* out) {
+__global__ void __launch_bounds__(kSweep) lle_reftwin_kernel(LleParams L, double* out) {
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= L.nPoints) return;
     out[o] = lle_point_reftwin<S>(L, L.pBegin + o);
@@ -76,7 +83,7 @@ __global__ void legacy_draws_kernel(int kind, long long n, int nx, double* out) 
 // semi_result layout, LLE/src/LLECUDA.cu:102-111): point k's row of 2*NX + NA
 // values holds the orbit after the transient, the parameters and the twin.
 template <int S>
-__global__ void __launch_bounds__(kBlock) lle_states_kernel(LleParams L, const double* states, double* out) {
+__global__ void __launch_bounds__(kSweep) lle_states_kernel(LleParams L, const double* states, double* out) {
     constexpr int NX = Traits<S>::NX, NA = Traits<S>::NA, W = 2 * NX + NA;
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= L.nPoints) return;
@@ -94,7 +101,7 @@ __global__ void __launch_bounds__(kBlock) lle_states_kernel(LleParams L, const d
 
 // Lyapunov spectrum, out[p*SIZE_X + j]
 template <int S>
-__global__ void __launch_bounds__(kBlock) spectrum_kernel(LleParams L, double* out) {
+__global__ void __launch_bounds__(kSweep) spectrum_kernel(LleParams L, double* out) {
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= L.nPoints) return;
     spectrum_point_full<S>(L, L.pBegin + o, out);
@@ -102,7 +109,7 @@ __global__ void __launch_bounds__(kBlock) spectrum_kernel(LleParams L, double* o
 
 // The legacy library's spectrum kernel's scheme (L.legacyLoop).
 template <int S>
-__global__ void __launch_bounds__(kBlock) spectrum_legacy_kernel(LleParams L, double* out) {
+__global__ void __launch_bounds__(kSweep) spectrum_legacy_kernel(LleParams L, double* out) {
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= L.nPoints) return;
     spectrum_point_legacy<S>(L, L.pBegin + o, out);
@@ -112,7 +119,7 @@ __global__ void __launch_bounds__(kBlock) spectrum_legacy_kernel(LleParams L, do
 // (scatter = 1). The same device function as lle_kernel, so a point's value
 // is the FP64 map's value bit for bit.
 template <int S>
-__global__ void __launch_bounds__(kBlock) lle_list_kernel(LleParams L, const int* list, const int* count,
+__global__ void __launch_bounds__(kSweep) lle_list_kernel(LleParams L, const int* list, const int* count,
                                                           double* out, int scatter) {
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= *count) return;
@@ -170,6 +177,7 @@ __global__ void __launch_bounds__(kBlock) trajectory_kernel(const double* x0, co
 }
 
 inline unsigned grid_for(long long n) { return (unsigned)((n + kBlock - 1) / kBlock); }
+inline unsigned warps_for(long long n) { return (unsigned)((n + kSweep - 1) / kSweep); }
 
 #define CHAOS_SYSTEM_SWITCH(sys, CALL) \
     switch (sys) {                     \
@@ -286,8 +294,8 @@ cudaError_t launch_bif_f64(const SweepParams& P, const BifOut& O, cudaStream_t s
     if (P.nPoints <= 0) return cudaSuccess;
 #define CALL(S)                                                             \
     {                                                                       \
-        if (P.legacyLoop) bif_kernel<S, true><<<grid_for(P.nPoints), kBlock, 0, st>>>(P, O); \
-        else bif_kernel<S, false><<<grid_for(P.nPoints), kBlock, 0, st>>>(P, O); \
+        if (P.legacyLoop) bif_kernel<S, true><<<warps_for(P.nPoints), kSweep, 0, st>>>(P, O); \
+        else bif_kernel<S, false><<<warps_for(P.nPoints), kSweep, 0, st>>>(P, O); \
         note_launch();                                                      \
     }
     CHAOS_SYSTEM_SWITCH(P.system, CALL)
@@ -297,7 +305,7 @@ cudaError_t launch_bif_f64(const SweepParams& P, const BifOut& O, cudaStream_t s
 
 cudaError_t launch_basins_f64(const SweepParams& P, const BasinsOut& O, cudaStream_t st) {
     if (P.nPoints <= 0) return cudaSuccess;
-#define CALL(S) (basins_kernel<S><<<grid_for(P.nPoints), kBlock, 0, st>>>(P, O), note_launch())
+#define CALL(S) (basins_kernel<S><<<warps_for(P.nPoints), kSweep, 0, st>>>(P, O), note_launch())
     CHAOS_SYSTEM_SWITCH(P.system, CALL)
 #undef CALL
     return cudaGetLastError();
@@ -307,9 +315,9 @@ cudaError_t launch_lle_f64(const LleParams& L, double* out, cudaStream_t st) {
     if (L.nPoints <= 0) return cudaSuccess;
 #define CALL(S)                                                               \
     {                                                                         \
-        if (L.legacyLoop) lle_legacy_kernel<S><<<grid_for(L.nPoints), kBlock, 0, st>>>(L, out); \
-        else if (L.twin == 2) lle_reftwin_kernel<S><<<grid_for(L.nPoints), kBlock, 0, st>>>(L, out); \
-        else lle_kernel<S><<<grid_for(L.nPoints), kBlock, 0, st>>>(L, out); \
+        if (L.legacyLoop) lle_legacy_kernel<S><<<warps_for(L.nPoints), kSweep, 0, st>>>(L, out); \
+        else if (L.twin == 2) lle_reftwin_kernel<S><<<warps_for(L.nPoints), kSweep, 0, st>>>(L, out); \
+        else lle_kernel<S><<<warps_for(L.nPoints), kSweep, 0, st>>>(L, out); \
         note_launch();                                                        \
     }
     CHAOS_SYSTEM_SWITCH(L.system, CALL)
@@ -326,7 +334,7 @@ cudaError_t launch_legacy_draws(int kind, long long n, int nx, double* out, cuda
 
 cudaError_t launch_lle_states_f64(const LleParams& L, const double* states, double* out, cudaStream_t st) {
     if (L.nPoints <= 0) return cudaSuccess;
-#define CALL(S) (lle_states_kernel<S><<<grid_for(L.nPoints), kBlock, 0, st>>>(L, states, out), note_launch())
+#define CALL(S) (lle_states_kernel<S><<<warps_for(L.nPoints), kSweep, 0, st>>>(L, states, out), note_launch())
     CHAOS_SYSTEM_SWITCH(L.system, CALL)
 #undef CALL
     return cudaGetLastError();
@@ -336,8 +344,8 @@ cudaError_t launch_spectrum_f64(const LleParams& L, double* out, cudaStream_t st
     if (L.nPoints <= 0) return cudaSuccess;
 #define CALL(S)                                                                    \
     {                                                                              \
-        if (L.legacyLoop) spectrum_legacy_kernel<S><<<grid_for(L.nPoints), kBlock, 0, st>>>(L, out); \
-        else spectrum_kernel<S><<<grid_for(L.nPoints), kBlock, 0, st>>>(L, out); \
+        if (L.legacyLoop) spectrum_legacy_kernel<S><<<warps_for(L.nPoints), kSweep, 0, st>>>(L, out); \
+        else spectrum_kernel<S><<<warps_for(L.nPoints), kSweep, 0, st>>>(L, out); \
         note_launch();                                                             \
     }
     CHAOS_SYSTEM_SWITCH(L.system, CALL)
@@ -349,8 +357,8 @@ cudaError_t launch_bif_list_f64(const SweepParams& P, const BifOut& O, const int
     if (count <= 0) return cudaSuccess;
 #define CALL(S)                                                                       \
     {                                                                                 \
-        if (P.legacyLoop) bif_list_kernel<S, true><<<grid_for(count), kBlock, 0, st>>>(P, O, list, count); \
-        else bif_list_kernel<S, false><<<grid_for(count), kBlock, 0, st>>>(P, O, list, count); \
+        if (P.legacyLoop) bif_list_kernel<S, true><<<warps_for(count), kSweep, 0, st>>>(P, O, list, count); \
+        else bif_list_kernel<S, false><<<warps_for(count), kSweep, 0, st>>>(P, O, list, count); \
         note_launch();                                                                \
     }
     CHAOS_SYSTEM_SWITCH(P.system, CALL)
@@ -382,7 +390,7 @@ cudaError_t launch_lle_list_f64(const LleParams& L, const int* list, const int* 
                                 double* out, bool scatter, cudaStream_t st) {
     if (maxCount <= 0) return cudaSuccess;
 #define CALL(S) \
-    (lle_list_kernel<S><<<grid_for(maxCount), kBlock, 0, st>>>(L, list, count, out, scatter ? 1 : 0), note_launch())
+    (lle_list_kernel<S><<<warps_for(maxCount), kSweep, 0, st>>>(L, list, count, out, scatter ? 1 : 0), note_launch())
     CHAOS_SYSTEM_SWITCH(L.system, CALL)
 #undef CALL
     return cudaGetLastError();

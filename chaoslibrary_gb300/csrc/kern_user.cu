@@ -18,7 +18,7 @@ namespace chaos {
 template <> __device__ void user_step<double>(double* x, const double* a, double h) { CALC_DISCRETE_MODEL(x, a, h); }
 
 namespace {
-constexpr int kBlock = 128;
+constexpr int kBlock = 32;  // one warp, as the built-in FP64 sweeps
 inline unsigned grid_for(long long n) { return (unsigned)((n + kBlock - 1) / kBlock); }
 
 __global__ void __launch_bounds__(kBlock) bif_kernel_user(SweepParams P, BifOut O) {
