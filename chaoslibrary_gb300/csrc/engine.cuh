@@ -217,13 +217,17 @@ template <int L> struct Window {
     // Judges the candidates of one window that starts at sample index k: the
     // lanes' candidates one after the other in one loop, so that a warp goes
     // round as often as its busiest thread has candidates. open: bit l set
-    // while lane l's detector is on a plateau. on_peak(l, detector, val, t)
-    // sees the detector before the peak is counted.
+    // while lane l's detector is on a plateau; moved: those of them whose
+    // window is not all one value (an orbit that has come to rest leaves its
+    // plateau open for good, and walking along it would cost more than its
+    // steps: 1,000 Lorenz points with such orbits among them 1.33 -> 0.93 ms).
+    // on_peak(l, detector, val, t) sees the detector before the peak is counted.
     template <class OnPeak>
-    __device__ __forceinline__ void judge(int k, unsigned c0, unsigned c1, int m0, int m1, unsigned& open,
-                                          OnPeak&& on_peak) const {
-        auto run = [&](int l, int j, int m) {  // j < 0: a plateau from the window before
-            PeakWindow d = detector(l);
+    __device__ __forceinline__ void judge(int k, unsigned c0, unsigned c1, int m0, int m1, unsigned moved,
+                                          unsigned& open, OnPeak&& on_peak) const {
+        PeakWindow d0 = detector(0), d1 = d0;
+        if (L == 2) d1 = detector(1);
+        auto run = [&](PeakWindow& d, int l, int j, int m) {  // j < 0: a plateau from the window before
             auto a = [&](int i) { return at(l, i); };
             auto peak = [&](float val, int t) {
                 on_peak(l, d, val, t);
@@ -232,21 +236,28 @@ template <int L> struct Window {
             };
             if (j < 0) d.walk(k, 0, m, a, peak);
             else d.judge(k, j, m, a, peak);
-            open = (open & ~(1u << l)) | (d.i0 >= 0 ? 1u << l : 0u);
-            keep(l, d);
         };
-        if (open != 0u) {
-            if (open & 1u) run(0, -1, m0);
-            if (L == 2 && (open & 2u)) run(1, -1, m1);
-        }
+        if (moved & 1u) run(d0, 0, -1, m0);
+        if (L == 2 && (moved & 2u)) run(d1, 1, -1, m1);
         while ((c0 | c1) != 0u) {
-            const int l = L == 2 && c0 == 0u ? 1 : 0, m = l ? m1 : m0;
-            unsigned c = l ? c1 : c0;
-            const int j = PeakWindow::next(c, m);
-            if (l) c1 = c;
-            else c0 = c;
-            run(l, j, m);
+            if (L == 1) {
+                const int j = PeakWindow::next(c0, m0);
+                run(d0, 0, j, m0);
+            } else {
+                const int l = c0 == 0u ? 1 : 0, m = l ? m1 : m0;
+                unsigned c = l ? c1 : c0;
+                const int j = PeakWindow::next(c, m);
+                if (l) c1 = c;
+                else c0 = c;
+                PeakWindow d = l ? d1 : d0;
+                run(d, l, j, m);
+                if (l) d1 = d;
+                else d0 = d;
+            }
         }
+        open = (d0.i0 >= 0 ? 1u : 0u) | (L == 2 && d1.i0 >= 0 ? 2u : 0u);
+        keep(0, d0);
+        if (L == 2) keep(1, d1);
     }
 };
 
@@ -300,7 +311,8 @@ __device__ __forceinline__ int record_windows(int B, float* x, float* xp, Compon
             p = w.at(0, m - 1);
         }
         const unsigned cand = PeakWindow::candidates(mask, up, m);
-        if ((cand | open) != 0u) w.judge(i, cand, 0u, m, 0, open, on_peak);
+        const unsigned moved = open != 0u && (mask != 0u || p != w.at(0, -1)) ? 1u : 0u;
+        if ((cand | moved) != 0u) w.judge(i, cand, 0u, m, 0, moved, open, on_peak);
         if (dv) break;
         up = mask & 1u;
         w.put(-2, w.at(0, K - 2));
@@ -321,7 +333,7 @@ __device__ __forceinline__ int record_windows(int B, float* x, float* xp, Compon
         }
         if (m > 0) {
             const unsigned cand = PeakWindow::candidates(mask, up, m);
-            if ((cand | open) != 0u) w.judge(i, cand, 0u, m, 0, open, on_peak);
+            if ((cand | open) != 0u) w.judge(i, cand, 0u, m, 0, open, open, on_peak);
         }
     }
     last = p;
@@ -590,6 +602,28 @@ template <> struct PeakSums<float> {
     __device__ __forceinline__ double intervals(double hI) const { return __dmul_rn((double)span, hI); }
 };
 
+// The results of a basins point: kept peaks, the sums of their values and
+// intervals, the last recorded sample. Called by every lane of the warp that
+// has a point to write (they fold the clustering's keys together).
+__device__ __forceinline__ void write_basins_point(const BasinsOut& O, long long o, int flag, int kept, double peaks,
+                                                   double intervals, double last) {
+    double ap, ai;
+    if (flag == 0) { ap = 999.0; ai = 999.0; }
+    else if (flag == -1) { ap = last; ai = -1.0; }
+    else if (kept <= 0) { ap = 1000.0; ai = 1000.0; }
+    else { ap = peaks / (double)kept; ai = intervals / (double)kept; }
+    O.flags[o] = flag;
+    O.avgPeaks[o] = ap;
+    O.avgIntervals[o] = ai;
+    if (O.counts) O.counts[o] = flag == 1 ? kept : 0;
+    if (O.last) O.last[o] = last;
+    if (O.mm) {  // the clustering's normalisation bounds
+        FeatureKeys fk;
+        fk.add(flag, flag == 1 ? kept : 0, ap, ai, last);
+        fk.flush(O.mm);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Basins point (reference calculateTransTimeCUDA + calculateDiscreteModelCUDA
 // + avgPeakFinderCUDA, basinsCUDA.cu:233-314 and 818-864), fused. PRE1: the
@@ -642,23 +676,7 @@ __device__ __forceinline__ void basins_record(const SweepParams& P, const Basins
         n = ps.n;
     }
     if (flag == 1 && P.B > 0 && basins_fixed<NX>(x, xp)) flag = -1;
-    const double last = (double)lastT;
-    const int kept = n > 1 ? n - 1 : 0;
-    double ap, ai;
-    if (flag == 0) { ap = 999.0; ai = 999.0; }
-    else if (flag == -1) { ap = last; ai = -1.0; }
-    else if (kept <= 0) { ap = 1000.0; ai = 1000.0; }
-    else { ap = sums.peaks() / (double)kept; ai = sums.intervals(P.hInterval) / (double)kept; }
-    O.flags[o] = flag;
-    O.avgPeaks[o] = ap;
-    O.avgIntervals[o] = ai;
-    if (O.counts) O.counts[o] = flag == 1 ? kept : 0;
-    if (O.last) O.last[o] = last;
-    if (O.mm) {  // the clustering's normalisation bounds
-        FeatureKeys fk;
-        fk.add(flag, flag == 1 ? kept : 0, ap, ai, last);
-        fk.flush(O.mm);
-    }
+    write_basins_point(O, o, flag, n > 1 ? n - 1 : 0, sums.peaks(), sums.intervals(P.hInterval), (double)lastT);
 }
 
 template <int S, class T, bool PRE1, int W>
@@ -1246,7 +1264,11 @@ __device__ __forceinline__ void record_pair_windows(int B, P2* x, P2* xp, Compon
         }
         const unsigned c0 = rec[0] ? PeakWindow::candidates(mask0, up0, m0) : 0u;
         const unsigned c1 = rec[1] ? PeakWindow::candidates(mask1, up1, m1) : 0u;
-        if ((c0 | c1 | open) != 0u) w.judge(i, c0, c1, m0, m1, open, on_peak);
+        unsigned moved = 0;
+        if (open != 0u)
+            moved = open & ((mask0 != 0u || w.at(0, m0 - 1) != w.at(0, -1) ? 1u : 0u) |
+                            (mask1 != 0u || w.at(1, m1 - 1) != w.at(1, -1) ? 2u : 0u));
+        if ((c0 | c1 | moved) != 0u) w.judge(i, c0, c1, m0, m1, moved, open, on_peak);
         if (rec[0]) last[0] = w.at(0, m0 - 1);
         if (rec[1]) last[1] = w.at(1, m1 - 1);
         if (rec[0] && dv0) {
@@ -1289,7 +1311,7 @@ __device__ __forceinline__ void record_pair_windows(int B, P2* x, P2* xp, Compon
     }
     const unsigned c0 = m0 > 0 ? PeakWindow::candidates(mask0, up0, m0) : 0u;
     const unsigned c1 = m1 > 0 ? PeakWindow::candidates(mask1, up1, m1) : 0u;
-    if ((c0 | c1 | open) != 0u) w.judge(i, c0, c1, m0, m1, open, on_peak);
+    if ((c0 | c1 | open) != 0u) w.judge(i, c0, c1, m0, m1, open, open, on_peak);
 }
 
 template <class F, int W>

@@ -68,11 +68,10 @@ __global__ void __launch_bounds__(kBlock) spectrum_kernel_f32(LleParams L, doubl
 }
 
 // Bifurcation / basins, two points per thread in packed FP32x2 lanes (RK4
-// systems). Bound by the FMA pipe; registers capped at 64 (four blocks of 256,
-// eight of 128 per SM), where the step loop still spills nothing: 1024^2
-// Lorenz basins 34.3 -> 34.1 ms against the 77 it takes unbounded.
+// systems). Bound by the FMA pipe. Registers capped at 80: six blocks of 128
+// per SM, as many as the sample windows leave room for.
 template <class F, int W>
-__global__ void __launch_bounds__(kMaxBlock, 4) bif_pair_kernel_f32(SweepParams P, BifOut O) {
+__global__ void __launch_bounds__(kMaxBlock, 3) bif_pair_kernel_f32(SweepParams P, BifOut O) {
     const long long o = 2 * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
     if (o >= P.nPoints) return;
     const bool two = o + 1 < P.nPoints;

@@ -19,7 +19,7 @@ __global__ void __launch_bounds__(kMaxBlock) basins_kernel_f32(SweepParams P, Ba
 // Two points per thread in packed FP32x2 lanes (RK4 systems); registers capped
 // as in the bifurcation's pair kernel.
 template <class F, bool PRE1, int W>
-__global__ void __launch_bounds__(kMaxBlock, 4) basins_pair_kernel_f32(SweepParams P, BasinsOut O) {
+__global__ void __launch_bounds__(kMaxBlock, 3) basins_pair_kernel_f32(SweepParams P, BasinsOut O) {
     const long long o = 2 * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
     if (o >= P.nPoints) return;
     const bool two = o + 1 < P.nPoints;

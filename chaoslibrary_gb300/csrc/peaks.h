@@ -146,7 +146,7 @@ template <class T, bool Sel = false> struct PeakStream {
     }
 };
 
-// The windowed form of the float detector: the samples of a window are judged
+// The windowed form of the detector: the samples of a window are judged
 // together once it is full. Per sample it keeps one bit, "above its
 // predecessor", and the sample itself in the caller's buffer; only a sample
 // that is not above a predecessor that was can end a rise, so the exact rules
@@ -161,6 +161,10 @@ struct PeakWindow {
     int tprev;  // time index of the previous detected peak
 
     CHAOS_HD void init() { nc = 1; i0 = -1; n = 0; tprev = 0; }
+
+    // a difference clear of the peak finder's threshold
+    static CHAOS_HD bool below(float d) { return d < -1e-13f; }
+    static CHAOS_HD bool below(double d) { return d < -1e-13; }
 
     // Candidates of a window of m (1..32) samples, bit m-1-j for sample j:
     // mask holds the samples' "above its predecessor" bits in the same order,
@@ -186,9 +190,10 @@ struct PeakWindow {
     // detected peak.
     template <class At, class OnPeak> CHAOS_HD void walk(int k, int j, int m, At&& at, OnPeak&& on_peak) {
         for (; j < m; ++j) {
-            const float p = at(j - 1), d = at(j) - p;
-            if (d > 0.f || d < -1e-13f) {
-                if (d < -1e-13f) on_peak(p, (i0 + k + j - 1) >> 1);
+            const auto p = at(j - 1);
+            const auto d = at(j) - p;
+            if (d > 0 || below(d)) {
+                if (below(d)) on_peak(p, (i0 + k + j - 1) >> 1);
                 nc = k + j + 1;
                 i0 = -1;
                 return;
@@ -199,9 +204,9 @@ struct PeakWindow {
     // Judges the candidate whose drop is sample j.
     template <class At, class OnPeak> CHAOS_HD void judge(int k, int j, int m, At&& at, OnPeak&& on_peak) {
         if (k + j <= nc) return;
-        const float p = at(j - 1);
-        if (!(p - at(j - 2) > 1e-13f)) return;
-        if (at(j) - p < -1e-13f) {
+        const auto p = at(j - 1);
+        if (!below(at(j - 2) - p)) return;
+        if (below(at(j) - p)) {
             on_peak(p, k + j - 1);
             nc = k + j + 1;
         } else {
