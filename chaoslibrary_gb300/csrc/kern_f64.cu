@@ -8,6 +8,7 @@
 
 #include "engine.cuh"
 #include "legacy_lle.cuh"
+#include "team.cuh"
 
 namespace chaos {
 
@@ -51,6 +52,22 @@ __global__ void __launch_bounds__(kSweep) lle_kernel(LleParams L, double* out) {
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= L.nPoints) return;
     out[o] = lle_point_full<S, double>(L, L.pBegin + o);
+}
+
+// Small sweeps of the RK4 systems, a team of three lanes per trajectory (team.cuh).
+template <class F>
+__global__ void __launch_bounds__(kSweep) bif_team_kernel(SweepParams P, BifOut O) {
+    __shared__ double cols[kTeamColumn * TeamLane::kTeams];
+    bif_teams<F>(P, O, cols);
+}
+template <class F>
+__global__ void __launch_bounds__(kSweep) basins_team_kernel(SweepParams P, BasinsOut O) {
+    __shared__ double cols[kTeamColumn * TeamLane::kTeams];
+    basins_teams<F>(P, O, cols);
+}
+template <class F, int G>
+__global__ void __launch_bounds__(kSweep) lle_team_kernel(LleParams L, double* out) {
+    lle_teams<F, G>(L, out);
 }
 
 // The legacy library's LLE kernels' scheme (L.legacyLoop).
@@ -290,8 +307,50 @@ bool system_supported(int system) {
 }
 int launch_block_size() { return kBlock; }
 
+// Which sweeps run in teams, by points per SM. Their time grows with the
+// points, that of the kernels with a point per thread with whole warps per SM
+// (flat up to three, 128 points 7 % more, 160 points 1.47 times). Measured,
+// point per thread against teams, Lorenz, 4,000 steps: 1,000 points 6.47 /
+// 3.24 ms, 9,000 6.46 / 3.66, 15,200 6.90 / 5.58, 18,240 (120 per SM) 6.90 /
+// 6.63, 19,456 (128) 6.90 / 7.48, 22,800 (150) 9.49 / 8.28; a 150^2 basins map
+// (25,000 steps) 60.7 / 47.3 ms. LLE maps (with the blocks' norms and logs,
+// which every lane of a team takes), 3,020 steps of orbit and twin, Rossler
+// 40^2 7.12 / 4.24 ms, 100^2 7.12 / 6.10, 110^2 (80 per SM) 7.12 / 6.95, 116^2
+// 7.12 / 8.23; orbit and twin in a team each 40^2 2.62 ms, 77^2 (39 per SM)
+// 4.33 against 4.41 in one team, 90^2 5.95 against 5.32.
+long long sm_points(long long perSm) {
+    static long long sms = [] {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return (long long)(n > 1 ? n : 1);
+    }();
+    return perSm * sms;
+}
+bool team_sweep(long long n) {
+    return n <= sm_points(120) || (n > sm_points(128) && n <= sm_points(160));
+}
+bool team_lle(long long n) { return n <= sm_points(80); }
+bool split_lle(long long n) { return n <= sm_points(40); }
+inline unsigned team_blocks(long long n, int perWarp) { return (unsigned)((n + perWarp - 1) / perWarp); }
+
+#define CHAOS_RK4_SWITCH(sys, CALL)                  \
+    switch (sys) {                                   \
+        case SYS_LORENZ_RK4: CALL(Lorenz); break;    \
+        case SYS_ROSSLER_RK4: CALL(Rossler); break;  \
+        case SYS_CHEN_RK4: CALL(Chen); break;        \
+        default: return cudaErrorInvalidValue;       \
+    }
+
 cudaError_t launch_bif_f64(const SweepParams& P, const BifOut& O, cudaStream_t st) {
     if (P.nPoints <= 0) return cudaSuccess;
+    if (P.system <= SYS_CHEN_RK4 && !P.legacyLoop && !P.sweepStep && team_sweep(P.nPoints)) {
+#define CALL(F) bif_team_kernel<F><<<team_blocks(P.nPoints, TeamLane::kTeams), kSweep, 0, st>>>(P, O)
+        CHAOS_RK4_SWITCH(P.system, CALL)
+#undef CALL
+        note_launch();
+        return cudaGetLastError();
+    }
 #define CALL(S)                                                             \
     {                                                                       \
         if (P.legacyLoop) bif_kernel<S, true><<<warps_for(P.nPoints), kSweep, 0, st>>>(P, O); \
@@ -305,6 +364,13 @@ cudaError_t launch_bif_f64(const SweepParams& P, const BifOut& O, cudaStream_t s
 
 cudaError_t launch_basins_f64(const SweepParams& P, const BasinsOut& O, cudaStream_t st) {
     if (P.nPoints <= 0) return cudaSuccess;
+    if (P.system <= SYS_CHEN_RK4 && team_sweep(P.nPoints)) {
+#define CALL(F) basins_team_kernel<F><<<team_blocks(P.nPoints, TeamLane::kTeams), kSweep, 0, st>>>(P, O)
+        CHAOS_RK4_SWITCH(P.system, CALL)
+#undef CALL
+        note_launch();
+        return cudaGetLastError();
+    }
 #define CALL(S) (basins_kernel<S><<<warps_for(P.nPoints), kSweep, 0, st>>>(P, O), note_launch())
     CHAOS_SYSTEM_SWITCH(P.system, CALL)
 #undef CALL
@@ -313,6 +379,16 @@ cudaError_t launch_basins_f64(const SweepParams& P, const BasinsOut& O, cudaStre
 
 cudaError_t launch_lle_f64(const LleParams& L, double* out, cudaStream_t st) {
     if (L.nPoints <= 0) return cudaSuccess;
+    if (L.system <= SYS_CHEN_RK4 && !L.legacyLoop && L.twin != 2 && team_lle(L.nPoints)) {
+        const bool split = split_lle(L.nPoints);
+#define CALL(F)                                                                                                 \
+    (split ? lle_team_kernel<F, 2><<<team_blocks(L.nPoints, TeamLane::kTeams / 2), kSweep, 0, st>>>(L, out)     \
+           : lle_team_kernel<F, 1><<<team_blocks(L.nPoints, TeamLane::kTeams), kSweep, 0, st>>>(L, out))
+        CHAOS_RK4_SWITCH(L.system, CALL)
+#undef CALL
+        note_launch();
+        return cudaGetLastError();
+    }
 #define CALL(S)                                                               \
     {                                                                         \
         if (L.legacyLoop) lle_legacy_kernel<S><<<warps_for(L.nPoints), kSweep, 0, st>>>(L, out); \
