@@ -1127,6 +1127,74 @@ __device__ __forceinline__ void lle_pair_twin(const LleParams& L, long long p, l
     if (outq) *outq = s1.result(L.tMax);
 }
 
+// Two spectrum points per thread (indices p and q; q == p writes once), lanes
+// of P2: spectrum_point_twin per lane, Gram-Schmidt packed too, with the
+// divisions, logs and reciprocal roots per lane.
+template <class F>
+__device__ __forceinline__ void spectrum_pair_twin(const LleParams& L, long long p, long long q, double* out) {
+    P2 x[3], a[3], e[3][3];
+    float xs[2][3], as[2][3];
+    lle_load<3, 3>(L, p, xs[0], as[0]);
+    lle_load<3, 3>(L, q, xs[1], as[1]);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        a[k] = P2(as[0][k], as[1][k]);
+        x[k] = P2(xs[0][k], xs[1][k]);
+    }
+    const RK4H<P2> c((float)L.h);
+    for (int s = 0; s < L.trans; ++s) rk4_step<F>(x, a, c);
+    const float eps = (float)L.eps;
+    const float inv_eps2 = (float)(1.0 / (L.eps * L.eps));
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) e[j][i] = i == j ? P2(eps, eps) : P2(0.0);
+    double sum[2][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
+    const int nb = L.calcBlocks + 1;
+    for (int b0 = 0; b0 < nb; b0 += kLleGroup) {
+        const int bn = min(kLleGroup, nb - b0);
+        P2 part[3] = {P2(0.0), P2(0.0), P2(0.0)};
+        for (int b = 0; b < bn; ++b) {
+            for (int s = 0; s < L.ntp; ++s) rk4_step_multi<F, 3>(x, e, a, c);
+#pragma unroll
+            for (int j = 1; j < 3; ++j) {
+                // e[m] for m < j hold the orthogonal vectors already; the
+                // projections take the vector as it was before them
+                const P2 d[3] = {e[j][0], e[j][1], e[j][2]};
+#pragma unroll
+                for (int m = 0; m < j; ++m) {
+                    const P2* g = e[m];
+                    const P2 num = fmaT(d[0], g[0], fmaT(d[1], g[1], d[2] * g[2]));
+                    const P2 den = fmaT(g[0], g[0], fmaT(g[1], g[1], g[2] * g[2]));
+                    const P2 frac(den.v.x == 0.f ? -0.f : -(num.v.x / den.v.x),
+                                  den.v.y == 0.f ? -0.f : -(num.v.y / den.v.y));
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) e[j][i] = fmaT(frac, g[i], e[j][i]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const P2 n2 = fmaT(e[j][0], e[j][0], fmaT(e[j][1], e[j][1], e[j][2] * e[j][2]));
+                part[j] = part[j] + P2(__log2f(n2.v.x * inv_eps2), __log2f(n2.v.y * inv_eps2));
+                const P2 r(n2.v.x > 0.f ? eps * rsqrtf(n2.v.x) : 0.f, n2.v.y > 0.f ? eps * rsqrtf(n2.v.y) : 0.f);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) e[j][i] *= r;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            sum[0][j] += (double)part[j].v.x;
+            sum[1][j] += (double)part[j].v.y;
+        }
+    }
+#pragma unroll
+    for (int l = 0; l < 2; ++l) {
+        const long long o = l ? q : p;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) out[o * 3 + j] = sum[l][j] * (0.5 * 0.69314718055994530942) / L.tMax;
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Two bifurcation / basins points per thread in packed FP32x2 lanes (RK4
 // systems). Each lane keeps its own flag, peak detector and outputs and

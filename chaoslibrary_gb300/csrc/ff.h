@@ -124,7 +124,10 @@ template <class W> struct FFH {
 // order and sums), and with TWIN the exact FP32 difference e = p - x of the
 // twin advanced beside it as rk4_step_twin advances it: its stages take the
 // high words of the FF stage states. x is normalised at the end of the step.
-template <class F, bool TWIN, class W>
+// FUSED: the twin's last sum as rk4_step_twin takes it (first_sum), which the
+// LLE maps do with one point per thread and with two; the stage on caller's
+// states (chaos_lle_from_states) rounds product and sum apart.
+template <class F, bool TWIN, bool FUSED = true, class W>
 CHAOS_HD void ff_rk4_step(FF<W>* x, W* e, const FF<W>* a, const W* af, const FFH<W>& c, const RK4H<W>& cf) {
     FF<W> k[3], y[3], acc[3];
     W yw[3], d[3], g[3], dacc[3];
@@ -166,7 +169,11 @@ CHAOS_UNROLL
 CHAOS_UNROLL
     for (int i = 0; i < 3; ++i) {
         x[i] = normalise(fmaT(c.h6, acc[i] + k[i], x[i]));
-        if (TWIN) e[i] = fmaT(cf.h6, dacc[i] + d[i], e[i]);
+        if (TWIN) {
+            if (FUSED && i == 0) dacc[0] = first_sum<F>(g, af, d[0], dacc[0]);
+            else dacc[i] = addR(dacc[i], d[i]);
+            e[i] = fmaT(cf.h6, dacc[i], e[i]);
+        }
     }
 }
 

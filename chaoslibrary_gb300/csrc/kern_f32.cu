@@ -60,11 +60,17 @@ __global__ void __launch_bounds__(kBlock) trajectory_kernel_f32(const double* x0
     trajectory_point<S, float>(x0, a0, h, nSteps, out, t);
 }
 
+// Two points per thread in packed FP32x2 lanes, the first `singles` blocks one.
+// Bound by the FMA pipe; 120 registers, four blocks per SM (a cap at 80 spills:
+// 384^2 Lorenz points, 2,510 steps, 2.28 ms uncapped, 2.33 at five blocks,
+// 2.65 at six; a point per thread 2.52).
 template <class F>
-__global__ void __launch_bounds__(kBlock) spectrum_kernel_f32(LleParams L, double* out) {
-    const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kBlock) spectrum_pair_kernel_f32(LleParams L, double* out, unsigned singles) {
+    bool pair;
+    const long long o = mixed_point(singles, pair);
     if (o >= L.nPoints) return;
-    spectrum_point_twin<F>(L, L.pBegin + o, out);
+    if (pair) spectrum_pair_twin<F>(L, L.pBegin + o, L.pBegin + (o + 1 < L.nPoints ? o + 1 : o), out);
+    else spectrum_point_twin<F>(L, L.pBegin + o, out);
 }
 
 // Bifurcation / basins, two points per thread in packed FP32x2 lanes (RK4
@@ -84,7 +90,8 @@ namespace {
 
 // Variant of the FP32 LLE kernel: 12 / 16 = one point per thread shaped for
 // 12 or 16 resident blocks per SM; 2 = two points per thread in packed
-// FP32x2 lanes. CHAOS_LLE_MINB forces one, otherwise the measured default.
+// FP32x2 lanes. CHAOS_LLE_MINB forces one; otherwise the pair kernel runs, with
+// the blocks that single_blocks says on one point per thread.
 std::atomic<int> g_lle_variant{0};
 
 int lle_env_variant() {
@@ -222,10 +229,17 @@ cudaError_t launch_bif_list_f32(const SweepParams& P, const BifOut& O, const int
 // (from 3.37 waves of resident blocks to 2.99) and the Lorenz map from 39.1
 // to 36.2 ms, results unchanged. Blocks of 64, 128 and 256 (the tuner's
 // choices) all launch under the bound.
+// singles: the first blocks, which run one point per thread (single_blocks),
+// with the default renormalisation only.
 template <class F, int RN = kRenormPow2>
-__global__ void __launch_bounds__(384, 3) lle_pair_kernel_f32(LleParams L, double* out) {
-    const long long o = 2 * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void __launch_bounds__(384, 3) lle_pair_kernel_f32(LleParams L, double* out, unsigned singles) {
+    bool pair;
+    const long long o = mixed_point(singles, pair);
     if (o >= L.nPoints) return;
+    if (RN == kRenormPow2 && !pair) {
+        out[o] = lle_point_twin<F>(L, L.pBegin + o);
+        return;
+    }
     const bool two = o + 1 < L.nPoints;
     lle_pair_twin<F, RN>(L, L.pBegin + o, L.pBegin + (two ? o + 1 : o), out + o, two ? out + o + 1 : nullptr);
 }
@@ -240,9 +254,11 @@ static void launch_twin(const LleParams& L, double* out, cudaStream_t st, int mi
     const int rn = g_lle_renorm.load(std::memory_order_relaxed);
     const unsigned gp = grid_of((L.nPoints + 1) / 2, minb == 2 ? block : kBlock);
     const int bp = minb == 2 ? block : kBlock;
-    if (rn == kRenormF32Log) lle_pair_kernel_f32<F, kRenormF32Log><<<gp, bp, 0, st>>>(L, out);
-    else if (rn == kRenormF64) lle_pair_kernel_f32<F, kRenormF64><<<gp, bp, 0, st>>>(L, out);
-    else if (minb == 2) lle_pair_kernel_f32<F><<<gp, bp, 0, st>>>(L, out);
+    const unsigned singles = single_blocks(L.nPoints);
+    if (rn == kRenormF32Log) lle_pair_kernel_f32<F, kRenormF32Log><<<gp, bp, 0, st>>>(L, out, 0u);
+    else if (rn == kRenormF64) lle_pair_kernel_f32<F, kRenormF64><<<gp, bp, 0, st>>>(L, out, 0u);
+    else if (minb == 0) lle_pair_kernel_f32<F><<<mixed_grid(L.nPoints, singles), kBlock, 0, st>>>(L, out, singles);
+    else if (minb == 2) lle_pair_kernel_f32<F><<<gp, bp, 0, st>>>(L, out, 0u);
     else if (minb >= 16) lle_twin_kernel_f32<F, 16><<<grid_for(L.nPoints), kBlock, 0, st>>>(L, out);
     else lle_twin_kernel_f32<F, 12><<<grid_for(L.nPoints), kBlock, 0, st>>>(L, out);
     note_launch();
@@ -274,7 +290,7 @@ int get_lle_renorm() { return g_lle_renorm.load(); }
 cudaError_t launch_lle_f32(const LleParams& L, double* out, cudaStream_t st) {
     if (L.nPoints <= 0) return cudaSuccess;
     // an explicit variant (chaos_set_tuning / CHAOS_LLE_MINB) wins, then a tuned shape
-    int minb = lle_occupancy_variant(L.system), block = kBlock;
+    int minb = lle_variant_forced() ? lle_occupancy_variant(L.system) : 0, block = kBlock;
     const int shape = shape_of(2, L.system);
     if (shape && !lle_variant_forced()) {
         minb = shape / 1024;
@@ -293,14 +309,18 @@ cudaError_t launch_lle_f32(const LleParams& L, double* out, cudaStream_t st) {
     return cudaGetLastError();
 }
 
+template <class F> static void launch_spectrum(const LleParams& L, double* out, cudaStream_t st) {
+    const unsigned singles = single_blocks(L.nPoints);
+    spectrum_pair_kernel_f32<F><<<mixed_grid(L.nPoints, singles), kBlock, 0, st>>>(L, out, singles);
+}
+
 cudaError_t launch_spectrum_f32(const LleParams& L, double* out, cudaStream_t st) {
     if (L.nPoints <= 0) return cudaSuccess;
-    const unsigned g = grid_for(L.nPoints);
     switch (L.system) {
-        case SYS_LORENZ_RK4: spectrum_kernel_f32<Lorenz><<<g, kBlock, 0, st>>>(L, out); break;
-        case SYS_ROSSLER_RK4: spectrum_kernel_f32<Rossler><<<g, kBlock, 0, st>>>(L, out); break;
-        case SYS_CHEN_RK4: spectrum_kernel_f32<Chen><<<g, kBlock, 0, st>>>(L, out); break;
-        case SYS_CHAMELEON: spectrum_chameleon_kernel_f32<<<g, kBlock, 0, st>>>(L, out); break;
+        case SYS_LORENZ_RK4: launch_spectrum<Lorenz>(L, out, st); break;
+        case SYS_ROSSLER_RK4: launch_spectrum<Rossler>(L, out, st); break;
+        case SYS_CHEN_RK4: launch_spectrum<Chen>(L, out, st); break;
+        case SYS_CHAMELEON: spectrum_chameleon_kernel_f32<<<grid_for(L.nPoints), kBlock, 0, st>>>(L, out); break;
         default: return cudaErrorNotSupported;
     }
     note_launch();

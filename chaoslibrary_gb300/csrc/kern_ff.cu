@@ -20,11 +20,12 @@
 
 #include "batch.h"
 #include "engine.cuh"
+#include "sweep_launch.h"
 
 namespace chaos {
 
 namespace {
-constexpr int kBlock = 128;
+constexpr int kBlock = kSweepBlock;
 
 // frexp exponent of a positive normal float (0 for +0 gives -126).
 __device__ __forceinline__ int exp_of(float v) { return (int)((__float_as_uint(v) >> 23) & 0xff) - 126; }
@@ -34,14 +35,14 @@ __device__ __forceinline__ double finite_or_nan(double v) { return isfinite(v) ?
 // The Benettin blocks of an FF orbit x with the FP32 twin difference e
 // (started where the caller put it), renormalised by powers of two; the
 // stretch of the blocks relative to eps, as the reference measures it.
-template <class F>
+template <class F, bool FUSED = true>
 __device__ __forceinline__ double ff_benettin(const LleParams& L, FF<float>* x, float* e, const FF<float>* a,
                                               const float* af, const FFH<float>& c, const RK4H<float>& cf) {
     const int eps2Exp = exp_of((float)L.eps * (float)L.eps);
     int ktot = 0;
     const int nb = L.calcBlocks + 1;
     for (int b = 0; b < nb; ++b) {
-        for (int s = 0; s < L.ntp; ++s) ff_rk4_step<F, true>(x, e, a, af, c, cf);
+        for (int s = 0; s < L.ntp; ++s) ff_rk4_step<F, true, FUSED>(x, e, a, af, c, cf);
         if (b + 1 < nb) {
             const float n2 = fmaf(e[0], e[0], fmaf(e[1], e[1], e[2] * e[2]));
             const int k = pow2_rescale_exponent(n2, eps2Exp);
@@ -100,7 +101,7 @@ __global__ void __launch_bounds__(kBlock) lle_ff_states_kernel(LleParams L, cons
         af[i] = (float)r[3 + i];
         e[i] = (float)(r[6 + i] - r[i]);
     }
-    out[k] = ff_benettin<F>(L, x, e, a, af, ff_consts(L.h), RK4H<float>((float)L.h));
+    out[k] = ff_benettin<F, false>(L, x, e, a, af, ff_consts(L.h), RK4H<float>((float)L.h));
 }
 
 // Two points per thread: FF words are packed pairs (one paired FP32
@@ -160,10 +161,16 @@ __global__ void __launch_bounds__(kBlock) lle_ff_kernel(LleParams L, double* out
     out[o] = lle_point_ff<F>(L, L.pBegin + o);
 }
 
+// Two points per thread, the first `singles` blocks one.
 template <class F>
-__global__ void __launch_bounds__(kBlock) lle_ff_pair_kernel(LleParams L, double* out) {
-    const long long o = 2 * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void __launch_bounds__(kBlock) lle_ff_pair_kernel(LleParams L, double* out, unsigned singles) {
+    bool pair;
+    const long long o = mixed_point(singles, pair);
     if (o >= L.nPoints) return;
+    if (!pair) {
+        out[o] = lle_point_ff<F>(L, L.pBegin + o);
+        return;
+    }
     const bool two = o + 1 < L.nPoints;
     lle_pair_ff<F>(L, L.pBegin + o, L.pBegin + (two ? o + 1 : o), out + o, two ? out + o + 1 : nullptr);
 }
@@ -237,13 +244,16 @@ GroupFF group_ff_for(int system) {
 
 unsigned blocks_for(long long threads) { return (unsigned)((threads + kBlock - 1) / kBlock); }
 
-// 1 (default): two points per thread in packed words; 0: one point per thread.
+// 1 (default): two points per thread in packed words where that is faster
+// (single_blocks); 0: one point per thread.
 // Results are identical either way (every paired operation rounds each lane as
 // the scalar operation does).
 std::atomic<int> g_ff_pairs{1};
 
 template <class F> void launch_ff(const LleParams& L, double* out, cudaStream_t st) {
-    if (g_ff_pairs.load(std::memory_order_relaxed)) lle_ff_pair_kernel<F><<<blocks_for((L.nPoints + 1) / 2), kBlock, 0, st>>>(L, out);
+    const unsigned singles = single_blocks(L.nPoints);
+    if (g_ff_pairs.load(std::memory_order_relaxed))
+        lle_ff_pair_kernel<F><<<mixed_grid(L.nPoints, singles), kBlock, 0, st>>>(L, out, singles);
     else lle_ff_kernel<F><<<blocks_for(L.nPoints), kBlock, 0, st>>>(L, out);
     note_launch();
 }

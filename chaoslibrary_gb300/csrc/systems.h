@@ -107,7 +107,13 @@ CHAOS_HD double addR(double a, double b) {
     return a + b;
 #endif
 }
-CHAOS_HD float addR(float a, float b) { return a + b; }
+CHAOS_HD float addR(float a, float b) {
+#if defined(__CUDA_ARCH__)
+    return __fadd_rn(a, b);
+#else
+    return a + b;
+#endif
+}
 
 // a*b + c as each arithmetic's kernels round it: FP64 as written, a product
 // and a sum (the FP64 translation units and the host checker compile without
@@ -167,6 +173,20 @@ struct Chen {
     }
 };
 
+// The last stage's sums acc + f(y) of a classic RK4 step. Where a component's
+// derivative is a product (a[0] times a difference, Lorenz and Chen), the FP32
+// forms add it as one fused multiply-add, written out: left to the compiler,
+// the choice depends on the kernel around the step, and one point per thread
+// has to round as two in packed lanes. FP64 rounds the product and the sum.
+template <class F> struct FirstIsProduct { static constexpr bool value = false; };
+template <> struct FirstIsProduct<Lorenz> { static constexpr bool value = true; };
+template <> struct FirstIsProduct<Chen> { static constexpr bool value = true; };
+
+template <class F, class T> CHAOS_HD T first_sum(const T* v, const T* a, const T& k0, const T& acc0) {
+    if constexpr (FirstIsProduct<F>::value && !std::is_same<T, double>::value) return fmaT(a[0], v[1] - v[0], acc0);
+    else return addR(acc0, k0);
+}
+
 // Step-size constants of one classic RK4 step, computed once per launch.
 template <class T> struct RK4H {
     T h, hh, h6;
@@ -214,8 +234,11 @@ CHAOS_UNROLL
             wy = fmaT(-hs, k[2], w);
         }
     }
+    acc[0] = first_sum<Lorenz>(y, a, k[0], acc[0]);
+    acc[1] = addR(acc[1], k[1]);
+    acc[2] = addR(acc[2], k[2]);
 CHAOS_UNROLL
-    for (int i = 0; i < 3; ++i) x[i] = fmaT(c.h6, addR(acc[i], k[i]), x[i]);
+    for (int i = 0; i < 3; ++i) x[i] = fmaT(c.h6, acc[i], x[i]);
 }
 
 template <class F, class T> CHAOS_HD void rk4_step(T* x, const T* a, const RK4H<T>& c) {
@@ -234,8 +257,11 @@ CHAOS_UNROLL
 CHAOS_UNROLL
     for (int i = 0; i < 3; ++i) { acc[i] = fmaT(T(2), k[i], acc[i]); y[i] = fmaT(c.h, k[i], x[i]); }
     F::f(y, a, k);
+    acc[0] = first_sum<F>(y, a, k[0], acc[0]);
+    acc[1] = addR(acc[1], k[1]);
+    acc[2] = addR(acc[2], k[2]);
 CHAOS_UNROLL
-    for (int i = 0; i < 3; ++i) x[i] = fmaT(c.h6, addR(acc[i], k[i]), x[i]);
+    for (int i = 0; i < 3; ++i) x[i] = fmaT(c.h6, acc[i], x[i]);
 }
 
 // One RK4 step of the base trajectory x together with the exact difference
@@ -273,10 +299,16 @@ CHAOS_UNROLL
     }
     F::f(y, a, k);
     F::df(y, g, a, d);
+    acc[0] = first_sum<F>(y, a, k[0], acc[0]);
+    dacc[0] = first_sum<F>(g, a, d[0], dacc[0]);
 CHAOS_UNROLL
     for (int i = 0; i < 3; ++i) {
-        x[i] = fmaT(c.h6, acc[i] + k[i], x[i]);
-        e[i] = fmaT(c.h6, dacc[i] + d[i], e[i]);
+        if (i > 0) {
+            acc[i] = addR(acc[i], k[i]);
+            dacc[i] = addR(dacc[i], d[i]);
+        }
+        x[i] = fmaT(c.h6, acc[i], x[i]);
+        e[i] = fmaT(c.h6, dacc[i], e[i]);
     }
 }
 
@@ -328,11 +360,18 @@ CHAOS_UNROLL
     F::f(y, a, k);
 CHAOS_UNROLL
     for (int q = 0; q < NE; ++q) F::df(y, g[q], a, d[q]);
+    acc[0] = first_sum<F>(y, a, k[0], acc[0]);
+CHAOS_UNROLL
+    for (int q = 0; q < NE; ++q) dacc[q][0] = first_sum<F>(g[q], a, d[q][0], dacc[q][0]);
 CHAOS_UNROLL
     for (int i = 0; i < 3; ++i) {
-        x[i] = fmaT(c.h6, acc[i] + k[i], x[i]);
+        if (i > 0) acc[i] = addR(acc[i], k[i]);
+        x[i] = fmaT(c.h6, acc[i], x[i]);
 CHAOS_UNROLL
-        for (int q = 0; q < NE; ++q) e[q][i] = fmaT(c.h6, dacc[q][i] + d[q][i], e[q][i]);
+        for (int q = 0; q < NE; ++q) {
+            if (i > 0) dacc[q][i] = addR(dacc[q][i], d[q][i]);
+            e[q][i] = fmaT(c.h6, dacc[q][i], e[q][i]);
+        }
     }
 }
 
