@@ -10,12 +10,11 @@
 //   1. one pass over the points: the cell of every point (floor(f / side) per
 //      dimension, side = eps / sqrt(D) shrunk by 1e-9, so two points of one
 //      cell are always within eps and a neighbour within eps is at most R = 2
-//      cells away per dimension) goes into an open-addressing hash table; the
-//      runs of equal cells along a warp fold into it, with one atomic per
-//      quantity, their point count, bounding box (float bounds rounded
-//      outward: still a box around the points), smallest and largest index
-//      (the cell's representatives) and smallest fixed-point index, and a
-//      clamped/NaN mark; the point keeps its slot;
+//      cells away per dimension) goes into an open-addressing hash table with
+//      the cell's point count, bounding box (float bounds rounded outward:
+//      still a box around the points), smallest index and another one (its
+//      representatives), smallest fixed-point index and a clamped/NaN mark,
+//      gathered per block in shared memory; the point keeps its slot;
 //   2. per cell: dense (a safe cell with >= minPts points -- every included
 //      point in the reference mode: all its points are core) or not; the
 //      occupied neighbour cells; per neighbouring pair, the bounding boxes
@@ -68,7 +67,7 @@ constexpr int kTPB = 256;
 constexpr unsigned long long kEmpty = ~0ull;
 constexpr long long kLim = 1LL << 19;  // clamp of cell coordinates (21-bit packing for D = 3)
 constexpr int kR = 2;                  // neighbour reach in cells
-constexpr int kReps = 2;               // representatives per cell: its smallest and largest point index
+constexpr int kReps = 2;               // representatives per cell: its smallest point index and another
 
 __device__ __forceinline__ unsigned long long pack(const long long* c, int D) {
     if (D <= 2) {
@@ -306,31 +305,42 @@ struct BasinSrc {
 };
 
 // ---- the cell table: slot-indexed statistics of the occupied cells ---------------
+struct alignas(16) CellStats {
+    unsigned lo[3];  // order keys of the feature minima rounded down to float
+    unsigned hi[3];  // order keys of the feature maxima rounded up to float
+    int cnt;         // points
+    int bad;         // a clamped or NaN point
+    int minIdx;      // smallest point index
+    int other;       // some point's index, mostly far from the smallest (-1: none yet)
+    int minFix;      // smallest fixed-point index (reference mode)
+    int pad;
+};
 struct Table {
     unsigned long long* key;  // packed cell coordinates, kEmpty for a free slot
     unsigned long long mask;  // capacity - 1 (a power of two)
-    int* cnt;                 // points
-    unsigned* lo;             // 3 per slot: order keys of the feature minima rounded down to float
-    unsigned* hi;             // 3 per slot: order keys of the feature maxima rounded up to float
-    int* minIdx;              // smallest point index
-    int* maxIdx;              // largest point index
-    int* minFix;              // smallest fixed-point index (reference mode)
-    int* bad;                 // a clamped or NaN point
+    CellStats* st;
 };
+
+__device__ __forceinline__ CellStats empty_stats() {
+    CellStats s;
+    for (int d = 0; d < 3; ++d) {
+        s.lo[d] = kFKeyPosInf;
+        s.hi[d] = kFKeyNegInf;
+    }
+    s.cnt = 0;
+    s.bad = 0;
+    s.minIdx = INT_MAX;
+    s.other = -1;
+    s.minFix = INT_MAX;
+    s.pad = 0;
+    return s;
+}
 
 __global__ void table_init_kernel(Table T, long long cap) {
     const long long h = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (h >= cap) return;
     T.key[h] = kEmpty;
-    T.cnt[h] = 0;
-    for (int d = 0; d < 3; ++d) {
-        T.lo[3 * h + d] = kFKeyPosInf;
-        T.hi[3 * h + d] = kFKeyNegInf;
-    }
-    T.minIdx[h] = INT_MAX;
-    T.maxIdx[h] = -1;
-    T.minFix[h] = INT_MAX;
-    T.bad[h] = 0;
+    T.st[h] = empty_stats();
 }
 
 __device__ __forceinline__ long long table_insert(unsigned long long* tab, unsigned long long mask,
@@ -442,97 +452,143 @@ __device__ __forceinline__ long long table_slot(unsigned long long* tab, unsigne
     return -1;
 }
 
-// Step 1, one point per thread. Consecutive grid points mostly share a cell,
-// so a warp's lanes form runs of equal keys; each run's statistics are
-// reduced to its first lane (warp-wide reductions when the whole row is one
-// run, shuffles otherwise), which finds the slot (a read once the cell is in
-// the table) and folds the run in with one 32-bit atomic per quantity: a
-// run's smallest and largest index are its end lanes', its smallest
-// fixed-point index and its clamped/NaN mark come from ballots, its box from
-// the reductions. (Folding each block's runs into a shared-memory table
-// first, or keeping extreme points as representatives with 64-bit atomics,
-// measured slower on a 2048^2 basin map: 338 and 494 against 267 us.) Fout
-// (basin maps, when the caller asks for the normalised features) receives
-// each point's row.
+// Step 1. Each block takes a contiguous run of points and folds them into a
+// small table of cells in shared memory, which it adds to the cell table at
+// its end: the lanes of a warp that share a cell form a group, whose first
+// lane finds (or claims) the cell's entry, adds the group's count and keeps
+// its smallest and largest index; a lane whose point lies outside the box it
+// reads widens it. A group that finds no room goes to the cell table itself.
+// Bound by the read of the points. Folding every run of equal cells straight
+// into the cell table, with an atomic per quantity, spent its time on the
+// addresses of the few cells that hold most points: 1,000,000 points in
+// random order 480 -> 55 us, a 2048^2 basin map 284 -> 273 us; reading a cell's
+// values there before an atomic (1,440 us) waits at the same addresses.
+constexpr int kCellBlock = 512, kCellBlocksPerSm = 2;
+constexpr int kBlockCells = 512;  // entries of a block's table, a power of two
+constexpr int kBlockProbes = 4;
+
+struct BlockCells {
+    unsigned long long key[kBlockCells];
+    int slot[kBlockCells];  // in the cell table, -1 until found
+    CellStats st[kBlockCells];
+};
+
+// Adds a cell's statistics (of some of its points) to its slot.
+__device__ __forceinline__ void fold_stats(CellStats* to, const CellStats& s, int D, long long n) {
+    atomicAdd(&to->cnt, s.cnt);
+    if (s.minIdx < __ldcg(&to->minIdx)) atomicMin(&to->minIdx, s.minIdx);
+    const int other = __ldcg(&to->other);
+    if (other < 0 || s.other - other > (int)(n >> 6)) __stcg(&to->other, s.other);  // (any writer's will do)
+    if (s.minFix != INT_MAX) atomicMin(&to->minFix, s.minFix);
+    if (s.bad) atomicOr(&to->bad, 1);
+    for (int d = 0; d < D; ++d) {
+        if (s.lo[d] < __ldcg(&to->lo[d])) atomicMin(&to->lo[d], s.lo[d]);
+        if (s.hi[d] > __ldcg(&to->hi[d])) atomicMax(&to->hi[d], s.hi[d]);
+    }
+}
+
+// Fout (basin maps, when the caller asks for the normalised features) receives
+// each point's row. chunk: points of a block, a multiple of its threads.
 template <class Src>
-__global__ void __launch_bounds__(kTPB) cells_kernel(Src S, long long n, double invSide, Table T, int* slot,
-                                                     double* Fout, int* err) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kCellBlock, kCellBlocksPerSm)
+cells_kernel(Src S, long long n, long long chunk, double invSide, Table T, int* slot, double* Fout, int* err) {
+    extern __shared__ unsigned long long cell_smem[];
+    BlockCells& B = *reinterpret_cast<BlockCells*>(cell_smem);
+    for (int e = threadIdx.x; e < kBlockCells; e += blockDim.x) {
+        B.key[e] = kEmpty;
+        B.slot[e] = -1;
+        B.st[e] = empty_stats();
+    }
+    __syncthreads();
     const int lane = threadIdx.x & 31;
-    unsigned long long key = kEmpty;
-    double v[3] = {0.0, 0.0, 0.0};
-    bool bad = false, fix = false;
-    if (i < n && S.included(i)) {
-        S.load(i, v);
-        long long c[3] = {0, 0, 0};
-        bad = cell_coords(v, S.D, invSide, c);
-        key = pack(c, S.D);
-        fix = S.fix(i);
-    }
-    if (Fout && i < n)
-        for (int d = 0; d < 3; ++d) Fout[i * 3 + d] = v[d];
-    // runs of equal keys: heads, and each lane's run [head, tail]
-    const unsigned long long prevKey = __shfl_up_sync(0xffffffffu, key, 1);
-    const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || prevKey != key);
-    const unsigned upTo = 0xffffffffu >> (31 - lane);  // lanes 0..lane
-    const int head = 31 - __clz(heads & upTo);
-    const unsigned after = heads & ~upTo;               // heads above this lane
-    const int tail = after ? __ffs(after) - 2 : 31;
-    const bool isHead = lane == head;
-    long long h = -1;
-    if (isHead && key != kEmpty) {
-        h = table_slot(T.key, T.mask, key);
-        if (h < 0) atomicAdd(err, 1);
-    }
-    h = __shfl_sync(0xffffffffu, h, head);
-    if (i < n) slot[i] = key == kEmpty || h < 0 ? -1 : (int)h;
-    // box (float, rounded outward), reduced toward the head
-    unsigned lo[3], hi[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const bool skip = d >= S.D || is_nan(v[d]) || key == kEmpty;
-        lo[d] = skip ? kFKeyPosInf : fkey(__double2float_rd(v[d]));
-        hi[d] = skip ? kFKeyNegInf : fkey(__double2float_ru(v[d]));
-    }
-    if (heads == 1u) {  // the whole row is one run (the common case)
+    const long long begin = blockIdx.x * chunk, end = begin + chunk < n ? begin + chunk : n;
+    for (long long i0 = begin; i0 < end; i0 += blockDim.x) {
+        const long long i = i0 + threadIdx.x;
+        unsigned long long key = kEmpty;
+        double v[3] = {0.0, 0.0, 0.0};
+        bool bad = false, fix = false;
+        if (i < end && S.included(i)) {
+            S.load(i, v);
+            long long c[3] = {0, 0, 0};
+            bad = cell_coords(v, S.D, invSide, c);
+            key = pack(c, S.D);
+            fix = S.fix(i);
+        }
+        if (Fout && i < end)
+            for (int d = 0; d < 3; ++d) Fout[i * 3 + d] = v[d];
+        // the lanes of this lane's cell (a row of one cell, common in a map, without the match)
+        const unsigned long long key0 = __shfl_sync(0xffffffffu, key, 0);
+        const unsigned grp = __all_sync(0xffffffffu, key == key0) ? 0xffffffffu : __match_any_sync(0xffffffffu, key);
+        const int leader = __ffs(grp) - 1;
+        int e = -1, h = -1;  // the entry of the block's table (-1: no room), the slot of the cell table
+        if (lane == leader && key != kEmpty) {
+            unsigned p = (unsigned)(mix(key) >> 40);
+            for (int k = 0; k < kBlockProbes; ++k, ++p) {
+                const int q = (int)(p & (kBlockCells - 1));
+                unsigned long long t = *(volatile unsigned long long*)&B.key[q];
+                if (t == kEmpty) {
+                    t = atomicCAS(&B.key[q], kEmpty, key);
+                    if (t == kEmpty) t = key;
+                }
+                if (t == key) {
+                    e = q;
+                    h = *(volatile int*)&B.slot[q];
+                    break;
+                }
+            }
+            if (h < 0) {
+                h = (int)table_slot(T.key, T.mask, key);
+                if (h < 0) atomicAdd(err, 1);
+                if (e >= 0) *(volatile int*)&B.slot[e] = h;
+            }
+        }
+        e = __shfl_sync(0xffffffffu, e, leader);
+        h = __shfl_sync(0xffffffffu, h, leader);
+        if (i < end) slot[i] = key == kEmpty ? -1 : h;
+        const unsigned fixes = __ballot_sync(0xffffffffu, fix) & grp;
+        const unsigned bads = __ballot_sync(0xffffffffu, bad) & grp;
+        if (key == kEmpty || h < 0) continue;
+        unsigned lo[3], hi[3];  // the point's box (float, rounded outward)
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            if (d >= S.D) continue;
-            lo[d] = __reduce_min_sync(0xffffffffu, lo[d]);
-            hi[d] = __reduce_max_sync(0xffffffffu, hi[d]);
+            const bool skip = d >= S.D || is_nan(v[d]);
+            lo[d] = skip ? kFKeyPosInf : fkey(__double2float_rd(v[d]));
+            hi[d] = skip ? kFKeyNegInf : fkey(__double2float_ru(v[d]));
         }
-    } else {
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const bool in = lane + o <= tail;
+        const int last = (int)(i - lane) + 31 - __clz(grp);
+        const int firstFix = fixes ? (int)(i - lane) + __ffs(fixes) - 1 : INT_MAX;
+        if (e >= 0) {
+            CellStats& st = B.st[e];
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
                 if (d >= S.D) continue;
-                const unsigned a = __shfl_down_sync(0xffffffffu, lo[d], o);
-                const unsigned b = __shfl_down_sync(0xffffffffu, hi[d], o);
-                if (in) {
-                    lo[d] = a < lo[d] ? a : lo[d];
-                    hi[d] = b > hi[d] ? b : hi[d];
-                }
+                if (lo[d] < *(volatile unsigned*)&st.lo[d]) atomicMin(&st.lo[d], lo[d]);
+                if (hi[d] > *(volatile unsigned*)&st.hi[d]) atomicMax(&st.hi[d], hi[d]);
             }
+            if (lane == leader) {
+                atomicAdd(&st.cnt, __popc(grp));
+                atomicMin(&st.minIdx, (int)i);
+                atomicMax(&st.other, last);
+                if (fixes) atomicMin(&st.minFix, firstFix);
+                if (bads) atomicOr(&st.bad, 1);
+            }
+        } else {
+            CellStats s = empty_stats();
+            for (int d = 0; d < S.D; ++d) {
+                s.lo[d] = __reduce_min_sync(grp, lo[d]);
+                s.hi[d] = __reduce_max_sync(grp, hi[d]);
+            }
+            s.cnt = __popc(grp);
+            s.minIdx = (int)i;
+            s.other = last;
+            s.minFix = firstFix;
+            s.bad = bads != 0u;
+            if (lane == leader) fold_stats(T.st + h, s, S.D, n);
         }
     }
-    const unsigned fixes = __ballot_sync(0xffffffffu, fix);
-    const unsigned bads = __ballot_sync(0xffffffffu, bad);
-    if (!isHead || key == kEmpty || h < 0) return;
-    const unsigned run = (tail == 31 ? 0xffffffffu : ((1u << (tail + 1)) - 1u)) & ~((1u << head) - 1u);
-    const long long base = i - lane;  // index of lane 0
-    atomicAdd(&T.cnt[h], tail - head + 1);
-    atomicMin(&T.minIdx[h], (int)i);
-    atomicMax(&T.maxIdx[h], (int)(base + tail));
-    if (fixes & run) atomicMin(&T.minFix[h], (int)(base + __ffs(fixes & run) - 1));
-    if (bads & run) atomicOr(&T.bad[h], 1);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        if (d >= S.D) continue;
-        atomicMin(&T.lo[3 * h + d], lo[d]);
-        atomicMax(&T.hi[3 * h + d], hi[d]);
-    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < kBlockCells; e += blockDim.x)
+        if (B.key[e] != kEmpty && B.slot[e] >= 0) fold_stats(T.st + B.slot[e], B.st[e], S.D, n);
 }
 
 __global__ void occupied_kernel(const unsigned long long* tab, long long cap, int* occ) {
@@ -579,26 +635,27 @@ __global__ void finalize_kernel(Src S, Cells K, const int* cellSlot, Table T, in
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= K.C) return;
     const long long h = cellSlot[c];
-    const int n = T.cnt[h];
+    const CellStats t = T.st[h];
+    const int n = t.cnt;
     K.cnt[c] = n;
     for (int d = 0; d < 3; ++d) {
-        K.lo[3 * c + d] = d < K.D ? (double)unfkey(T.lo[3 * h + d]) : 0.0;
-        K.hi[3 * c + d] = d < K.D ? (double)unfkey(T.hi[3 * h + d]) : 0.0;
+        K.lo[3 * c + d] = d < K.D ? (double)unfkey(t.lo[d]) : 0.0;
+        K.hi[3 * c + d] = d < K.D ? (double)unfkey(t.hi[d]) : 0.0;
     }
-    const bool unsafe = T.bad[h] != 0 || zeroEps;
+    const bool unsafe = t.bad != 0 || zeroEps;
     const bool dense = !unsafe && (compat || n >= minPts);
     K.unsafe[c] = unsafe ? 1 : 0;
     K.dense[c] = dense ? 1 : 0;
-    K.minIdx[c] = T.minIdx[h];
-    K.minFix[c] = T.minFix[h];
+    K.minIdx[c] = t.minIdx;
+    K.minFix[c] = t.minFix;
     K.hasCore[c] = dense ? 1 : 0;
     K.minCore[c] = INT_MAX;
     K.sb[c] = 0;
     K.se[c] = 0;
     K.need[c] = 0;
     int idx[kReps], m = 0;
-    idx[m++] = T.minIdx[h];
-    if (T.maxIdx[h] != T.minIdx[h]) idx[m++] = T.maxIdx[h];
+    idx[m++] = t.minIdx;
+    if (t.other != t.minIdx) idx[m++] = t.other;
     K.repN[c] = m;
     for (int j = 0; j < m; ++j) {
         double v[3] = {0.0, 0.0, 0.0};
@@ -1449,21 +1506,23 @@ int cell_cluster(Call& c, const Src& S, long long n, double eps, int minPts, boo
     Table T;
     T.mask = cap - 1;
     T.key = (unsigned long long*)c.alloc(cap * sizeof(unsigned long long));
-    T.cnt = (int*)c.alloc(cap * sizeof(int));
-    T.lo = (unsigned*)c.alloc(cap * 3 * sizeof(unsigned));
-    T.hi = (unsigned*)c.alloc(cap * 3 * sizeof(unsigned));
-    T.minIdx = (int*)c.alloc(cap * sizeof(int));
-    T.maxIdx = (int*)c.alloc(cap * sizeof(int));
-    T.minFix = (int*)c.alloc(cap * sizeof(int));
-    T.bad = (int*)c.alloc(cap * sizeof(int));
+    T.st = (CellStats*)c.alloc(cap * sizeof(CellStats));
     int* slot = (int*)c.alloc(n * sizeof(int));
     int* occ = (int*)c.alloc(cap * sizeof(int));
     int* slotCell = (int*)c.alloc(cap * sizeof(int));
     NEED(!c.failed);
     table_init_kernel<<<blocks(cap), kTPB, 0, st>>>(T, (long long)cap);
     note_launch();
-    cells_kernel<Src><<<blocks(n), kTPB, 0, st>>>(S, n, invSide, T, slot, Fout, err);
-    note_launch();
+    {
+        int sms = 0;
+        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device));
+        const long long most = (long long)std::max(sms, 1) * kCellBlocksPerSm;
+        const long long rows = (n + kCellBlock - 1) / kCellBlock, per = (rows + most - 1) / most;
+        CK(cudaFuncSetAttribute(cells_kernel<Src>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BlockCells)));
+        cells_kernel<Src><<<(unsigned)((rows + per - 1) / per), kCellBlock, sizeof(BlockCells), st>>>(
+            S, n, per * kCellBlock, invSide, T, slot, Fout, err);
+        note_launch();
+    }
     occupied_kernel<<<blocks(cap), kTPB, 0, st>>>(T.key, cap, occ);
     note_launch();
     CKL();
