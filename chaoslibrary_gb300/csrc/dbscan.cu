@@ -841,6 +841,7 @@ __global__ void join_all_kernel(const int* nbOwner, const int* nbList, const int
 // one pass over the slots; only those points' features are read.
 struct Sorted {
     double* s[3];
+    float* r[3];  // the same relative to the lower corner of the cell's box, rounded to float (safe cells)
     int* order;
     int* cell;
     unsigned char* core;  // 0 / 1, 2 = not decided yet
@@ -857,7 +858,7 @@ struct Sorted {
 
 template <class Src>
 __global__ void sort_kernel(Src S, long long n, const int* slot, const int* slotCell, const int* begin, int* cursor,
-                            Sorted Q, const unsigned char* dense, int compat) {
+                            Sorted Q, const unsigned char* dense, const double* boxLo, int compat) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     const int h = i < n ? slot[i] : -1;
@@ -877,7 +878,10 @@ __global__ void sort_kernel(Src S, long long n, const int* slot, const int* slot
     S.load(i, v);
 #pragma unroll
     for (int d = 0; d < 3; ++d)
-        if (d < Q.D) Q.s[d][pos] = v[d];
+        if (d < Q.D) {
+            Q.s[d][pos] = v[d];
+            Q.r[d][pos] = (float)(v[d] - boxLo[3 * (long long)c + d]);
+        }
     Q.core[pos] = compat || dense[c] ? 1 : 0;
     if (Q.fix) Q.fix[pos] = S.fix(i) ? 1 : 0;
 }
@@ -911,6 +915,135 @@ __device__ __forceinline__ int node_of(const Cells& K, int c, int p) { return K.
 
 __device__ __forceinline__ bool sorted_cell(const Sorted& Q, int c) { return Q.se[c] > Q.sb[c]; }
 
+// Long scans. A point near a dense cell that it may or may not reach has to be
+// compared with the cell's points, hundreds of thousands in a map whose points
+// settled on one attractor; a warp on its own would read them for
+// milliseconds. Scans of safe cells of more than kLongScan points go to a
+// queue instead (as long as it has room), and long_scan_kernel spreads each
+// over blocks. It reads the points as float offsets from the cell's box: an
+// offset is at most a few cells long and is off by less than 1e-7 of a cell,
+// so a squared distance in float that is clear of eps^2 by 1e-4 decides, and
+// the others are taken in FP64.
+constexpr int kLongScan = 1024;
+constexpr int kScanSplit = 16;  // parts of a queued scan
+constexpr float kFloatOut = 1.0001f, kFloatIn = 0.9999f;
+
+struct ScanQueue {
+    int* point;
+    int* cell;
+    int* count;  // entries asked for; those beyond the capacity were scanned on the spot
+    int cap;
+    __device__ __forceinline__ bool push(int p, int c) const {  // by one lane
+        if (cap == 0) return false;
+        const int k = atomicAdd(count, 1);
+        if (k >= cap) return false;
+        point[k] = p;
+        cell[k] = c;
+        return true;
+    }
+};
+
+// Points per block of 256 threads: the parts of the queued scans, one after
+// the other. labels false: the points of the cell within eps of the point are
+// counted into acc[p] until it reaches minPts. labels true: a core point
+// within eps offers its component's key, the smallest wins in best[p].
+__global__ void __launch_bounds__(256) long_scan_kernel(Sorted Q, Cells K, ScanQueue W, double eps, int minPts,
+                                                        int labels, int* acc, unsigned long long* best, int* parent,
+                                                        const int* compMin) {
+    const int tasks = min(*W.count, W.cap);
+    const float eps2 = (float)(eps * eps);
+    const bool range = eps2 > 1e-30f && eps2 < 1e30f;  // else every distance is taken in FP64
+    for (long long w = blockIdx.x; w < (long long)tasks * kScanSplit; w += gridDim.x) {
+        const int t = (int)(w / kScanSplit), part = (int)(w % kScanSplit);
+        const int p = W.point[t], c = W.cell[t];
+        const int b = Q.sb[c], n = Q.se[c] - b;
+        const int q0 = b + (int)((long long)n * part / kScanSplit), q1 = b + (int)((long long)n * (part + 1) / kScanSplit);
+        double me[3] = {0, 0, 0};
+        Q.load(p, me);
+        float o[3] = {0.f, 0.f, 0.f};
+        for (int d = 0; d < K.D; ++d) o[d] = (float)(me[d] - K.lo[3 * (long long)c + d]);
+        unsigned long long key = 0;
+        if (labels) {
+            const int r = uf_find(parent, c);
+            key = ((unsigned long long)(unsigned)compMin[r] << 32) | (unsigned)r;
+        }
+        const bool allCore = K.dense[c] != 0;
+        int found = 0;
+        constexpr int kStep = 4;  // points in flight per thread
+        for (int q = q0 + threadIdx.x; q - (int)threadIdx.x < q1; q += kStep * blockDim.x) {
+            // (the break is uniform over the warp: its lanes read the same word)
+            if (labels ? __ldcg(best + p) <= key : __ldcg(acc + p) >= minPts) break;
+            float d2[kStep];
+#pragma unroll
+            for (int k = 0; k < kStep; ++k) {
+                const int i = q + k * blockDim.x;
+                d2[k] = __int_as_float(0x7f800000);
+                if (i < q1) {
+                    float sum = 0.f;
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        if (d >= K.D) continue;
+                        const float df = o[d] - Q.r[d][i];
+                        sum = fmaf(df, df, sum);
+                    }
+                    d2[k] = range ? sum : __int_as_float(0x7fc00000);
+                }
+            }
+            int hits = 0;
+#pragma unroll
+            for (int k = 0; k < kStep; ++k) {
+                if (d2[k] > eps2 * kFloatOut) continue;
+                const int i = q + k * blockDim.x;
+                bool in = d2[k] < eps2 * kFloatIn;
+                if (!in) {
+                    double v[3];
+                    Q.load(i, v);
+                    in = within_eps(dist2(me, v, K.D), eps);
+                }
+                if (in && labels && !allCore) in = Q.core[i] == 1;
+                hits += in ? 1 : 0;
+            }
+            found = (int)__reduce_add_sync(0xffffffffu, (unsigned)hits);
+            if (found == 0) continue;
+            if ((threadIdx.x & 31) == 0) {
+                if (labels) atomicMin(best + p, key);
+                else atomicAdd(acc + p, found);
+            }
+            if (labels) break;
+        }
+    }
+}
+
+// After the queued scans: the core flags of the undecided points (those marked
+// 2), and their cells' links to the dense cells wholly within eps.
+__global__ void core_finish_kernel(Sorted Q, Cells K, const int* nbStart, const int* nbList, int M1, double eps,
+                                   int minPts, const int* acc, int* parent) {
+    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (w >= M1) return;
+    const int p = (int)w;
+    if (Q.core[p] != 2) return;
+    const int c = Q.cell[p];
+    const bool core = acc[p] >= minPts;
+    __syncwarp();  // every lane has read the mark before lane 0 clears it
+    if (lane == 0) Q.core[p] = core ? 1 : 0;
+    if (!core) return;
+    if (lane == 0 && !K.unsafe[c]) {
+        atomicOr(&K.hasCore[c], 1);
+        atomicMin(&K.minCore[c], Q.order[p]);
+    }
+    double me[3] = {0, 0, 0};
+    Q.load(p, me);
+    const double eps2 = eps * eps;
+    for (int e = nbStart[c] + lane; e < nbStart[c + 1]; e += 32) {
+        const int b = nbList[e];
+        if (K.unsafe[b] || !K.dense[b]) continue;
+        double near2, far2;
+        box_dist2(me, K.lo + 3 * (long long)b, K.hi + 3 * (long long)b, K.D, near2, far2);
+        if (near2 <= eps2 * kBoxOut && far2 < eps2 * kBoxIn) uf_unite(parent, node_of(K, c, p), b);
+    }
+}
+
 // Warp per sorted point of a cell that is not dense (textbook mode), in
 // [0, M1): the lanes classify the neighbour cells (at most 124, four per
 // lane) by their boxes -- beyond eps: nothing; wholly within eps: counted
@@ -919,11 +1052,11 @@ __device__ __forceinline__ bool sorted_cell(const Sorted& Q, int c) { return Q.s
 // are scanned 32 points at a time until minPts. A point that stays below
 // minPts with a lower-bound cell is left undecided (core = 2) and those cells
 // are marked for the second sort. redo: only the undecided points, counted
-// exactly; one found core joins the dense cells wholly within eps of it.
+// exactly into acc, long scans through the queue; core_finish_kernel decides.
 constexpr int kNbPerLane = 4;  // (2R+1)^3 - 1 = 124 neighbour cells at most
 
 __global__ void core_kernel(Sorted Q, Cells K, const int* nbStart, const int* nbList, int M1, double eps, int minPts,
-                            int redo, int* parent) {
+                            int redo, ScanQueue W, int* acc) {
     const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (w >= M1) return;
@@ -980,16 +1113,38 @@ __global__ void core_kernel(Sorted Q, Cells K, const int* nbStart, const int* nb
         }
     };
     if (K.unsafe[c] && cnt < minPts) scan_cell(c);
+    unsigned queued[kNbPerLane];  // long scans left to the queue (redo)
 #pragma unroll
     for (int j = 0; j < kNbPerLane; ++j) {
         unsigned m = __ballot_sync(0xffffffffu, cls[j] == 2);
+        queued[j] = 0;
         while (m && cnt < minPts) {
             const int src = __ffs(m) - 1;
             m &= m - 1;
-            scan_cell(nbList[e0 + src + 32 * j]);
+            const int b = nbList[e0 + src + 32 * j];
+            if (redo && !K.unsafe[b] && Q.se[b] - Q.sb[b] > kLongScan) queued[j] |= 1u << src;
+            else scan_cell(b);
         }
     }
-    const int core = cnt >= minPts ? 1 : (inexact && !redo ? 2 : 0);
+    if (redo) {  // core_finish_kernel decides, after the queued scans
+        bool full = false;
+        if (lane == 0) acc[p] = cnt;
+#pragma unroll
+        for (int j = 0; j < kNbPerLane; ++j)
+            while (queued[j] && cnt < minPts) {
+                const int src = __ffs(queued[j]) - 1;
+                queued[j] &= queued[j] - 1;
+                const int b = nbList[e0 + src + 32 * j];
+                if (!full) full = __shfl_sync(0xffffffffu, lane == 0 && !W.push(p, b), 0);
+                if (full) {
+                    const int before = cnt;
+                    scan_cell(b);
+                    if (lane == 0) atomicAdd(acc + p, cnt - before);
+                }
+            }
+        return;
+    }
+    const int core = cnt >= minPts ? 1 : (inexact ? 2 : 0);
     if (lane == 0) {
         Q.core[p] = (unsigned char)core;
         if (core == 1 && !K.unsafe[c]) {
@@ -998,11 +1153,8 @@ __global__ void core_kernel(Sorted Q, Cells K, const int* nbStart, const int* nb
         }
     }
 #pragma unroll
-    for (int j = 0; j < kNbPerLane; ++j) {
+    for (int j = 0; j < kNbPerLane; ++j)
         if (cls[j] == 3 && core == 2) K.need[nbList[e0 + lane + 32 * j]] = 1;  // to be sorted
-        if (cls[j] == 1 && redo && core == 1 && K.dense[nbList[e0 + lane + 32 * j]])
-            uf_unite(parent, node_of(K, c, p), nbList[e0 + lane + 32 * j]);
-    }
 }
 
 // Warp per sorted point of a cell that is not dense, in [0, M1), after the
@@ -1316,10 +1468,12 @@ __global__ void labels_kernel(const int* slot, const int* slotCell, long long n,
 // point takes its component's label; a border point the component with the
 // smallest core index among the core points within eps (lanes settle the
 // neighbour cells by box or representatives, the rest are scanned by the
-// warp, a safe cell only while it could still lower the answer); the rest
-// are noise (-1).
+// warp or, the long ones, through the queue, a safe cell only while it could
+// still lower the answer); the rest are noise (-1). border_labels_kernel
+// writes those that are not core.
 __global__ void sorted_labels_kernel(Sorted Q, Cells K, const int* nbStart, const int* nbList, int M1, double eps,
-                                     int* parent, const int* compMin, const int* compLabel, int* labels) {
+                                     int* parent, const int* compMin, const int* compLabel, int* labels, ScanQueue W,
+                                     unsigned long long* bests) {
     const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (w >= M1) return;
@@ -1393,16 +1547,44 @@ __global__ void sorted_labels_kernel(Sorted Q, Cells K, const int* nbStart, cons
         }
     };
     if (K.unsafe[c]) scan(c);
+    bool full = false;
+    unsigned queued[kNbPerLane];  // long scans left to the queue
 #pragma unroll
     for (int j = 0; j < kNbPerLane; ++j) {
         unsigned m = __ballot_sync(0xffffffffu, scanIt[j]);
+        queued[j] = 0;
         while (m) {
             const int src = __ffs(m) - 1;
             m &= m - 1;
-            scan(nbList[e0 + src + 32 * j]);
+            const int b = nbList[e0 + src + 32 * j];
+            if (!K.unsafe[b] && Q.se[b] - Q.sb[b] > kLongScan) queued[j] |= 1u << src;
+            else scan(b);
         }
     }
-    if (lane == 0) labels[Q.order[p]] = best == ~0ull ? -1 : compLabel[(int)(best & 0xffffffffull)];
+    if (lane == 0) bests[p] = best;
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < kNbPerLane; ++j)
+        while (queued[j]) {
+            const int src = __ffs(queued[j]) - 1;
+            queued[j] &= queued[j] - 1;
+            const int b = nbList[e0 + src + 32 * j];
+            if (key_of(uf_find(parent, b)) >= best) continue;  // could not lower the answer
+            if (!full) full = __shfl_sync(0xffffffffu, lane == 0 && !W.push(p, b), 0);
+            if (full) {
+                scan(b);
+                if (lane == 0) atomicMin(bests + p, best);
+            }
+        }
+}
+
+// After the queued scans: the labels of the points that are not core.
+__global__ void border_labels_kernel(Sorted Q, int M1, const unsigned long long* bests, const int* compLabel,
+                                     int* labels) {
+    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= M1 || Q.core[p] == 1) return;
+    const unsigned long long best = bests[p];
+    labels[Q.order[p]] = best == ~0ull ? -1 : compLabel[(int)(best & 0xffffffffull)];
 }
 
 #define CK(x)                                                   \
@@ -1513,9 +1695,9 @@ int cell_cluster(Call& c, const Src& S, long long n, double eps, int minPts, boo
     NEED(!c.failed);
     table_init_kernel<<<blocks(cap), kTPB, 0, st>>>(T, (long long)cap);
     note_launch();
+    int sms = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device));
     {
-        int sms = 0;
-        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device));
         const long long most = (long long)std::max(sms, 1) * kCellBlocksPerSm;
         const long long rows = (n + kCellBlock - 1) / kCellBlock, per = (rows + most - 1) / most;
         CK(cudaFuncSetAttribute(cells_kernel<Src>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BlockCells)));
@@ -1625,7 +1807,10 @@ int cell_cluster(Call& c, const Src& S, long long n, double eps, int minPts, boo
     Q.cell = (int*)c.alloc((size_t)(n + 1) * sizeof(int));
     Q.core = (unsigned char*)c.alloc((size_t)n + 1);
     Q.fix = compat ? (unsigned char*)c.alloc((size_t)n + 1) : nullptr;
-    for (int d = 0; d < 3; ++d) Q.s[d] = d < D ? (double*)c.alloc((size_t)(n + 1) * sizeof(double)) : nullptr;
+    for (int d = 0; d < 3; ++d) {
+        Q.s[d] = d < D ? (double*)c.alloc((size_t)(n + 1) * sizeof(double)) : nullptr;
+        Q.r[d] = d < D ? (float*)c.alloc((size_t)(n + 1) * sizeof(float)) : nullptr;
+    }
     Q.sb = K.sb;
     Q.se = K.se;
     Q.D = D;
@@ -1640,7 +1825,7 @@ int cell_cluster(Call& c, const Src& S, long long n, double eps, int minPts, boo
             phase_begin_kernel<<<blocks(C), kTPB, 0, st>>>(C, cursor, take, 0, begin, K.sb, K.se, K.cnt);
             note_launch();
             CK(cudaMemsetAsync(cursor, 0, (size_t)C * sizeof(int), st));
-            sort_kernel<Src><<<blocks(n), kTPB, 0, st>>>(S, n, slot, slotCell, begin, cursor, Q, K.dense,
+            sort_kernel<Src><<<blocks(n), kTPB, 0, st>>>(S, n, slot, slotCell, begin, cursor, Q, K.dense, K.lo,
                                                          compat ? 1 : 0);
             note_launch();
             CKL();
@@ -1650,7 +1835,7 @@ int cell_cluster(Call& c, const Src& S, long long n, double eps, int minPts, boo
     if (M1 > 0) {
         if (!compat) {
             core_kernel<<<blocks((long long)M1 * 32), kTPB, 0, st>>>(Q, K, nbStart, nbList, M1, eps, minPts, 0,
-                                                                     nullptr);
+                                                                     ScanQueue{}, nullptr);
             note_launch();
         }
         dense_links_kernel<<<blocks((long long)M1 * 32), kTPB, 0, st>>>(Q, K, nbStart, nbList, M1, eps, parentC,
@@ -1674,7 +1859,7 @@ int cell_cluster(Call& c, const Src& S, long long n, double eps, int minPts, boo
             phase_begin_kernel<<<blocks(C), kTPB, 0, st>>>(C, cursor, take, M1, begin, K.sb, K.se, K.cnt);
             note_launch();
             CK(cudaMemsetAsync(cursor, 0, (size_t)C * sizeof(int), st));
-            sort_kernel<Src><<<blocks(n), kTPB, 0, st>>>(S, n, slot, slotCell, begin, cursor, Q, K.dense,
+            sort_kernel<Src><<<blocks(n), kTPB, 0, st>>>(S, n, slot, slotCell, begin, cursor, Q, K.dense, K.lo,
                                                          compat ? 1 : 0);
             note_launch();
             CKL();
@@ -1696,9 +1881,34 @@ int cell_cluster(Call& c, const Src& S, long long n, double eps, int minPts, boo
     iota_kernel<<<blocks(N + 1), kTPB, 0, st>>>(parent, N + 1);
     note_launch();
     if (C > 0) CK(cudaMemcpyAsync(parent, parentC, (size_t)C * sizeof(int), cudaMemcpyDeviceToDevice, st));
+    // the queue of the long scans, and what they find per sorted point: a
+    // count, later the best component's key
+    ScanQueue W{};
+    unsigned long long* found = nullptr;
+    const unsigned scanBlocks = (unsigned)(8 * std::max(sms, 1));
+    if (M1 > 0 && M2 > 0) {  // (cells are scanned exactly only once the second phase has sorted them)
+        W.cap = std::max(4096, M1);
+        W.point = (int*)c.alloc((size_t)W.cap * sizeof(int));
+        W.cell = (int*)c.alloc((size_t)W.cap * sizeof(int));
+        W.count = (int*)c.alloc(2 * sizeof(int));
+        NEED(!c.failed);
+        CK(cudaMemsetAsync(W.count, 0, 2 * sizeof(int), st));
+    }
+    if (M1 > 0) {
+        found = (unsigned long long*)c.alloc((size_t)M1 * sizeof(unsigned long long));
+        NEED(found);
+    }
     if (M1 > 0 && !compat) {  // the undecided counts, exactly (their neighbours are sorted now)
-        core_kernel<<<blocks((long long)M1 * 32), kTPB, 0, st>>>(Q, K, nbStart, nbList, M1, eps, minPts, 1,
-                                                                 parent);
+        core_kernel<<<blocks((long long)M1 * 32), kTPB, 0, st>>>(Q, K, nbStart, nbList, M1, eps, minPts, 1, W,
+                                                                 (int*)found);
+        note_launch();
+        if (W.cap > 0) {
+            long_scan_kernel<<<scanBlocks, 256, 0, st>>>(Q, K, W, eps, minPts, 0, (int*)found, nullptr, nullptr,
+                                                         nullptr);
+            note_launch();
+        }
+        core_finish_kernel<<<blocks((long long)M1 * 32), kTPB, 0, st>>>(Q, K, nbStart, nbList, M1, eps, minPts,
+                                                                        (const int*)found, parent);
         note_launch();
         CKL();
     }
@@ -1742,8 +1952,15 @@ int cell_cluster(Call& c, const Src& S, long long n, double eps, int minPts, boo
     labels_kernel<<<blocks(n), kTPB, 0, st>>>(slot, slotCell, n, K.dense, cellLabel, compat ? 1 : 0, labels);
     note_launch();
     if (M1 > 0) {
+        if (W.cap > 0) ++W.count;  // the second counter
         sorted_labels_kernel<<<blocks((long long)M1 * 32), kTPB, 0, st>>>(Q, K, nbStart, nbList, M1, eps, parent,
-                                                                          compMin, compLabel, labels);
+                                                                          compMin, compLabel, labels, W, found);
+        note_launch();
+        if (W.cap > 0) {
+            long_scan_kernel<<<scanBlocks, 256, 0, st>>>(Q, K, W, eps, minPts, 1, nullptr, found, parent, compMin);
+            note_launch();
+        }
+        border_labels_kernel<<<blocks(M1), kTPB, 0, st>>>(Q, M1, found, compLabel, labels);
         note_launch();
     }
     CKL();
