@@ -961,7 +961,9 @@ __global__ void __launch_bounds__(256) long_scan_kernel(Sorted Q, Cells K, ScanQ
         double me[3] = {0, 0, 0};
         Q.load(p, me);
         float o[3] = {0.f, 0.f, 0.f};
-        for (int d = 0; d < K.D; ++d) o[d] = (float)(me[d] - K.lo[3 * (long long)c + d]);
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+            if (d < K.D) o[d] = (float)(me[d] - K.lo[3 * (long long)c + d]);
         unsigned long long key = 0;
         if (labels) {
             const int r = uf_find(parent, c);
@@ -1272,8 +1274,11 @@ constexpr int kCrossPasses = 3;
 __constant__ int kPassOuter[kCrossPasses] = {2, 32, 0x7fffffff};
 __constant__ int kPassChunks[kCrossPasses] = {2, 8, 0x7fffffff};
 
+constexpr long long kLongPair = 1 << 16;  // point pairs of two cells that one warp takes on in the last pass
+
 __global__ void cross_cell_kernel(Sorted Q, Cells K, const int* nbOwner, const int* nbList, long long E,
-                                  const unsigned char* st, double eps, int* parent, int pass, unsigned char* deferred) {
+                                  const unsigned char* st, double eps, int* parent, int pass, unsigned char* deferred,
+                                  int* longPairs, int* nLong) {
     const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (w >= E) return;
@@ -1302,6 +1307,10 @@ __global__ void cross_cell_kernel(Sorted Q, Cells K, const int* nbOwner, const i
         const int t = ca;
         ca = cb;
         cb = t;
+    }
+    if (last && safe && (long long)(Q.se[ca] - Q.sb[ca]) * (Q.se[cb] - Q.sb[cb]) > kLongPair) {
+        if (lane == 0) longPairs[atomicAdd(nLong, 1)] = (int)w;  // long_pairs_kernel
+        return;
     }
     const double* lo = K.lo + 3 * (long long)cb;
     const double* hi = K.hi + 3 * (long long)cb;
@@ -1361,6 +1370,82 @@ __global__ void cross_cell_kernel(Sorted Q, Cells K, const int* nbOwner, const i
         }
     }
     if (cut && lane == 0) deferred[w] = 1;
+}
+
+// The listed pairs of safe cells that the passes left apart and whose points
+// make more than kLongPair pairs: the larger cell's points, a block of them
+// at a time, against all of the smaller cell's, as long as the two are in two
+// components. One warp for a whole pair took 9.5 ms where a few points face a
+// cell of 250,000 just out of reach. Distances as in long_scan_kernel.
+__global__ void __launch_bounds__(256) long_pairs_kernel(Sorted Q, Cells K, const int* nbOwner, const int* nbList,
+                                                         const int* longPairs, const int* nLong, double eps,
+                                                         int* parent) {
+    __shared__ float so[3][256];
+    __shared__ int apart;
+    const int n = *nLong;
+    const float eps2 = (float)(eps * eps);
+    const bool range = eps2 > 1e-30f && eps2 < 1e30f;
+    // all blocks on one pair, or at least 16 on each of many
+    const int team = n > 0 ? max(16, (int)gridDim.x / n) : 1, teams = max(1, (int)gridDim.x / team);
+    if ((int)blockIdx.x >= team * teams) return;
+    for (int t = blockIdx.x / team; t < n; t += teams) {
+        int ca = nbOwner[longPairs[t]], cb = nbList[longPairs[t]];
+        if (Q.se[ca] - Q.sb[ca] > Q.se[cb] - Q.sb[cb]) {
+            const int x = ca;
+            ca = cb;
+            cb = x;
+        }
+        const double* lo = K.lo + 3 * (long long)cb;
+        const bool coreA = K.dense[ca] != 0, coreB = K.dense[cb] != 0;
+        const int endA = Q.se[ca], endB = Q.se[cb];
+        for (int q0 = Q.sb[cb] + (int)(blockIdx.x % team) * 256; q0 < endB; q0 += team * 256) {
+            __syncthreads();
+            if (threadIdx.x == 0) apart = uf_find(parent, ca) != uf_find(parent, cb);
+            __syncthreads();
+            if (!apart) break;
+            const int q = q0 + threadIdx.x;
+            const bool mine = q < endB && (coreB || Q.core[q] == 1);
+            float r[3] = {0.f, 0.f, 0.f};
+            if (mine) {
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    if (d < K.D) r[d] = Q.r[d][q];
+            }
+            bool hit = false;
+            for (int p0 = Q.sb[ca]; p0 < endA; p0 += 256) {
+                const int p = p0 + threadIdx.x;
+                __syncthreads();
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    if (d >= K.D) continue;
+                    so[d][threadIdx.x] = p < endA && (coreA || Q.core[p] == 1) ? (float)(Q.s[d][p] - lo[d])
+                                                                              : __int_as_float(0x7f800000);
+                }
+                __syncthreads();
+                const int m = min(256, endA - p0);
+                for (int k = 0; k < m && mine && !hit; ++k) {
+                    float sum = 0.f;
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        if (d >= K.D) continue;
+                        const float df = r[d] - so[d][k];
+                        sum = fmaf(df, df, sum);
+                    }
+                    if (sum > eps2 * kFloatOut && (range || sum == __int_as_float(0x7f800000))) continue;
+                    if (range && sum < eps2 * kFloatIn) {
+                        hit = true;
+                        continue;
+                    }
+                    double a[3] = {0, 0, 0}, b[3] = {0, 0, 0};
+                    Q.load(p0 + k, a);
+                    Q.load(q, b);
+                    hit = (coreA || Q.core[p0 + k] == 1) && within_eps(dist2(a, b, K.D), eps);
+                }
+                if (__syncthreads_or(hit)) break;
+            }
+            if (hit) uf_unite(parent, ca, cb);
+        }
+    }
 }
 
 // ---- step 6: components and labels ------------------------------------------------
@@ -1920,12 +2005,17 @@ int cell_cluster(Call& c, const Src& S, long long n, double eps, int minPts, boo
         unsafe_cell_kernel<<<blocks((long long)C * 32), kTPB, 0, st>>>(Q, K, eps, parent);
         note_launch();
     }
-    if (E > 0 && M > 0)
+    if (E > 0 && M > 0) {
+        int* nLong = nOpen;  // (the open list has been read: its memory serves the long pairs)
+        CK(cudaMemsetAsync(nLong, 0, sizeof(int), st));
         for (int pass = 0; pass < kCrossPasses; ++pass) {
             cross_cell_kernel<<<blocks((long long)E * 32), kTPB, 0, st>>>(Q, K, nbOwner, nbList, E, pst, eps, parent,
-                                                                          pass, deferred);
+                                                                          pass, deferred, openList, nLong);
             note_launch();
         }
+        long_pairs_kernel<<<scanBlocks, 256, 0, st>>>(Q, K, nbOwner, nbList, openList, nLong, eps, parent);
+        note_launch();
+    }
     CKL();
     // components, numbered
     CK(cudaMemsetAsync(nRoots, 0, sizeof(int), st));
