@@ -209,6 +209,20 @@ __device__ __forceinline__ void box_dist2(const double* v, const double* lo, con
     }
 }
 
+// ---- counts the pipeline keeps on the device ---------------------------------------
+// The sizes of the later steps stay in device memory: their kernels read them
+// (a fixed grid loops over the work), and the host waits once, for the number
+// of cells.
+enum Count {
+    kCells, kErr, kEntries, kOpen, kJoinedCount, kSparse, kNeeded, kRoots, kActive, kLong, kScanA, kScanB, kCounts
+};
+constexpr int kLoopBlocksPerSm = 8;  // blocks of kTPB threads of a looping kernel
+
+__device__ __forceinline__ long long first_warp() { return ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; }
+__device__ __forceinline__ long long warp_stride() { return ((long long)gridDim.x * blockDim.x) >> 5; }
+// sorted points, and nodes of the union-find over cells and sorted points
+__device__ __forceinline__ int sorted_points(const int* counts) { return counts[kSparse] + counts[kNeeded]; }
+
 // ---- union-find (parent[v] <= v) --------------------------------------------
 __device__ __forceinline__ int uf_find(int* parent, int x) {
     int cur = __ldcg(parent + x);
@@ -736,11 +750,13 @@ __device__ __forceinline__ bool rep_within(const Cells& K, int b, const double* 
 
 // Thread per neighbour entry (owner < neighbour): the box tests; pairs of
 // dense cells that the boxes leave open are listed for the representatives.
-__global__ void pair_kernel(Cells K, const int* nbOwner, const int* nbList, long long E, double eps,
-                            unsigned char* st, int* open, int* nOpen, int* joined, int* nJoined) {
+__global__ void pair_kernel(Cells K, const int* nbOwner, const int* nbList, double eps, unsigned char* st, int* open,
+                            int* joined, int* active, unsigned char* openE, unsigned char* settledE,
+                            unsigned char* deferred, int* counts) {
     const long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    bool take = false, join = false;
-    if (w < E) {
+    bool take = false, join = false, act = false;
+    if (w < counts[kEntries]) {
+        openE[w] = settledE[w] = deferred[w] = 0;
         const int a = nbOwner[w], b = nbList[w];
         unsigned char state = kFar;
         if (b > a) {
@@ -758,22 +774,21 @@ __global__ void pair_kernel(Cells K, const int* nbOwner, const int* nbList, long
                 }
             } else {
                 state = !K.unsafe[a] && !K.unsafe[b] && span2 < eps2 * kBoxIn ? kWhole : kPoints;
+                act = state == kPoints;
             }
         }
         st[w] = state;
     }
-    list_append(take, (int)w, open, nOpen);
-    list_append(join, (int)w, joined, nJoined);
+    list_append(take, (int)w, open, counts + kOpen);
+    list_append(join, (int)w, joined, counts + kJoinedCount);
+    list_append(act, (int)w, active, counts + kActive);
 }
 
 // Warp per listed pair of dense cells: the lanes share the representative
 // pairs; one within eps marks the two cells joined.
-__global__ void rep_pairs_kernel(Cells K, const int* nbOwner, const int* nbList, const int* open, int nOpen,
-                                 double eps, unsigned char* st, int* joined, int* nJoined) {
-    const long long wi = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__device__ __forceinline__ void rep_pair(const Cells& K, const int* nbOwner, const int* nbList, int w, double eps,
+                                         unsigned char* st, int* joined, int* nJoined) {
     const int lane = threadIdx.x & 31;
-    if (wi >= nOpen) return;
-    const int w = open[wi];
     const int a = nbOwner[w], b = nbList[w];
     const int na = K.repN[a], nb = K.repN[b];
     bool hit = false;
@@ -786,6 +801,12 @@ __global__ void rep_pairs_kernel(Cells K, const int* nbOwner, const int* nbList,
         st[w] = kJoined;
         joined[atomicAdd(nJoined, 1)] = w;
     }
+}
+__global__ void rep_pairs_kernel(Cells K, const int* nbOwner, const int* nbList, const int* open, double eps,
+                                 unsigned char* st, int* joined, int* counts) {
+    const int n = counts[kOpen];
+    for (long long k = first_warp(); k < n; k += warp_stride())
+        rep_pair(K, nbOwner, nbList, open[k], eps, st, joined, counts + kJoinedCount);
 }
 
 // The components of the dense cells over the joined pairs. Thousands of
@@ -858,7 +879,8 @@ struct Sorted {
 
 template <class Src>
 __global__ void sort_kernel(Src S, long long n, const int* slot, const int* slotCell, const int* begin, int* cursor,
-                            Sorted Q, const unsigned char* dense, const double* boxLo, int compat) {
+                            Sorted Q, const unsigned char* dense, const double* boxLo, int compat, const int* total) {
+    if (*total == 0) return;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     const int h = i < n ? slot[i] : -1;
@@ -886,10 +908,11 @@ __global__ void sort_kernel(Src S, long long n, const int* slot, const int* slot
     if (Q.fix) Q.fix[pos] = S.fix(i) ? 1 : 0;
 }
 
-__global__ void phase_begin_kernel(int C, const int* scan, const int* take, int offset, int* begin, int* sb, int* se,
+__global__ void phase_begin_kernel(int C, int* scan, const int* take, const int* before, int* begin, int* sb, int* se,
                                    const int* cnt) {
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
+    const int offset = before ? *before : 0;
     if (take[c]) {
         begin[c] = offset + scan[c];
         sb[c] = offset + scan[c];
@@ -897,6 +920,7 @@ __global__ void phase_begin_kernel(int C, const int* scan, const int* take, int 
     } else {
         begin[c] = -1;
     }
+    scan[c] = 0;  // from here on the sort's cursor
 }
 
 __global__ void take_sparse_kernel(Cells K, int* take) {
@@ -1018,11 +1042,9 @@ __global__ void __launch_bounds__(256) long_scan_kernel(Sorted Q, Cells K, ScanQ
 
 // After the queued scans: the core flags of the undecided points (those marked
 // 2), and their cells' links to the dense cells wholly within eps.
-__global__ void core_finish_kernel(Sorted Q, Cells K, const int* nbStart, const int* nbList, int M1, double eps,
-                                   int minPts, const int* acc, int* parent) {
-    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__device__ __forceinline__ void core_finish_point(Sorted Q, Cells K, const int* nbStart, const int* nbList, double eps,
+                                   int minPts, const int* acc, int* parent, long long w) {
     const int lane = threadIdx.x & 31;
-    if (w >= M1) return;
     const int p = (int)w;
     if (Q.core[p] != 2) return;
     const int c = Q.cell[p];
@@ -1046,6 +1068,13 @@ __global__ void core_finish_kernel(Sorted Q, Cells K, const int* nbStart, const 
     }
 }
 
+__global__ void core_finish_kernel(Sorted Q, Cells K, const int* nbStart, const int* nbList, double eps,
+                                   int minPts, const int* acc, int* parent, const int* counts) {
+    const int n = counts[kSparse];
+    for (long long w = first_warp(); w < n; w += warp_stride())
+        core_finish_point(Q, K, nbStart, nbList, eps, minPts, acc, parent, w);
+}
+
 // Warp per sorted point of a cell that is not dense (textbook mode), in
 // [0, M1): the lanes classify the neighbour cells (at most 124, four per
 // lane) by their boxes -- beyond eps: nothing; wholly within eps: counted
@@ -1057,11 +1086,9 @@ __global__ void core_finish_kernel(Sorted Q, Cells K, const int* nbStart, const 
 // exactly into acc, long scans through the queue; core_finish_kernel decides.
 constexpr int kNbPerLane = 4;  // (2R+1)^3 - 1 = 124 neighbour cells at most
 
-__global__ void core_kernel(Sorted Q, Cells K, const int* nbStart, const int* nbList, int M1, double eps, int minPts,
-                            int redo, ScanQueue W, int* acc) {
-    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__device__ __forceinline__ void core_point(Sorted Q, Cells K, const int* nbStart, const int* nbList, double eps, int minPts,
+                            int redo, ScanQueue W, int* acc, long long w) {
     const int lane = threadIdx.x & 31;
-    if (w >= M1) return;
     const int p = (int)w;
     if (redo && Q.core[p] != 2) return;
     const int c = Q.cell[p];
@@ -1159,6 +1186,13 @@ __global__ void core_kernel(Sorted Q, Cells K, const int* nbStart, const int* nb
         if (cls[j] == 3 && core == 2) K.need[nbList[e0 + lane + 32 * j]] = 1;  // to be sorted
 }
 
+__global__ void core_kernel(Sorted Q, Cells K, const int* nbStart, const int* nbList, double eps, int minPts,
+                            int redo, ScanQueue W, int* acc, const int* counts) {
+    const int n = counts[kSparse];
+    for (long long w = first_warp(); w < n; w += warp_stride())
+        core_point(Q, K, nbStart, nbList, eps, minPts, redo, W, acc, w);
+}
+
 // Warp per sorted point of a cell that is not dense, in [0, M1), after the
 // core flags, lanes over the neighbour cells: a core point of a safe cell
 // joins its cell to every dense neighbour that is whole within eps of it or
@@ -1168,11 +1202,9 @@ __global__ void core_kernel(Sorted Q, Cells K, const int* nbStart, const int* nb
 // scan (partly within eps, no representative within eps), and a point of an
 // unsafe cell every dense neighbour within reach: those are sorted in the
 // second pass.
-__global__ void dense_links_kernel(Sorted Q, Cells K, const int* nbStart, const int* nbList, int M1, double eps,
-                                   int* parent, unsigned char* openE, unsigned char* settledE) {
-    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__device__ __forceinline__ void dense_links_point(Sorted Q, Cells K, const int* nbStart, const int* nbList, double eps,
+                                   int* parent, unsigned char* openE, unsigned char* settledE, long long w) {
     const int lane = threadIdx.x & 31;
-    if (w >= M1) return;
     const int p = (int)w;
     const int c = Q.cell[p];
     const int core = Q.core[p];
@@ -1204,18 +1236,26 @@ __global__ void dense_links_kernel(Sorted Q, Cells K, const int* nbStart, const 
     }
 }
 
+__global__ void dense_links_kernel(Sorted Q, Cells K, const int* nbStart, const int* nbList, double eps,
+                                   int* parent, unsigned char* openE, unsigned char* settledE, const int* counts) {
+    const int n = counts[kSparse];
+    for (long long w = first_warp(); w < n; w += warp_stride())
+        dense_links_point(Q, K, nbStart, nbList, eps, parent, openE, settledE, w);
+}
+
 // Entry pass after the shortcuts' unions: two dense cells still apart, and
 // open entries of a cell whose core points did not reach a dense neighbour,
 // get point tests (both cells sorted) when they are in two components; pairs
 // with an unsafe cell are tested point by point.
-__global__ void open_pairs_kernel(Cells K, const int* nbOwner, const int* nbList, long long E, int* parent,
-                                  unsigned char* st, const unsigned char* openE, const unsigned char* settledE) {
+__global__ void open_pairs_kernel(Cells K, const int* nbOwner, const int* nbList, int* parent, unsigned char* st,
+                                  const unsigned char* openE, const unsigned char* settledE, int* active, int* counts) {
     const long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= E) return;
+    if (w >= counts[kEntries]) return;
     const int a = nbOwner[w], b = nbList[w];
     if (st[w] == kDenseOpen) {
         if (uf_find(parent, a) != uf_find(parent, b)) {
             st[w] = kDensePts;
+            active[atomicAdd(counts + kActive, 1)] = (int)w;
             K.need[a] = 1;
             K.need[b] = 1;
         } else {
@@ -1231,10 +1271,10 @@ __global__ void open_pairs_kernel(Cells K, const int* nbOwner, const int* nbList
 
 // ---- step 5: unions ------------------------------------------------------------
 
-__global__ void whole_pairs_kernel(Cells K, const int* nbOwner, const int* nbList, long long E,
-                                   const unsigned char* st, int* parent) {
+__global__ void whole_pairs_kernel(Cells K, const int* nbOwner, const int* nbList, const unsigned char* st, int* parent,
+                                   const int* counts) {
     const long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= E || st[w] != kWhole) return;
+    if (w >= counts[kEntries] || st[w] != kWhole) return;
     const int a = nbOwner[w], b = nbList[w];
     if (K.hasCore[a] && K.hasCore[b]) uf_unite(parent, a, b);
 }
@@ -1258,7 +1298,7 @@ __global__ void unsafe_cell_kernel(Sorted Q, Cells K, double eps, int* parent) {
     }
 }
 
-// warp per entry in state kPoints / kDensePts whose two cells are sorted:
+// warp per listed entry (state kPoints / kDensePts) whose two cells are sorted:
 // unite the two cells' core points if any core pair is within eps. The
 // smaller cell's points are walked one by one, the larger cell's 32 at a
 // time.
@@ -1276,13 +1316,9 @@ __constant__ int kPassChunks[kCrossPasses] = {2, 8, 0x7fffffff};
 
 constexpr long long kLongPair = 1 << 16;  // point pairs of two cells that one warp takes on in the last pass
 
-__global__ void cross_cell_kernel(Sorted Q, Cells K, const int* nbOwner, const int* nbList, long long E,
-                                  const unsigned char* st, double eps, int* parent, int pass, unsigned char* deferred,
-                                  int* longPairs, int* nLong) {
-    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__device__ __forceinline__ void cross_cells(Sorted Q, Cells K, const int* nbOwner, const int* nbList,                                   double eps, int* parent, int pass, unsigned char* deferred,
+                                  int* longPairs, int* nLong, long long w) {
     const int lane = threadIdx.x & 31;
-    if (w >= E) return;
-    if (st[w] != kPoints && st[w] != kDensePts) return;
     int ca = nbOwner[w], cb = nbList[w];
     if (!sorted_cell(Q, ca) || !sorted_cell(Q, cb)) return;
     const bool last = pass == kCrossPasses - 1;
@@ -1372,6 +1408,13 @@ __global__ void cross_cell_kernel(Sorted Q, Cells K, const int* nbOwner, const i
     if (cut && lane == 0) deferred[w] = 1;
 }
 
+__global__ void cross_cell_kernel(Sorted Q, Cells K, const int* nbOwner, const int* nbList,                                   double eps, int* parent, int pass, unsigned char* deferred,
+                                  int* longPairs, int* nLong, const int* active, const int* counts) {
+    const int n = counts[kActive];
+    for (long long k = first_warp(); k < n; k += warp_stride())
+        cross_cells(Q, K, nbOwner, nbList, eps, parent, pass, deferred, longPairs, nLong, active[k]);
+}
+
 // The listed pairs of safe cells that the passes left apart and whose points
 // make more than kLongPair pairs: the larger cell's points, a block of them
 // at a time, against all of the smaller cell's, as long as the two are in two
@@ -1454,9 +1497,15 @@ __global__ void iota_kernel(int* p, long long n) {
     if (i < n) p[i] = (int)i;
 }
 
-__global__ void fill_kernel(int* p, long long n, int v) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = v;
+// The nodes of the final union-find: the cells' components so far, then the
+// sorted points.
+__global__ void nodes_kernel(int C, const int* parentC, int* parent, int* compMin, int* compFix, const int* counts) {
+    const long long n = (long long)C + sorted_points(counts);
+    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
+        parent[v] = v < C ? parentC[v] : (int)v;
+        compMin[v] = INT_MAX;
+        compFix[v] = INT_MAX;
+    }
 }
 
 // node's smallest core (and fixed-point) index, folded into its component's root
@@ -1474,59 +1523,51 @@ __device__ __forceinline__ bool node_keys(const Sorted& Q, const Cells& K, int v
     return true;
 }
 
-__global__ void comp_kernel(Sorted Q, Cells K, long long N, int* parent, int* compMin, int* compFix) {
-    const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= N) return;
-    int key, fixKey;
-    if (!node_keys(Q, K, (int)v, key, fixKey)) return;
-    const int r = uf_find(parent, (int)v);
-    atomicMin(&compMin[r], key);
-    if (fixKey != INT_MAX) atomicMin(&compFix[r], fixKey);
+__global__ void comp_kernel(Sorted Q, Cells K, int* parent, int* compMin, int* compFix, const int* counts) {
+    const long long n = (long long)K.C + sorted_points(counts);
+    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
+        int key, fixKey;
+        if (!node_keys(Q, K, (int)v, key, fixKey)) continue;
+        const int r = uf_find(parent, (int)v);
+        atomicMin(&compMin[r], key);
+        if (fixKey != INT_MAX) atomicMin(&compFix[r], fixKey);
+    }
 }
 
-__global__ void roots_kernel(Sorted Q, Cells K, long long N, int* parent, const int* compMin, const int* compFix,
-                             int* rootList, int* rootMin, int* rootFix, int* nRoots) {
-    const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    bool take = false;
-    int key, fixKey;
-    if (v < N && node_keys(Q, K, (int)v, key, fixKey)) take = uf_find(parent, (int)v) == (int)v;
-    const unsigned m = __ballot_sync(0xffffffffu, take);
-    if (!m) return;
-    const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(nRoots, __popc(m));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (!take) return;
-    const int k = base + __popc(m & ((1u << lane) - 1));
-    rootList[k] = (int)v;
-    rootMin[k] = compMin[v];
-    rootFix[k] = compFix[v];
+// Numbering: textbook, the components by their smallest core index; reference
+// mode, those with a fixed point by their smallest fixed-point index (-1, -2,
+// ...), the others by their smallest index. Each root marks its index in a bit
+// array over the points (fixed-point components in a second one), whose prefix
+// sums rank it.
+__global__ void root_marks_kernel(Sorted Q, Cells K, int* parent, const int* compMin, const int* compFix, int compat,
+                                  unsigned* bits, unsigned* fixBits, const int* counts) {
+    const long long n = (long long)K.C + sorted_points(counts);
+    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
+        int key, fixKey;
+        if (!node_keys(Q, K, (int)v, key, fixKey) || uf_find(parent, (int)v) != (int)v) continue;
+        const bool fix = compat && compFix[v] != INT_MAX;
+        const int at = fix ? compFix[v] : compMin[v];
+        atomicOr((fix ? fixBits : bits) + (at >> 5), 1u << (at & 31));
+    }
 }
 
-__global__ void scatter_labels_kernel(const int* rootList, const int* lab, int K, int* compLabel) {
-    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < K) compLabel[rootList[k]] = lab[k];
+__global__ void bit_counts_kernel(const unsigned* bits, int* cnt, long long words) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < words) cnt[i] = __popc(bits[i]);
 }
 
-// Numbering on the device for many components: marks over the point indices,
-// then prefix sums (textbook: by smallest core index; reference: fixed-point
-// components by their smallest fixed-point index, the others by smallest index).
-__global__ void rank_marks_kernel(const int* rootMin, const int* rootFix, int K, int compat, int* markMin,
-                                  int* markFix) {
-    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= K) return;
-    if (compat && rootFix[k] != INT_MAX) markFix[rootFix[k]] = 1;
-    else markMin[rootMin[k]] = 1;
-}
-
-__global__ void rank_labels_kernel(const int* rootList, const int* rootMin, const int* rootFix, int K, int compat,
-                                   const int* rankMin, const int* rankFix, int* compLabel) {
-    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= K) return;
-    int lab;
-    if (compat) lab = rootFix[k] != INT_MAX ? -(rankFix[rootFix[k]] + 1) : rankMin[rootMin[k]] + 1;
-    else lab = rankMin[rootMin[k]];
-    compLabel[rootList[k]] = lab;
+__global__ void root_labels_kernel(Sorted Q, Cells K, int* parent, const int* compMin, const int* compFix, int compat,
+                                   const unsigned* bits, const unsigned* fixBits, const int* rank, const int* fixRank,
+                                   int* compLabel, const int* counts) {
+    const long long n = (long long)K.C + sorted_points(counts);
+    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
+        int key, fixKey;
+        if (!node_keys(Q, K, (int)v, key, fixKey) || uf_find(parent, (int)v) != (int)v) continue;
+        const bool fix = compat && compFix[v] != INT_MAX;
+        const int at = fix ? compFix[v] : compMin[v];
+        const int r = (fix ? fixRank : rank)[at >> 5] + __popc((fix ? fixBits : bits)[at >> 5] & ((1u << (at & 31)) - 1u));
+        compLabel[v] = fix ? -(r + 1) : (compat ? r + 1 : r);
+    }
 }
 
 __global__ void cell_labels_kernel(Cells K, int* parent, const int* compLabel, int* cellLabel) {
@@ -1556,12 +1597,10 @@ __global__ void labels_kernel(const int* slot, const int* slotCell, long long n,
 // warp or, the long ones, through the queue, a safe cell only while it could
 // still lower the answer); the rest are noise (-1). border_labels_kernel
 // writes those that are not core.
-__global__ void sorted_labels_kernel(Sorted Q, Cells K, const int* nbStart, const int* nbList, int M1, double eps,
+__device__ __forceinline__ void sorted_label(Sorted Q, Cells K, const int* nbStart, const int* nbList, double eps,
                                      int* parent, const int* compMin, const int* compLabel, int* labels, ScanQueue W,
-                                     unsigned long long* bests) {
-    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+                                     unsigned long long* bests, long long w) {
     const int lane = threadIdx.x & 31;
-    if (w >= M1) return;
     const int p = (int)w;
     const int c = Q.cell[p];
     if (Q.core[p] == 1) {
@@ -1663,13 +1702,23 @@ __global__ void sorted_labels_kernel(Sorted Q, Cells K, const int* nbStart, cons
         }
 }
 
+__global__ void sorted_labels_kernel(Sorted Q, Cells K, const int* nbStart, const int* nbList, double eps,
+                                     int* parent, const int* compMin, const int* compLabel, int* labels, ScanQueue W,
+                                     unsigned long long* bests, const int* counts) {
+    const int n = counts[kSparse];
+    for (long long w = first_warp(); w < n; w += warp_stride())
+        sorted_label(Q, K, nbStart, nbList, eps, parent, compMin, compLabel, labels, W, bests, w);
+}
+
 // After the queued scans: the labels of the points that are not core.
-__global__ void border_labels_kernel(Sorted Q, int M1, const unsigned long long* bests, const int* compLabel,
-                                     int* labels) {
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= M1 || Q.core[p] == 1) return;
-    const unsigned long long best = bests[p];
-    labels[Q.order[p]] = best == ~0ull ? -1 : compLabel[(int)(best & 0xffffffffull)];
+__global__ void border_labels_kernel(Sorted Q, const unsigned long long* bests, const int* compLabel, int* labels,
+                                     const int* counts) {
+    const int n = counts[kSparse];
+    for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
+        if (Q.core[p] == 1) continue;
+        const unsigned long long best = bests[p];
+        labels[Q.order[p]] = best == ~0ull ? -1 : compLabel[(int)(best & 0xffffffffull)];
+    }
 }
 
 #define CK(x)                                                   \
@@ -1681,64 +1730,39 @@ __global__ void border_labels_kernel(Sorted Q, int M1, const unsigned long long*
 #define NEED(p) \
     if (!(p)) return CHAOS_E_NOMEM
 
-// Components numbered on the host when there are few (their keys copied
-// back), on the device otherwise.
-constexpr int kHostRankMax = 1 << 18;
-
-int number_components(Call& c, long long n, int K, bool compat, const int* rootList, const int* rootMin,
-                      const int* rootFix, int* compLabel) {
-    cudaStream_t st = c.stream;
-    if (K <= 0) return CHAOS_OK;
-    if (K <= kHostRankMax) {
-        std::vector<int> hMin(K), hFix(K), lab(K), idx(K);
-        CK(cudaMemcpyAsync(hMin.data(), rootMin, K * sizeof(int), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(hFix.data(), rootFix, K * sizeof(int), cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        for (int k = 0; k < K; ++k) idx[k] = k;
-        if (compat) {
-            // fixed-point components by smallest fixed-point index (-1, -2, ...), the others by smallest index
-            std::vector<int> neg, pos;
-            for (int k = 0; k < K; ++k) (hFix[k] != INT_MAX ? neg : pos).push_back(k);
-            std::sort(neg.begin(), neg.end(), [&](int a, int b) { return hFix[a] < hFix[b]; });
-            std::sort(pos.begin(), pos.end(), [&](int a, int b) { return hMin[a] < hMin[b]; });
-            for (size_t r = 0; r < neg.size(); ++r) lab[neg[r]] = -(int)(r + 1);
-            for (size_t r = 0; r < pos.size(); ++r) lab[pos[r]] = (int)(r + 1);
-        } else {
-            std::sort(idx.begin(), idx.end(), [&](int a, int b) { return hMin[a] < hMin[b]; });
-            for (int r = 0; r < K; ++r) lab[idx[r]] = r;
+// Scratch arrays of one call, several to an allocation.
+struct Arena {
+    Call& c;
+    char* at = nullptr;
+    size_t left = 0;
+    template <class T> T* take(size_t count) {
+        const size_t bytes = (count * sizeof(T) + 255) / 256 * 256;
+        if (bytes > left) {
+            constexpr size_t kChunk = 4 << 20;
+            char* p = (char*)c.alloc(std::max(bytes, kChunk));
+            if (!p) return nullptr;
+            if (bytes >= kChunk) return (T*)p;
+            at = p;
+            left = kChunk;
         }
-        int* dLab = (int*)c.alloc((size_t)K * sizeof(int));
-        NEED(dLab);
-        CK(cudaMemcpyAsync(dLab, lab.data(), K * sizeof(int), cudaMemcpyHostToDevice, st));
-        scatter_labels_kernel<<<blocks(K), kTPB, 0, st>>>(rootList, dLab, K, compLabel);
-        note_launch();
-        CKL();
-        CK(cudaStreamSynchronize(st));  // lab is released on return
-        return CHAOS_OK;
+        T* r = (T*)at;
+        at += bytes;
+        left -= bytes;
+        return r;
     }
-    int* markMin = (int*)c.alloc(n * sizeof(int));
-    int* markFix = (int*)c.alloc(n * sizeof(int));
-    NEED(!c.failed);
-    CK(cudaMemsetAsync(markMin, 0, n * sizeof(int), st));
-    CK(cudaMemsetAsync(markFix, 0, n * sizeof(int), st));
-    rank_marks_kernel<<<blocks(K), kTPB, 0, st>>>(rootMin, rootFix, K, compat ? 1 : 0, markMin, markFix);
-    note_launch();
-    CKL();
-    int t = 0, rc;
-    if ((rc = exclusive_scan(c, markMin, markMin, n, &t))) return rc;
-    if (compat && (rc = exclusive_scan(c, markFix, markFix, n, &t))) return rc;
-    rank_labels_kernel<<<blocks(K), kTPB, 0, st>>>(rootList, rootMin, rootFix, K, compat ? 1 : 0, markMin, markFix,
-                                                   compLabel);
-    note_launch();
-    CKL();
-    return CHAOS_OK;
-}
+};
 
 // The pipeline. compat: the reference's eps-components (every included point
 // core, numbering by fixed points); otherwise textbook DBSCAN with minPts.
-// bound > 0: a bound on the occupied cells known from the source (else one
-// pass over the features measures their extent). Fout (basin maps) receives
-// the normalised features.
+// bound > 0: a bound on the occupied cells known from the source. Without one,
+// a small set's table is sized by its points (measuring their extent takes a
+// pass and a wait, more than the larger table costs), a large one's by the
+// extent of its cells. Every wait for a count costs the host's round trip and
+// an idle GPU: with one left of seven, and the scratch in few allocations,
+// 10,000 points take 256 instead of 445 us, 1,000,000 505 instead of 690. Fout
+// (basin maps) receives the normalised features.
+constexpr long long kSmallSet = 65536;
+
 template <class Src>
 int cell_cluster(Call& c, const Src& S, long long n, double eps, int minPts, bool compat, double bound, double* Fout,
                  int* labels) {
@@ -1747,11 +1771,16 @@ int cell_cluster(Call& c, const Src& S, long long n, double eps, int minPts, boo
     const bool zeroEps = !(eps > 0);
     const double side = zeroEps ? 1.0 : eps / sqrt((double)D) * (1.0 - 1e-9);
     const double invSide = 1.0 / side;
-    int* err = (int*)c.alloc(sizeof(int));
-    NEED(err);
-    CK(cudaMemsetAsync(err, 0, sizeof(int), st));
-    if (!(bound > 0)) {
-        long long* ext = (long long*)c.alloc(8 * sizeof(long long));
+    int sms = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device));
+    sms = std::max(sms, 1);
+    const unsigned loop = (unsigned)(kLoopBlocksPerSm * sms);
+    Arena A{c};
+    int* counts = A.take<int>(kCounts);
+    NEED(counts);
+    CK(cudaMemsetAsync(counts, 0, kCounts * sizeof(int), st));
+    if (!(bound > 0) && n > kSmallSet) {
+        long long* ext = A.take<long long>(8);
         NEED(ext);
         const long long init[8] = {LLONG_MIN, LLONG_MIN, LLONG_MIN, LLONG_MIN, LLONG_MIN, LLONG_MIN, 0, 0};
         CK(cudaMemcpyAsync(ext, init, sizeof init, cudaMemcpyHostToDevice, st));
@@ -1766,326 +1795,285 @@ int cell_cluster(Call& c, const Src& S, long long n, double eps, int minPts, boo
             for (int d = 0; d < D; ++d) prod *= (double)(hx[3 + d] + hx[d] + 1);
             bound += prod;
         }
+    } else if (!(bound > 0)) {
+        bound = (double)n;
     }
     bound = std::min(bound, (double)n);
     unsigned long long cap = 1024;
     while ((double)cap < 2.0 * bound + 2.0) cap <<= 1;
     Table T;
     T.mask = cap - 1;
-    T.key = (unsigned long long*)c.alloc(cap * sizeof(unsigned long long));
-    T.st = (CellStats*)c.alloc(cap * sizeof(CellStats));
-    int* slot = (int*)c.alloc(n * sizeof(int));
-    int* occ = (int*)c.alloc(cap * sizeof(int));
-    int* slotCell = (int*)c.alloc(cap * sizeof(int));
+    T.key = A.take<unsigned long long>(cap);
+    T.st = A.take<CellStats>(cap);
+    int* slot = A.take<int>(n);
+    int* occ = A.take<int>(cap);
+    int* slotCell = A.take<int>(cap);
     NEED(!c.failed);
     table_init_kernel<<<blocks(cap), kTPB, 0, st>>>(T, (long long)cap);
     note_launch();
-    int sms = 0;
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device));
     {
-        const long long most = (long long)std::max(sms, 1) * kCellBlocksPerSm;
+        const long long most = (long long)sms * kCellBlocksPerSm;
         const long long rows = (n + kCellBlock - 1) / kCellBlock, per = (rows + most - 1) / most;
         CK(cudaFuncSetAttribute(cells_kernel<Src>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BlockCells)));
         cells_kernel<Src><<<(unsigned)((rows + per - 1) / per), kCellBlock, sizeof(BlockCells), st>>>(
-            S, n, per * kCellBlock, invSide, T, slot, Fout, err);
+            S, n, per * kCellBlock, invSide, T, slot, Fout, counts + kErr);
         note_launch();
     }
     occupied_kernel<<<blocks(cap), kTPB, 0, st>>>(T.key, cap, occ);
     note_launch();
     CKL();
-    int C = 0;
-    int rc = exclusive_scan(c, occ, occ, (long long)cap, &C);
+    int rc = device_scan(c, occ, occ, (long long)cap, counts + kCells);
     if (rc) return rc;
-    {
-        int hErr = 0;
-        CK(cudaMemcpyAsync(&hErr, err, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        if (hErr) return set_error(CHAOS_E_CUDA, "clustering: cell table full");
-    }
+    int hc[2] = {0, 0};
+    static_assert(kErr == kCells + 1, "read together");
+    CK(cudaMemcpyAsync(hc, counts + kCells, sizeof hc, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (hc[1]) return set_error(CHAOS_E_CUDA, "clustering: cell table full");
+    const int C = hc[0];
     Cells K;
     K.C = C;
     K.D = D;
-    unsigned long long* cellKey = (unsigned long long*)c.alloc((size_t)(C + 1) * sizeof(unsigned long long));
-    int* cellSlot = (int*)c.alloc((size_t)(C + 1) * sizeof(int));
+    const size_t C1 = (size_t)C + 1;
+    unsigned long long* cellKey = A.take<unsigned long long>(C1);
+    int* cellSlot = A.take<int>(C1);
     K.key = cellKey;
-    K.cnt = (int*)c.alloc((size_t)(C + 1) * sizeof(int));
-    K.lo = (double*)c.alloc((size_t)(C + 1) * 3 * sizeof(double));
-    K.hi = (double*)c.alloc((size_t)(C + 1) * 3 * sizeof(double));
-    K.unsafe = (unsigned char*)c.alloc((size_t)C + 1);
-    K.dense = (unsigned char*)c.alloc((size_t)C + 1);
-    K.minIdx = (int*)c.alloc((size_t)(C + 1) * sizeof(int));
-    K.minFix = (int*)c.alloc((size_t)(C + 1) * sizeof(int));
-    K.repV = (double*)c.alloc((size_t)(C + 1) * kReps * 3 * sizeof(double));
-    K.repN = (int*)c.alloc((size_t)(C + 1) * sizeof(int));
-    K.hasCore = (int*)c.alloc((size_t)(C + 1) * sizeof(int));
-    K.minCore = (int*)c.alloc((size_t)(C + 1) * sizeof(int));
-    K.sb = (int*)c.alloc((size_t)(C + 1) * sizeof(int));
-    K.se = (int*)c.alloc((size_t)(C + 1) * sizeof(int));
-    K.need = (int*)c.alloc((size_t)(C + 1) * sizeof(int));
-    int* nbStart = (int*)c.alloc((size_t)(C + 1) * sizeof(int));
-    int* take = (int*)c.alloc((size_t)(C + 1) * sizeof(int));
-    int* begin = (int*)c.alloc((size_t)(C + 1) * sizeof(int));
-    int* cursor = (int*)c.alloc((size_t)(C + 1) * sizeof(int));
-    int* parentC = (int*)c.alloc((size_t)(C + 1) * sizeof(int));
+    K.cnt = A.take<int>(C1);
+    K.lo = A.take<double>(3 * C1);
+    K.hi = A.take<double>(3 * C1);
+    K.unsafe = A.take<unsigned char>(C1);
+    K.dense = A.take<unsigned char>(C1);
+    K.minIdx = A.take<int>(C1);
+    K.minFix = A.take<int>(C1);
+    K.repV = A.take<double>(C1 * kReps * 3);
+    K.repN = A.take<int>(C1);
+    K.hasCore = A.take<int>(C1);
+    K.minCore = A.take<int>(C1);
+    K.sb = A.take<int>(C1);
+    K.se = A.take<int>(C1);
+    K.need = A.take<int>(C1);
+    int* nbStart = A.take<int>(C1);
+    int* take = A.take<int>(C1);
+    int* begin = A.take<int>(C1);
+    int* cursor = A.take<int>(C1);
+    int* parentC = A.take<int>(C1);
+    int* cellLabel = A.take<int>(C1);
     NEED(!c.failed);
-    if (C > 0) {
-        cell_ids_kernel<<<blocks(cap), kTPB, 0, st>>>(T.key, cap, occ, slotCell, cellKey, cellSlot);
-        note_launch();
-        finalize_kernel<Src><<<blocks(C), kTPB, 0, st>>>(S, K, cellSlot, T, compat ? 1 : 0, zeroEps ? 1 : 0, minPts);
-        note_launch();
-        neighbours_kernel<<<blocks((long long)C * 32), kTPB, 0, st>>>(cellKey, C, D, T.key, T.mask, slotCell,
-                                                                      nbStart, nullptr, nullptr, nullptr);
-        note_launch();
-        iota_kernel<<<blocks(C), kTPB, 0, st>>>(parentC, C);
+    if (C == 0) {  // no point takes part
+        labels_kernel<<<blocks(n), kTPB, 0, st>>>(slot, slotCell, n, K.dense, cellLabel, compat ? 1 : 0, labels);
         note_launch();
         CKL();
+        return CHAOS_OK;
     }
+    cell_ids_kernel<<<blocks(cap), kTPB, 0, st>>>(T.key, cap, occ, slotCell, cellKey, cellSlot);
+    note_launch();
+    finalize_kernel<Src><<<blocks(C), kTPB, 0, st>>>(S, K, cellSlot, T, compat ? 1 : 0, zeroEps ? 1 : 0, minPts);
+    note_launch();
+    neighbours_kernel<<<blocks((long long)C * 32), kTPB, 0, st>>>(cellKey, C, D, T.key, T.mask, slotCell, nbStart,
+                                                                  nullptr, nullptr, nullptr);
+    note_launch();
+    iota_kernel<<<blocks(C), kTPB, 0, st>>>(parentC, C);
+    note_launch();
+    CKL();
     CK(cudaMemsetAsync(nbStart + C, 0, sizeof(int), st));
-    int E = 0;
-    if ((rc = exclusive_scan(c, nbStart, nbStart, C + 1, &E))) return rc;
-    int* nbList = (int*)c.alloc((size_t)(E + 1) * sizeof(int));
-    int* nbOwner = (int*)c.alloc((size_t)(E + 1) * sizeof(int));
-    unsigned char* pst = (unsigned char*)c.alloc((size_t)E + 1);
-    unsigned char* openE = (unsigned char*)c.alloc((size_t)E + 1);
-    unsigned char* settledE = (unsigned char*)c.alloc((size_t)E + 1);
-    unsigned char* deferred = (unsigned char*)c.alloc((size_t)E + 1);
-    int* openList = (int*)c.alloc((size_t)(E + 1) * sizeof(int));
-    int* nOpen = (int*)c.alloc(sizeof(int));
-    int* joinList = (int*)c.alloc((size_t)(E + 1) * sizeof(int));
-    int* nJoined = (int*)c.alloc(sizeof(int));
+    if ((rc = device_scan(c, nbStart, nbStart, (long long)C + 1, counts + kEntries))) return rc;
+    // room for the neighbour entries: by their bound while that is small,
+    // otherwise by their number, which takes a wait
+    long long E = (long long)C * (D == 1 ? 2 * kR : (D == 2 ? 24 : 124));
+    if (E > (1 << 20)) {
+        int hE = 0;
+        CK(cudaMemcpyAsync(&hE, counts + kEntries, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        E = hE;
+    }
+    const size_t E1 = (size_t)E + 1;
+    int* nbList = A.take<int>(E1);
+    int* nbOwner = A.take<int>(E1);
+    unsigned char* pst = A.take<unsigned char>(E1);
+    unsigned char* openE = A.take<unsigned char>(E1);
+    unsigned char* settledE = A.take<unsigned char>(E1);
+    unsigned char* deferred = A.take<unsigned char>(E1);
+    int* openList = A.take<int>(E1);
+    int* joinList = A.take<int>(E1);
+    int* active = A.take<int>(E1);
     NEED(!c.failed);
     if (E > 0) {
         neighbours_kernel<<<blocks((long long)C * 32), kTPB, 0, st>>>(cellKey, C, D, T.key, T.mask, slotCell,
                                                                       nullptr, nbStart, nbList, nbOwner);
         note_launch();
-        CK(cudaMemsetAsync(openE, 0, (size_t)E, st));
-        CK(cudaMemsetAsync(settledE, 0, (size_t)E, st));
-        CK(cudaMemsetAsync(deferred, 0, (size_t)E, st));
-        CK(cudaMemsetAsync(nOpen, 0, sizeof(int), st));
-        CK(cudaMemsetAsync(nJoined, 0, sizeof(int), st));
-        pair_kernel<<<blocks(E), kTPB, 0, st>>>(K, nbOwner, nbList, E, eps, pst, openList, nOpen, joinList, nJoined);
+        pair_kernel<<<blocks(E), kTPB, 0, st>>>(K, nbOwner, nbList, eps, pst, openList, joinList, active, openE,
+                                                settledE, deferred, counts);
         note_launch();
-        CKL();
-        int hOpen = 0;
-        CK(cudaMemcpyAsync(&hOpen, nOpen, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        if (hOpen > 0) {
-            rep_pairs_kernel<<<blocks((long long)hOpen * 32), kTPB, 0, st>>>(K, nbOwner, nbList, openList, hOpen, eps,
-                                                                             pst, joinList, nJoined);
-            note_launch();
-            CKL();
-        }
+        rep_pairs_kernel<<<loop, kTPB, 0, st>>>(K, nbOwner, nbList, openList, eps, pst, joinList, counts);
+        note_launch();
         if (C <= kSharedCells) {
             const size_t shm = (size_t)C * sizeof(int);
             if (shm > 48 * 1024)
                 CK(cudaFuncSetAttribute(cell_components_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-            cell_components_kernel<<<1, 1024, shm, st>>>(C, nbOwner, nbList, joinList, nJoined, parentC);
+            cell_components_kernel<<<1, 1024, shm, st>>>(C, nbOwner, nbList, joinList, counts + kJoinedCount, parentC);
         } else {
-            join_all_kernel<<<blocks(E), kTPB, 0, st>>>(nbOwner, nbList, joinList, nJoined, parentC);
+            join_all_kernel<<<blocks(E), kTPB, 0, st>>>(nbOwner, nbList, joinList, counts + kJoinedCount, parentC);
         }
         note_launch();
         CKL();
     }
     // first sort: the points of the cells that are not dense
+    const size_t n1 = (size_t)n + 1;
     Sorted Q;
-    Q.order = (int*)c.alloc((size_t)(n + 1) * sizeof(int));
-    Q.cell = (int*)c.alloc((size_t)(n + 1) * sizeof(int));
-    Q.core = (unsigned char*)c.alloc((size_t)n + 1);
-    Q.fix = compat ? (unsigned char*)c.alloc((size_t)n + 1) : nullptr;
+    Q.order = A.take<int>(n1);
+    Q.cell = A.take<int>(n1);
+    Q.core = A.take<unsigned char>(n1);
+    Q.fix = compat ? A.take<unsigned char>(n1) : nullptr;
     for (int d = 0; d < 3; ++d) {
-        Q.s[d] = d < D ? (double*)c.alloc((size_t)(n + 1) * sizeof(double)) : nullptr;
-        Q.r[d] = d < D ? (float*)c.alloc((size_t)(n + 1) * sizeof(float)) : nullptr;
+        Q.s[d] = d < D ? A.take<double>(n1) : nullptr;
+        Q.r[d] = d < D ? A.take<float>(n1) : nullptr;
     }
     Q.sb = K.sb;
     Q.se = K.se;
     Q.D = D;
+    // what the long scans find per sorted point (a count, later the best
+    // component's key), and their queue
+    unsigned long long* found = A.take<unsigned long long>(n1);
+    ScanQueue W;
+    W.cap = (int)std::min<long long>(std::max<long long>(4096, n), 1 << 20);
+    W.point = A.take<int>(W.cap);
+    W.cell = A.take<int>(W.cap);
+    W.count = counts + kScanA;
+    // nodes: the cells, then the sorted points
+    const size_t N = (size_t)C + (size_t)n + 1;
+    int* parent = A.take<int>(N);
+    int* compMin = A.take<int>(N);
+    int* compFix = A.take<int>(N);
+    int* compLabel = A.take<int>(N);
+    const long long words = (n + 31) / 32;
+    unsigned* bits = A.take<unsigned>(2 * words);
+    int* ranks = A.take<int>(2 * words);
     NEED(!c.failed);
-    int M1 = 0;
-    if (C > 0) {
-        take_sparse_kernel<<<blocks(C), kTPB, 0, st>>>(K, take);
+    auto sort_phase = [&](const int* before, int* total) -> int {
+        int r = device_scan(c, take, cursor, C, total);
+        if (r) return r;
+        phase_begin_kernel<<<blocks(C), kTPB, 0, st>>>(C, cursor, take, before, begin, K.sb, K.se, K.cnt);
+        note_launch();
+        sort_kernel<Src><<<blocks(n), kTPB, 0, st>>>(S, n, slot, slotCell, begin, cursor, Q, K.dense, K.lo,
+                                                     compat ? 1 : 0, total);
         note_launch();
         CKL();
-        if ((rc = exclusive_scan(c, take, cursor, C, &M1))) return rc;
-        if (M1 > 0) {
-            phase_begin_kernel<<<blocks(C), kTPB, 0, st>>>(C, cursor, take, 0, begin, K.sb, K.se, K.cnt);
-            note_launch();
-            CK(cudaMemsetAsync(cursor, 0, (size_t)C * sizeof(int), st));
-            sort_kernel<Src><<<blocks(n), kTPB, 0, st>>>(S, n, slot, slotCell, begin, cursor, Q, K.dense, K.lo,
-                                                         compat ? 1 : 0);
-            note_launch();
-            CKL();
-        }
-    }
-    // core flags and the shortcuts' links of the points that are not in dense cells
-    if (M1 > 0) {
-        if (!compat) {
-            core_kernel<<<blocks((long long)M1 * 32), kTPB, 0, st>>>(Q, K, nbStart, nbList, M1, eps, minPts, 0,
-                                                                     ScanQueue{}, nullptr);
-            note_launch();
-        }
-        dense_links_kernel<<<blocks((long long)M1 * 32), kTPB, 0, st>>>(Q, K, nbStart, nbList, M1, eps, parentC,
-                                                                        openE, settledE);
-        note_launch();
-        CKL();
-    }
-    if (E > 0) {
-        open_pairs_kernel<<<blocks(E), kTPB, 0, st>>>(K, nbOwner, nbList, E, parentC, pst, openE, settledE);
-        note_launch();
-        CKL();
-    }
-    // second sort: the cells some pair, count or label still has to scan
-    int M2 = 0;
-    if (C > 0) {
-        take_needed_kernel<<<blocks(C), kTPB, 0, st>>>(K, take);
-        note_launch();
-        CKL();
-        if ((rc = exclusive_scan(c, take, cursor, C, &M2))) return rc;
-        if (M2 > 0) {
-            phase_begin_kernel<<<blocks(C), kTPB, 0, st>>>(C, cursor, take, M1, begin, K.sb, K.se, K.cnt);
-            note_launch();
-            CK(cudaMemsetAsync(cursor, 0, (size_t)C * sizeof(int), st));
-            sort_kernel<Src><<<blocks(n), kTPB, 0, st>>>(S, n, slot, slotCell, begin, cursor, Q, K.dense, K.lo,
-                                                         compat ? 1 : 0);
-            note_launch();
-            CKL();
-        }
-    }
-    // union-find over nodes: cells, then the sorted points (unsafe cells' core points)
-    const long long M = (long long)M1 + M2;
-    const long long N = (long long)C + M;
-    int* parent = (int*)c.alloc((size_t)(N + 1) * sizeof(int));
-    int* compMin = (int*)c.alloc((size_t)(N + 1) * sizeof(int));
-    int* compFix = (int*)c.alloc((size_t)(N + 1) * sizeof(int));
-    int* compLabel = (int*)c.alloc((size_t)(N + 1) * sizeof(int));
-    int* cellLabel = (int*)c.alloc((size_t)(C + 1) * sizeof(int));
-    int* rootList = (int*)c.alloc((size_t)(N + 1) * sizeof(int));
-    int* rootMin = (int*)c.alloc((size_t)(N + 1) * sizeof(int));
-    int* rootFix = (int*)c.alloc((size_t)(N + 1) * sizeof(int));
-    int* nRoots = (int*)c.alloc(sizeof(int));
-    NEED(!c.failed);
-    iota_kernel<<<blocks(N + 1), kTPB, 0, st>>>(parent, N + 1);
+        return CHAOS_OK;
+    };
+    take_sparse_kernel<<<blocks(C), kTPB, 0, st>>>(K, take);
     note_launch();
-    if (C > 0) CK(cudaMemcpyAsync(parent, parentC, (size_t)C * sizeof(int), cudaMemcpyDeviceToDevice, st));
-    // the queue of the long scans, and what they find per sorted point: a
-    // count, later the best component's key
-    ScanQueue W{};
-    unsigned long long* found = nullptr;
-    const unsigned scanBlocks = (unsigned)(8 * std::max(sms, 1));
-    if (M1 > 0 && M2 > 0) {  // (cells are scanned exactly only once the second phase has sorted them)
-        W.cap = std::max(4096, M1);
-        W.point = (int*)c.alloc((size_t)W.cap * sizeof(int));
-        W.cell = (int*)c.alloc((size_t)W.cap * sizeof(int));
-        W.count = (int*)c.alloc(2 * sizeof(int));
-        NEED(!c.failed);
-        CK(cudaMemsetAsync(W.count, 0, 2 * sizeof(int), st));
-    }
-    if (M1 > 0) {
-        found = (unsigned long long*)c.alloc((size_t)M1 * sizeof(unsigned long long));
-        NEED(found);
-    }
-    if (M1 > 0 && !compat) {  // the undecided counts, exactly (their neighbours are sorted now)
-        core_kernel<<<blocks((long long)M1 * 32), kTPB, 0, st>>>(Q, K, nbStart, nbList, M1, eps, minPts, 1, W,
-                                                                 (int*)found);
+    if ((rc = sort_phase(nullptr, counts + kSparse))) return rc;
+    // core flags and the shortcuts' links of the points that are not in dense cells
+    if (!compat) {
+        core_kernel<<<loop, kTPB, 0, st>>>(Q, K, nbStart, nbList, eps, minPts, 0, ScanQueue{}, nullptr, counts);
         note_launch();
-        if (W.cap > 0) {
-            long_scan_kernel<<<scanBlocks, 256, 0, st>>>(Q, K, W, eps, minPts, 0, (int*)found, nullptr, nullptr,
-                                                         nullptr);
-            note_launch();
-        }
-        core_finish_kernel<<<blocks((long long)M1 * 32), kTPB, 0, st>>>(Q, K, nbStart, nbList, M1, eps, minPts,
-                                                                        (const int*)found, parent);
-        note_launch();
-        CKL();
     }
+    dense_links_kernel<<<loop, kTPB, 0, st>>>(Q, K, nbStart, nbList, eps, parentC, openE, settledE, counts);
+    note_launch();
     if (E > 0) {
-        whole_pairs_kernel<<<blocks(E), kTPB, 0, st>>>(K, nbOwner, nbList, E, pst, parent);
+        open_pairs_kernel<<<blocks(E), kTPB, 0, st>>>(K, nbOwner, nbList, parentC, pst, openE, settledE, active, counts);
         note_launch();
     }
-    if (C > 0 && M > 0) {
-        unsafe_cell_kernel<<<blocks((long long)C * 32), kTPB, 0, st>>>(Q, K, eps, parent);
+    CKL();
+    // second sort: the cells some pair, count or label still has to scan
+    take_needed_kernel<<<blocks(C), kTPB, 0, st>>>(K, take);
+    note_launch();
+    if ((rc = sort_phase(counts + kSparse, counts + kNeeded))) return rc;
+    nodes_kernel<<<loop, kTPB, 0, st>>>(C, parentC, parent, compMin, compFix, counts);
+    note_launch();
+    if (!compat) {  // the undecided counts, exactly (their neighbours are sorted now)
+        core_kernel<<<loop, kTPB, 0, st>>>(Q, K, nbStart, nbList, eps, minPts, 1, W, (int*)found, counts);
+        note_launch();
+        long_scan_kernel<<<loop, 256, 0, st>>>(Q, K, W, eps, minPts, 0, (int*)found, nullptr, nullptr, nullptr);
+        note_launch();
+        core_finish_kernel<<<loop, kTPB, 0, st>>>(Q, K, nbStart, nbList, eps, minPts, (const int*)found, parent, counts);
         note_launch();
     }
-    if (E > 0 && M > 0) {
-        int* nLong = nOpen;  // (the open list has been read: its memory serves the long pairs)
-        CK(cudaMemsetAsync(nLong, 0, sizeof(int), st));
+    // unions
+    if (E > 0) {
+        whole_pairs_kernel<<<blocks(E), kTPB, 0, st>>>(K, nbOwner, nbList, pst, parent, counts);
+        note_launch();
+    }
+    unsafe_cell_kernel<<<blocks((long long)C * 32), kTPB, 0, st>>>(Q, K, eps, parent);
+    note_launch();
+    if (E > 0) {
+        // (the open list has been read: its memory serves the long pairs)
         for (int pass = 0; pass < kCrossPasses; ++pass) {
-            cross_cell_kernel<<<blocks((long long)E * 32), kTPB, 0, st>>>(Q, K, nbOwner, nbList, E, pst, eps, parent,
-                                                                          pass, deferred, openList, nLong);
+            cross_cell_kernel<<<loop, kTPB, 0, st>>>(Q, K, nbOwner, nbList, eps, parent, pass, deferred, openList,
+                                                     counts + kLong, active, counts);
             note_launch();
         }
-        long_pairs_kernel<<<scanBlocks, 256, 0, st>>>(Q, K, nbOwner, nbList, openList, nLong, eps, parent);
+        long_pairs_kernel<<<loop, 256, 0, st>>>(Q, K, nbOwner, nbList, openList, counts + kLong, eps, parent);
         note_launch();
     }
     CKL();
     // components, numbered
-    CK(cudaMemsetAsync(nRoots, 0, sizeof(int), st));
-    if (N > 0) {
-        fill_kernel<<<blocks(N), kTPB, 0, st>>>(compMin, N, INT_MAX);
-        note_launch();
-        fill_kernel<<<blocks(N), kTPB, 0, st>>>(compFix, N, INT_MAX);
-        note_launch();
-        comp_kernel<<<blocks(N), kTPB, 0, st>>>(Q, K, N, parent, compMin, compFix);
-        note_launch();
-        roots_kernel<<<blocks(N), kTPB, 0, st>>>(Q, K, N, parent, compMin, compFix, rootList, rootMin, rootFix,
-                                                 nRoots);
-        note_launch();
-        CKL();
-    }
-    int nK = 0;
-    CK(cudaMemcpyAsync(&nK, nRoots, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    if ((rc = number_components(c, n, nK, compat, rootList, rootMin, rootFix, compLabel))) return rc;
-    if (C > 0) {
-        cell_labels_kernel<<<blocks(C), kTPB, 0, st>>>(K, parent, compLabel, cellLabel);
-        note_launch();
-    }
+    comp_kernel<<<loop, kTPB, 0, st>>>(Q, K, parent, compMin, compFix, counts);
+    note_launch();
+    CK(cudaMemsetAsync(bits, 0, 2 * words * sizeof(unsigned), st));
+    root_marks_kernel<<<loop, kTPB, 0, st>>>(Q, K, parent, compMin, compFix, compat ? 1 : 0, bits, bits + words, counts);
+    note_launch();
+    const long long ranked = compat ? 2 * words : words;
+    bit_counts_kernel<<<blocks(ranked), kTPB, 0, st>>>(bits, ranks, ranked);
+    note_launch();
+    if ((rc = device_scan(c, ranks, ranks, words, nullptr))) return rc;
+    if (compat && (rc = device_scan(c, ranks + words, ranks + words, words, nullptr))) return rc;
+    root_labels_kernel<<<loop, kTPB, 0, st>>>(Q, K, parent, compMin, compFix, compat ? 1 : 0, bits, bits + words, ranks,
+                                              ranks + words, compLabel, counts);
+    note_launch();
+    cell_labels_kernel<<<blocks(C), kTPB, 0, st>>>(K, parent, compLabel, cellLabel);
+    note_launch();
     labels_kernel<<<blocks(n), kTPB, 0, st>>>(slot, slotCell, n, K.dense, cellLabel, compat ? 1 : 0, labels);
     note_launch();
-    if (M1 > 0) {
-        if (W.cap > 0) ++W.count;  // the second counter
-        sorted_labels_kernel<<<blocks((long long)M1 * 32), kTPB, 0, st>>>(Q, K, nbStart, nbList, M1, eps, parent,
-                                                                          compMin, compLabel, labels, W, found);
-        note_launch();
-        if (W.cap > 0) {
-            long_scan_kernel<<<scanBlocks, 256, 0, st>>>(Q, K, W, eps, minPts, 1, nullptr, found, parent, compMin);
-            note_launch();
-        }
-        border_labels_kernel<<<blocks(M1), kTPB, 0, st>>>(Q, M1, found, compLabel, labels);
-        note_launch();
-    }
+    W.count = counts + kScanB;
+    sorted_labels_kernel<<<loop, kTPB, 0, st>>>(Q, K, nbStart, nbList, eps, parent, compMin, compLabel, labels, W, found,
+                                                counts);
+    note_launch();
+    long_scan_kernel<<<loop, 256, 0, st>>>(Q, K, W, eps, minPts, 1, nullptr, found, parent, compMin);
+    note_launch();
+    border_labels_kernel<<<loop, kTPB, 0, st>>>(Q, found, compLabel, labels, counts);
+    note_launch();
     CKL();
     return CHAOS_OK;
 }
 
 }  // namespace
 
+// Exclusive prefix sums; dTotal (device memory, may be null) receives the total.
 template <class T>
-static int exclusive_scan_t(Call& c, const T* in, T* out, long long n, T* total) {
+static int device_scan_t(Call& c, const T* in, T* out, long long n, T* dTotal) {
     if (n <= 0) {
-        if (total) *total = 0;
+        if (dTotal) CK(cudaMemsetAsync(dTotal, 0, sizeof(T), c.stream));
         return CHAOS_OK;
     }
     const long long nb = (n + kScanItems - 1) / kScanItems;
-    T* sums = (T*)c.alloc((size_t)(nb + 1) * sizeof(T));
+    T* sums = nb == 1 && dTotal ? dTotal : (T*)c.alloc((size_t)nb * sizeof(T));
     if (!sums) return CHAOS_E_NOMEM;
     scan_block_kernel<T><<<(unsigned)nb, 1024, 0, c.stream>>>(in, out, sums, n);
     note_launch();
     CK(cudaGetLastError());
     if (nb > 1) {
-        int rc = exclusive_scan_t<T>(c, sums, sums, nb, total);
+        int rc = device_scan_t<T>(c, sums, sums, nb, dTotal);
         if (rc) return rc;
         add_offsets_kernel<T><<<blocks(n), kTPB, 0, c.stream>>>(out, sums, n);
         note_launch();
         CK(cudaGetLastError());
-    } else if (total) {
-        CK(cudaMemcpyAsync(total, sums, sizeof(T), cudaMemcpyDeviceToHost, c.stream));
-        CK(cudaStreamSynchronize(c.stream));
     }
     return CHAOS_OK;
 }
 
-int exclusive_scan(Call& c, const int* in, int* out, long long n, int* total) {
-    return exclusive_scan_t<int>(c, in, out, n, total);
+int device_scan(Call& c, const int* in, int* out, long long n, int* dTotal) {
+    return device_scan_t<int>(c, in, out, n, dTotal);
+}
+
+template <class T>
+static int exclusive_scan_t(Call& c, const T* in, T* out, long long n, T* total) {
+    T* d = total ? (T*)c.alloc(sizeof(T)) : nullptr;
+    if (total && !d) return CHAOS_E_NOMEM;
+    int rc = device_scan_t<T>(c, in, out, n, d);
+    if (rc || !total) return rc;
+    CK(cudaMemcpyAsync(total, d, sizeof(T), cudaMemcpyDeviceToHost, c.stream));
+    CK(cudaStreamSynchronize(c.stream));
+    return CHAOS_OK;
 }
 
 int exclusive_scan64(Call& c, const long long* in, long long* out, long long n, long long* total) {

@@ -22,9 +22,10 @@ int dbscan_basins_device(Call& c, const BasinsOut& O, long long n, const unsigne
 int dbscan_device(Call& c, const double* features, long long n, int dims, double eps, int minPts, const int* mask,
                   int* labels);
 
-// Exclusive prefix sum of n ints / 64-bit ints (device arrays; in == out
-// allowed); *total (host) receives the sum.
-int exclusive_scan(Call& c, const int* in, int* out, long long n, int* total);
+// Exclusive prefix sums of n ints / 64-bit ints (device arrays; in == out
+// allowed). dTotal (device memory, may be null) receives the sum without a
+// wait, *total (host) with one.
+int device_scan(Call& c, const int* in, int* out, long long n, int* dTotal);
 int exclusive_scan64(Call& c, const long long* in, long long* out, long long n, long long* total);
 
 }  // namespace chaos
