@@ -161,9 +161,15 @@ __global__ void __launch_bounds__(kBlock) lle_ff_kernel(LleParams L, double* out
     out[o] = lle_point_ff<F>(L, L.pBegin + o);
 }
 
-// Two points per thread, the first `singles` blocks one.
+// Two points per thread, the first `singles` blocks one. The FMA pipe bounds
+// it, and what keeps the pipe fed is the instructions in flight per warp, not
+// more warps: asked for two blocks per SM the compiler takes 154 registers
+// (Rossler) instead of the 94 it stops at unasked, and the 512^2 map (T = 500)
+// went from 183.6 to 171.6 ms, 2 rows of 128 points per SM (5,510 steps) from
+// 3.32 to 2.55 ms; 30 rows (3,510 steps) of Lorenz 27.7 -> 26.5 ms, of Chen
+// 28.5 -> 27.6.
 template <class F>
-__global__ void __launch_bounds__(kBlock) lle_ff_pair_kernel(LleParams L, double* out, unsigned singles) {
+__global__ void __launch_bounds__(kBlock, 2) lle_ff_pair_kernel(LleParams L, double* out, unsigned singles) {
     bool pair;
     const long long o = mixed_point(singles, pair);
     if (o >= L.nPoints) return;
