@@ -104,6 +104,7 @@ int group_resident_blocks(int kind, int system, int device) {
     if (kind == CHAOS_JOB_LLE2D_FF32) return group_ff_resident_blocks(system, device);
     GroupKernel k = group_kernel_for(kind, system);
     if (!k) return 0;
+    share_sms(k);
     int perSm = 0, sms = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k, kBatchBlock, group_shared_bytes(kind, system));
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -122,6 +123,7 @@ cudaError_t launch_group(int kind, int system, const JobDesc* jobs, const Chunk*
     GroupKernel k = group_kernel_for(kind, system);
     if (!k) return cudaErrorInvalidValue;
     if (count <= 0) return cudaSuccess;
+    share_sms(k);
     k<<<gridBlocks, kBatchBlock, group_shared_bytes(kind, system), st>>>(jobs, chunks, count, counter);
     note_launch();
     return cudaGetLastError();

@@ -10,6 +10,18 @@ namespace chaos {
 
 constexpr int kBatchBlock = 128;
 
+// The group kernels of a batch run at the same time, but an SM holds blocks of
+// two kernels only under one split of its memory between L1 and shared memory,
+// and left to itself a launch picks the split by the kernel's shared memory and
+// residency: blocks of a kernel with 96 registers waited for the SMs of one with
+// 104 to fall idle. All of them ask for the most shared memory (their loops
+// don't use L1). Six jobs of 84,163 to 841 points 5.68 -> 3.92 ms (a bifurcation
+// of 84,163 points alone 2.56, with one of 5,310 beside it 5.38 -> 2.56), nine
+// of 60,000 to 600 6.17 -> 5.20, fifteen of 100,000 to 1,000 10.1 either way.
+template <class K> void share_sms(K* kernel) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+}
+
 using GroupKernel = void (*)(const JobDesc*, const Chunk*, int, int*);
 GroupKernel bif_group_kernel(int system);
 GroupKernel basins_group_kernel(int system);

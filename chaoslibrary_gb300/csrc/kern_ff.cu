@@ -19,6 +19,7 @@
 #include <atomic>
 
 #include "batch.h"
+#include "batch_group.cuh"
 #include "engine.cuh"
 #include "sweep_launch.h"
 
@@ -297,6 +298,7 @@ cudaError_t launch_group_ff(int system, const JobDesc* jobs, const Chunk* chunks
     GroupFF k = group_ff_for(system);
     if (!k) return cudaErrorInvalidValue;
     if (count <= 0) return cudaSuccess;
+    share_sms(k);
     k<<<gridBlocks, kBlock, 0, st>>>(jobs, chunks, count, counter);
     note_launch();
     return cudaGetLastError();
