@@ -45,7 +45,7 @@ __device__ __forceinline__ void run_lle(const JobDesc& J, long long b, int cnt) 
     for (int t = 2 * threadIdx.x; t < cnt; t += 2 * blockDim.x) {
         const long long p = b + t;
         const bool two = t + 1 < cnt;
-        lle_pair_twin<F>(L, p, two ? p + 1 : p, J.lle + p, two ? J.lle + p + 1 : nullptr);
+        run_point<LlePair<F>>(L, p, two ? p + 1 : p, J.lle + p, two ? J.lle + p + 1 : nullptr);
     }
 }
 

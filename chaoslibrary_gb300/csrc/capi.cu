@@ -146,6 +146,18 @@ void* Call::alloc(size_t bytes) {
     return p;
 }
 
+void* Call::optional(size_t bytes) {
+    if (bytes == 0 || bytes > scratch_budget_bytes()) return nullptr;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    void* p = nullptr;
+    if (cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone &&
+        cudaMallocFromPoolAsync(&p, bytes, pool, stream) == cudaSuccess)
+        owned.push_back(p);
+    else
+        cudaGetLastError();
+    return p;
+}
+
 int Call::finish(int rc) {
     for (void* p : owned) cudaFreeAsync(p, stream);
     owned.clear();
@@ -245,11 +257,13 @@ static cudaError_t run_basins(int prec, const SweepParams& P, const BasinsOut& O
     if (P.system == SYS_USER) return prec == CHAOS_FP32 ? cudaErrorNotSupported : launch_basins_user(P, O, st);
     return prec == CHAOS_FP32 ? launch_basins_f32(P, O, st) : launch_basins_f64(P, O, st);
 }
-static cudaError_t run_lle(int prec, const LleParams& L, double* out, cudaStream_t st) {
+static cudaError_t run_lle(int prec, const LleParams& L, double* out, Call& c) {
+    cudaStream_t st = c.stream;
     if (L.legacyLoop) prec = CHAOS_FP64;  // the legacy kernels' arithmetic
     if (L.system == SYS_USER) return prec != CHAOS_FP64 ? cudaErrorNotSupported : launch_lle_user(L, out, st);
-    if (prec == CHAOS_FF32) return launch_lle_ff(L, out, st);
-    return prec == CHAOS_FP32 ? launch_lle_f32(L, out, st) : launch_lle_f64(L, out, st);
+    if (prec == CHAOS_FF32) return launch_lle_ff(L, out, st, (float*)c.optional(lle_ff_state_bytes(L)));
+    if (prec == CHAOS_FP32) return launch_lle_f32(L, out, st, (float*)c.optional(lle_f32_state_bytes(L)));
+    return launch_lle_f64(L, out, st);
 }
 
 // Values of a log-scale axis: the legacy getValueByIdxLog exponent
@@ -705,7 +719,7 @@ int chaos_lle2d(const chaos_exec* ex, int system, double tMax, double NT, int nP
     if ((rc = upload_fused_axes(c, 0, 2, nPts, ranges, L.table))) return c.finish(rc);
     double* dOut = (double*)c.output(lle, L.nPoints * sizeof(double));
     if (c.failed) return c.finish(CHAOS_E_NOMEM);
-    cudaError_t e = run_lle(c.ex.precision, L, dOut, c.stream);
+    cudaError_t e = run_lle(c.ex.precision, L, dOut, c);
     if (e != cudaSuccess) return c.finish(cuda_error(e, "LLE kernel"));
     rc = c.to_host(lle, dOut, L.nPoints * sizeof(double));
     return c.finish(rc);
@@ -744,7 +758,7 @@ static int run_legacy_scheme(const chaos_exec* ex, bool spectrum, int system, in
     const size_t outBytes = (size_t)L.nPoints * (spectrum ? nx : 1) * sizeof(double);
     double* dOut = (double*)c.output(out, outBytes);
     if (c.failed) return c.finish(CHAOS_E_NOMEM);
-    cudaError_t e = spectrum ? launch_spectrum_f64(L, dOut, c.stream) : run_lle(CHAOS_FP64, L, dOut, c.stream);
+    cudaError_t e = spectrum ? launch_spectrum_f64(L, dOut, c.stream) : run_lle(CHAOS_FP64, L, dOut, c);
     if (e != cudaSuccess) return c.finish(cuda_error(e, "legacy LLE kernel"));
     rc = c.to_host(out, dOut, outBytes);
     return c.finish(rc);
@@ -770,7 +784,7 @@ int chaos_lle_sweep(const chaos_exec* ex, int system, int dim, int gridMode, dou
     if ((rc = upload_log_axes(c, gridMode, dim, nPts, ranges, L.table))) return c.finish(rc);
     double* dOut = (double*)c.output(lle, L.nPoints * sizeof(double));
     if (c.failed) return c.finish(CHAOS_E_NOMEM);
-    cudaError_t e = run_lle(c.ex.precision, L, dOut, c.stream);
+    cudaError_t e = run_lle(c.ex.precision, L, dOut, c);
     if (e != cudaSuccess) return c.finish(cuda_error(e, "LLE kernel"));
     rc = c.to_host(lle, dOut, L.nPoints * sizeof(double));
     return c.finish(rc);
@@ -874,7 +888,8 @@ int chaos_lyapunov_spectrum(const chaos_exec* ex, int system, int dim, int gridM
     const size_t bytes = (size_t)L.nPoints * system_nx(system) * sizeof(double);
     double* dOut = (double*)c.output(spectrum, bytes);
     if (c.failed) return c.finish(CHAOS_E_NOMEM);
-    cudaError_t e = fp32 ? launch_spectrum_f32(L, dOut, c.stream) : launch_spectrum_f64(L, dOut, c.stream);
+    cudaError_t e = fp32 ? launch_spectrum_f32(L, dOut, c.stream, (float*)c.optional(spectrum_f32_state_bytes(L)))
+                         : launch_spectrum_f64(L, dOut, c.stream);
     if (e != cudaSuccess) return c.finish(cuda_error(e, "Lyapunov spectrum kernel"));
     rc = c.to_host(spectrum, dOut, bytes);
     return c.finish(rc);
@@ -906,7 +921,7 @@ int chaos_lle2d_checked(const chaos_exec* ex, int system, double tMax, double NT
     int* counts = (int*)c.alloc(2 * sizeof(int));
     int* list = (int*)c.alloc(n * sizeof(int));
     if (c.failed) return c.finish(CHAOS_E_NOMEM);
-    cudaError_t e = launch_lle_f32(L, dOut, c.stream);
+    cudaError_t e = run_lle(CHAOS_FP32, L, dOut, c);
     if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, 2 * sizeof(int), c.stream);
     if (e == cudaSuccess) e = launch_lle_select(dOut, n, band, list, counts, c.stream);
     int h0[2] = {0, 0};

@@ -12,6 +12,7 @@ namespace chaos {
 
 int set_error(int code, const char* fmt, ...);
 int cuda_error(cudaError_t e, const char* what);
+size_t scratch_budget_bytes();  // CHAOS_SCRATCH_BUDGET_MB
 
 // One C-ABI call: resolves the device and stream, hands out stream-ordered
 // device buffers from the library's pool (freed when the call finishes),
@@ -26,6 +27,10 @@ struct Call {
 
     int begin(const chaos_exec* e);
     void* alloc(size_t bytes);  // device scratch, freed at finish()
+    // device scratch that the call can do without: null for 0 bytes, over the
+    // scratch budget, while the stream is captured (a graph of the call stays
+    // free of allocations) or when there is no memory
+    void* optional(size_t bytes);
     const void* input(const void* user, size_t bytes);  // device view of a caller input
     void* output(void* user, size_t bytes);             // device buffer for a caller output
     int to_host(void* host, const void* dev, size_t bytes);  // copy back (host-memory calls)

@@ -874,14 +874,13 @@ __device__ __forceinline__ void twin_steps(T* x, T* e, const T* a, const RK4H<T>
     if (s < n) rk4_step_twin<F>(x, e, a, c);
 }
 
-// The Benettin blocks of an FP32 twin carried as a difference e (three state
-// components): steps(e, n) advances the orbit and e by n steps.
-template <int RN = kRenormPow2, class Steps>
-__device__ __forceinline__ double lle_twin_blocks(const LleParams& L, Steps&& steps) {
-    Stretch<RN> st = make_stretch<RN>(L);
-    float e[3] = {(float)L.eps, 0.f, 0.f};
+// The Benettin blocks b0 to b1 - 1 of an FP32 twin carried as a difference e
+// (three state components): steps(e, n) advances the orbit and e by n steps.
+template <int RN, class Steps>
+__device__ __forceinline__ void lle_twin_blocks(const LleParams& L, float* e, Stretch<RN>& st, int b0, int b1,
+                                                Steps&& steps) {
     const int nb = L.calcBlocks + 1;
-    for (int b = 0; b < nb; ++b) {
+    for (int b = b0; b < b1; ++b) {
         steps(e, L.ntp);
         if (b + 1 < nb) {
             const float r = st.renorm(e[0], e[1], e[2]);
@@ -892,16 +891,53 @@ __device__ __forceinline__ double lle_twin_blocks(const LleParams& L, Steps&& st
             st.last(e[0], e[1], e[2]);
         }
     }
-    return st.result(L.tMax);
 }
 
+// A map's point (or pair of points) as its kernels run it: from its start
+// through the transient and the blocks to its result, in one go or a slice of
+// the horizon at a time (lle_slices.h), between which words() hands its state
+// to io.
+template <class Point>
+__device__ __forceinline__ void run_point(const LleParams& L, long long p, long long q, double* outp, double* outq) {
+    Point z(L, p, q);
+    z.transient(L.trans);
+    z.blocks(L, 0, L.calcBlocks + 1);
+    z.result(L, outp, outq);
+}
+
+// FP32 LLE point of an RK4 system.
+template <class F> struct LlePoint {
+    static constexpr int kPoints = 1, kWords = 7;
+    float x[3], e[3], a[3];
+    const RK4H<float> c;
+    Stretch<kRenormPow2> st;
+    __device__ __forceinline__ LlePoint(const LleParams& L, long long p, long long)
+        : c((float)L.h), st(make_stretch<kRenormPow2>(L)) {
+        lle_load<3, 3>(L, p, x, a);
+        e[0] = (float)L.eps;
+        e[1] = 0.f;
+        e[2] = 0.f;
+    }
+    __device__ __forceinline__ void transient(int n) {
+        for (int s = 0; s < n; ++s) rk4_step<F>(x, a, c);
+    }
+    __device__ __forceinline__ void blocks(const LleParams& L, int b0, int b1) {
+        lle_twin_blocks(L, e, st, b0, b1, [&](float* d, int n) { twin_steps<F>(x, d, a, c, n); });
+    }
+    template <class IO> __device__ __forceinline__ void words(IO& io) {
+        io.word(x);
+        io.word(e);
+        io.word(st.k);
+    }
+    __device__ __forceinline__ void result(const LleParams& L, double* outp, double*) const {
+        *outp = st.result(L.tMax);
+    }
+};
 template <class F>
 __device__ __forceinline__ double lle_point_twin(const LleParams& L, long long p) {
-    float x[3], a[3];
-    lle_load<3, 3>(L, p, x, a);
-    const RK4H<float> c((float)L.h);
-    for (int s = 0; s < L.trans; ++s) rk4_step<F>(x, a, c);
-    return lle_twin_blocks(L, [&](float* e, int n) { twin_steps<F>(x, e, a, c, n); });
+    double v;
+    run_point<LlePoint<F>>(L, p, p, &v, nullptr);
+    return v;
 }
 
 // The FP32 LLE point of Chameleon (the reference's default system): the twin
@@ -911,9 +947,12 @@ __device__ __forceinline__ double lle_point_twin_chameleon(const LleParams& L, l
     lle_load<3, 7>(L, p, x, a);
     const float h = (float)L.h;
     for (int s = 0; s < L.trans; ++s) chameleon_step<float>(x, a, h);
-    return lle_twin_blocks(L, [&](float* e, int n) {
-        for (int s = 0; s < n; ++s) chameleon_step_twin<float>(x, e, a, h);
+    float e[3] = {(float)L.eps, 0.f, 0.f};
+    auto st = make_stretch<kRenormPow2>(L);
+    lle_twin_blocks(L, e, st, 0, L.calcBlocks + 1, [&](float* d, int n) {
+        for (int s = 0; s < n; ++s) chameleon_step_twin<float>(x, d, a, h);
     });
+    return st.result(L.tMax);
 }
 
 // ---------------------------------------------------------------------------
@@ -985,19 +1024,25 @@ __device__ __forceinline__ void spectrum_point_full(const LleParams& L, long lon
 // log2(|b_j|^2/eps^2) on the SFU summed in FP32 groups of kLleGroup blocks and
 // added into FP64, as the FP32 LLE map does. steps(e, n) advances the orbit
 // and the three differences by n steps.
+__device__ __forceinline__ void spectrum_start(const LleParams& L, float (*e)[3], double* sum) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) e[j][i] = i == j ? (float)L.eps : 0.f;
+        sum[j] = 0.0;
+    }
+}
+__device__ __forceinline__ double spectrum_result(const LleParams& L, double sum) {
+    return sum * (0.5 * 0.69314718055994530942) / L.tMax;
+}
+// Blocks from to to - 1; from is a multiple of kLleGroup.
 template <class Steps>
-__device__ __forceinline__ void spectrum_twin_blocks(const LleParams& L, long long p, double* out, Steps&& steps) {
-    float e[3][3];
+__device__ __forceinline__ void spectrum_twin_blocks(const LleParams& L, float (*e)[3], double* sum, int from, int to,
+                                                     Steps&& steps) {
     const float eps = (float)L.eps;
     const float inv_eps2 = (float)(1.0 / (L.eps * L.eps));
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-#pragma unroll
-        for (int i = 0; i < 3; ++i) e[j][i] = i == j ? eps : 0.f;
-    double sum[3] = {0.0, 0.0, 0.0};
-    const int nb = L.calcBlocks + 1;
-    for (int b0 = 0; b0 < nb; b0 += kLleGroup) {
-        const int bn = min(kLleGroup, nb - b0);
+    for (int b0 = from; b0 < to; b0 += kLleGroup) {
+        const int bn = min(kLleGroup, to - b0);
         float part[3] = {0.f, 0.f, 0.f};
         for (int b = 0; b < bn; ++b) {
             steps(e, L.ntp);
@@ -1027,29 +1072,50 @@ __device__ __forceinline__ void spectrum_twin_blocks(const LleParams& L, long lo
 #pragma unroll
         for (int j = 0; j < 3; ++j) sum[j] += (double)part[j];
     }
-#pragma unroll
-    for (int j = 0; j < 3; ++j) out[p * 3 + j] = sum[j] * (0.5 * 0.69314718055994530942) / L.tMax;
 }
 
-template <class F>
-__device__ __forceinline__ void spectrum_point_twin(const LleParams& L, long long p, double* out) {
-    float x[3], a[3];
-    lle_load<3, 3>(L, p, x, a);
-    const RK4H<float> c((float)L.h);
-    for (int s = 0; s < L.trans; ++s) rk4_step<F>(x, a, c);
-    spectrum_twin_blocks(L, p, out, [&](float (*e)[3], int n) {
-        for (int s = 0; s < n; ++s) rk4_step_multi<F, 3>(x, e, a, c);
-    });
-}
+// Results three to a point, at outp.
+template <class F> struct SpectrumPoint {
+    static constexpr int kPoints = 1, kWords = 18;
+    float x[3], a[3], e[3][3];
+    double sum[3];
+    const RK4H<float> c;
+    __device__ __forceinline__ SpectrumPoint(const LleParams& L, long long p, long long) : c((float)L.h) {
+        lle_load<3, 3>(L, p, x, a);
+        spectrum_start(L, e, sum);
+    }
+    __device__ __forceinline__ void transient(int n) {
+        for (int s = 0; s < n; ++s) rk4_step<F>(x, a, c);
+    }
+    __device__ __forceinline__ void blocks(const LleParams& L, int b0, int b1) {
+        spectrum_twin_blocks(L, e, sum, b0, b1, [&](float (*d)[3], int n) {
+            for (int s = 0; s < n; ++s) rk4_step_multi<F, 3>(x, d, a, c);
+        });
+    }
+    template <class IO> __device__ __forceinline__ void words(IO& io) {
+        io.word(x);
+        io.word(e);
+        io.word(sum);
+    }
+    __device__ __forceinline__ void result(const LleParams& L, double* outp, double*) const {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) outp[j] = spectrum_result(L, sum[j]);
+    }
+};
 
 __device__ __forceinline__ void spectrum_point_twin_chameleon(const LleParams& L, long long p, double* out) {
     float x[3], a[7];
     lle_load<3, 7>(L, p, x, a);
     const float h = (float)L.h;
     for (int s = 0; s < L.trans; ++s) chameleon_step<float>(x, a, h);
-    spectrum_twin_blocks(L, p, out, [&](float (*e)[3], int n) {
-        for (int s = 0; s < n; ++s) chameleon_step_multi<float, 3>(x, e, a, h);
+    float e[3][3];
+    double sum[3];
+    spectrum_start(L, e, sum);
+    spectrum_twin_blocks(L, e, sum, 0, L.calcBlocks + 1, [&](float (*d)[3], int n) {
+        for (int s = 0; s < n; ++s) chameleon_step_multi<float, 3>(x, d, a, h);
     });
+#pragma unroll
+    for (int j = 0; j < 3; ++j) out[p * 3 + j] = spectrum_result(L, sum[j]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1089,70 +1155,103 @@ template <> struct RK4H<P2> {
 };
 
 // Two LLE points per thread (indices p and q), lanes of P2. Same arithmetic
-// per lane as lle_point_twin with T = float; the per-block stretch and
-// renormalisation (Stretch mode RN) run per lane.
-template <class F, int RN = kRenormPow2>
-__device__ __forceinline__ void lle_pair_twin(const LleParams& L, long long p, long long q, double* outp,
-                                              double* outq) {
+// per lane as LlePoint; the per-block stretch and renormalisation (Stretch
+// mode RN) run per lane.
+template <class F, int RN = kRenormPow2> struct LlePair {
+    static constexpr int kPoints = 2, kWords = 14;
     P2 x[3], e[3], a[3];
-    float xs[2][3], as[2][3];
-    lle_load<3, 3>(L, p, xs[0], as[0]);
-    lle_load<3, 3>(L, q, xs[1], as[1]);
+    const RK4H<P2> c;
+    Stretch<RN> s0, s1;
+    __device__ __forceinline__ LlePair(const LleParams& L, long long p, long long q)
+        : c((float)L.h), s0(make_stretch<RN>(L)), s1(make_stretch<RN>(L)) {
+        float xs[2][3], as[2][3];
+        lle_load<3, 3>(L, p, xs[0], as[0]);
+        lle_load<3, 3>(L, q, xs[1], as[1]);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        a[k] = P2(as[0][k], as[1][k]);
-        x[k] = P2(xs[0][k], xs[1][k]);
+        for (int k = 0; k < 3; ++k) {
+            a[k] = P2(as[0][k], as[1][k]);
+            x[k] = P2(xs[0][k], xs[1][k]);
+        }
+        const float eps = (float)L.eps;
+        e[0] = P2((double)eps);
+        e[1] = P2(0.0);
+        e[2] = P2(0.0);
     }
-    const RK4H<P2> c((float)L.h);
-    for (int s = 0; s < L.trans; ++s) rk4_step<F>(x, a, c);
-    const float eps = (float)L.eps;
-    e[0] = P2((double)eps);
-    e[1] = P2(0.0);
-    e[2] = P2(0.0);
-    Stretch<RN> s0 = make_stretch<RN>(L), s1 = make_stretch<RN>(L);
-    const int nb = L.calcBlocks + 1;
-    for (int b = 0; b < nb; ++b) {
-        twin_steps<F>(x, e, a, c, L.ntp);
-        if (b + 1 < nb) {
-            const P2 r(s0.renorm(e[0].v.x, e[1].v.x, e[2].v.x), s1.renorm(e[0].v.y, e[1].v.y, e[2].v.y));
-            e[0] *= r;
-            e[1] *= r;
-            e[2] *= r;
-        } else {
-            s0.last(e[0].v.x, e[1].v.x, e[2].v.x);
-            s1.last(e[0].v.y, e[1].v.y, e[2].v.y);
+    __device__ __forceinline__ void transient(int n) {
+        for (int s = 0; s < n; ++s) rk4_step<F>(x, a, c);
+    }
+    __device__ __forceinline__ void blocks(const LleParams& L, int b0, int b1) {
+        const int nb = L.calcBlocks + 1;
+        for (int b = b0; b < b1; ++b) {
+            twin_steps<F>(x, e, a, c, L.ntp);
+            if (b + 1 < nb) {
+                const P2 r(s0.renorm(e[0].v.x, e[1].v.x, e[2].v.x), s1.renorm(e[0].v.y, e[1].v.y, e[2].v.y));
+                e[0] *= r;
+                e[1] *= r;
+                e[2] *= r;
+            } else {
+                s0.last(e[0].v.x, e[1].v.x, e[2].v.x);
+                s1.last(e[0].v.y, e[1].v.y, e[2].v.y);
+            }
         }
     }
-    *outp = s0.result(L.tMax);
-    if (outq) *outq = s1.result(L.tMax);
-}
-
-// Two spectrum points per thread (indices p and q; q == p writes once), lanes
-// of P2: spectrum_point_twin per lane, Gram-Schmidt packed too, with the
-// divisions, logs and reciprocal roots per lane.
-template <class F>
-__device__ __forceinline__ void spectrum_pair_twin(const LleParams& L, long long p, long long q, double* out) {
-    P2 x[3], a[3], e[3][3];
-    float xs[2][3], as[2][3];
-    lle_load<3, 3>(L, p, xs[0], as[0]);
-    lle_load<3, 3>(L, q, xs[1], as[1]);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        a[k] = P2(as[0][k], as[1][k]);
-        x[k] = P2(xs[0][k], xs[1][k]);
+    template <class IO> __device__ __forceinline__ void words(IO& io) {
+        io.word(x);
+        io.word(e);
+        io.word(s0.k);
+        io.word(s1.k);
     }
-    const RK4H<P2> c((float)L.h);
-    for (int s = 0; s < L.trans; ++s) rk4_step<F>(x, a, c);
+    __device__ __forceinline__ void result(const LleParams& L, double* outp, double* outq) const {
+        *outp = s0.result(L.tMax);
+        if (outq) *outq = s1.result(L.tMax);
+    }
+};
+
+// Two spectrum points per thread (indices p and q), lanes of P2: SpectrumPoint
+// per lane, Gram-Schmidt packed too, with the
+// divisions, logs and reciprocal roots per lane.
+template <class F> struct SpectrumPair {
+    static constexpr int kPoints = 2, kWords = 36;
+    P2 x[3], a[3], e[3][3];
+    double sum[2][3];
+    const RK4H<P2> c;
+    __device__ __forceinline__ SpectrumPair(const LleParams& L, long long p, long long q) : c((float)L.h) {
+        float xs[2][3], as[2][3];
+        lle_load<3, 3>(L, p, xs[0], as[0]);
+        lle_load<3, 3>(L, q, xs[1], as[1]);
+        const float eps = (float)L.eps;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            a[k] = P2(as[0][k], as[1][k]);
+            x[k] = P2(xs[0][k], xs[1][k]);
+            sum[0][k] = sum[1][k] = 0.0;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) e[k][i] = i == k ? P2(eps, eps) : P2(0.0);
+        }
+    }
+    __device__ __forceinline__ void transient(int n) {
+        for (int s = 0; s < n; ++s) rk4_step<F>(x, a, c);
+    }
+    template <class IO> __device__ __forceinline__ void words(IO& io) {
+        io.word(x);
+        io.word(e);
+        io.word(sum);
+    }
+    __device__ __forceinline__ void result(const LleParams& L, double* outp, double* outq) const {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) outp[j] = spectrum_result(L, sum[0][j]);
+        if (outq) {
+#pragma unroll
+            for (int j = 0; j < 3; ++j) outq[j] = spectrum_result(L, sum[1][j]);
+        }
+    }
+    __device__ __forceinline__ void blocks(const LleParams& L, int from, int to);
+};
+template <class F> __device__ __forceinline__ void SpectrumPair<F>::blocks(const LleParams& L, int from, int to) {
     const float eps = (float)L.eps;
     const float inv_eps2 = (float)(1.0 / (L.eps * L.eps));
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-#pragma unroll
-        for (int i = 0; i < 3; ++i) e[j][i] = i == j ? P2(eps, eps) : P2(0.0);
-    double sum[2][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
-    const int nb = L.calcBlocks + 1;
-    for (int b0 = 0; b0 < nb; b0 += kLleGroup) {
-        const int bn = min(kLleGroup, nb - b0);
+    for (int b0 = from; b0 < to; b0 += kLleGroup) {
+        const int bn = min(kLleGroup, to - b0);
         P2 part[3] = {P2(0.0), P2(0.0), P2(0.0)};
         for (int b = 0; b < bn; ++b) {
             for (int s = 0; s < L.ntp; ++s) rk4_step_multi<F, 3>(x, e, a, c);
@@ -1186,12 +1285,6 @@ __device__ __forceinline__ void spectrum_pair_twin(const LleParams& L, long long
             sum[0][j] += (double)part[j].v.x;
             sum[1][j] += (double)part[j].v.y;
         }
-    }
-#pragma unroll
-    for (int l = 0; l < 2; ++l) {
-        const long long o = l ? q : p;
-#pragma unroll
-        for (int j = 0; j < 3; ++j) out[o * 3 + j] = sum[l][j] * (0.5 * 0.69314718055994530942) / L.tMax;
     }
 }
 

@@ -7,6 +7,7 @@
 #include <cstdlib>
 
 #include "engine.cuh"
+#include "lle_slices.h"
 #include "sweep_launch.h"
 
 namespace chaos {
@@ -61,16 +62,19 @@ __global__ void __launch_bounds__(kBlock) trajectory_kernel_f32(const double* x0
 }
 
 // Two points per thread in packed FP32x2 lanes, the first `singles` blocks one.
-// Bound by the FMA pipe; 120 registers, four blocks per SM (a cap at 80 spills:
-// 384^2 Lorenz points, 2,510 steps, 2.28 ms uncapped, 2.33 at five blocks,
-// 2.65 at six; a point per thread 2.52).
+// Bound by the FMA pipe; 124 registers (Lorenz), four blocks per SM. 7.58 rows of
+// Lorenz points per SM, 3,510 steps: 3.31 ms asked for three blocks, 3.35 asked
+// for none or four, 3.89 at six (80 registers: spills).
 template <class F>
-__global__ void __launch_bounds__(kBlock) spectrum_pair_kernel_f32(LleParams L, double* out, unsigned singles) {
+__global__ void __launch_bounds__(kBlock, 3) spectrum_pair_kernel_f32(LleParams L, double* out, unsigned singles) {
     bool pair;
     const long long o = mixed_point(singles, pair);
     if (o >= L.nPoints) return;
-    if (pair) spectrum_pair_twin<F>(L, L.pBegin + o, L.pBegin + (o + 1 < L.nPoints ? o + 1 : o), out);
-    else spectrum_point_twin<F>(L, L.pBegin + o, out);
+    const long long p = L.pBegin + o;
+    const bool two = pair && o + 1 < L.nPoints;
+    double* outp = out + 3 * p;
+    if (pair) run_point<SpectrumPair<F>>(L, p, two ? p + 1 : p, outp, two ? outp + 3 : nullptr);
+    else run_point<SpectrumPoint<F>>(L, p, p, outp, nullptr);
 }
 
 // Bifurcation / basins, two points per thread in packed FP32x2 lanes (RK4
@@ -228,11 +232,14 @@ cudaError_t launch_bif_list_f32(const SweepParams& P, const BifOut& O, const int
 // outside the step loop; the 1024^2 Rössler map went from 133.7 to 128.6 ms
 // (from 3.37 waves of resident blocks to 2.99) and the Lorenz map from 39.1
 // to 36.2 ms, results unchanged. Blocks of 64, 128 and 256 (the tuner's
-// choices) all launch under the bound.
+// choices) all launch under the bound. Chen's step keeps more and is the faster
+// for 128 registers: 4 rows of 128 points per SM (5,510 steps) 1.42 -> 1.38 ms, 60
+// rows 20.2 -> 19.9 (Lorenz at 128 1.23 -> 1.30).
 // singles: the first blocks, which run one point per thread (single_blocks),
 // with the default renormalisation only.
 template <class F, int RN = kRenormPow2>
-__global__ void __launch_bounds__(384, 3) lle_pair_kernel_f32(LleParams L, double* out, unsigned singles) {
+__global__ void __launch_bounds__(std::is_same<F, Chen>::value ? kMaxBlock : 384, std::is_same<F, Chen>::value ? 2 : 3)
+lle_pair_kernel_f32(LleParams L, double* out, unsigned singles) {
     bool pair;
     const long long o = mixed_point(singles, pair);
     if (o >= L.nPoints) return;
@@ -241,7 +248,23 @@ __global__ void __launch_bounds__(384, 3) lle_pair_kernel_f32(LleParams L, doubl
         return;
     }
     const bool two = o + 1 < L.nPoints;
-    lle_pair_twin<F, RN>(L, L.pBegin + o, L.pBegin + (two ? o + 1 : o), out + o, two ? out + o + 1 : nullptr);
+    run_point<LlePair<F, RN>>(L, L.pBegin + o, L.pBegin + (two ? o + 1 : o), out + o, two ? out + o + 1 : nullptr);
+}
+
+// A slice of the jobs whose turn it is (lle_slices.h). At the 56 registers of
+// the kernel above this one spills in its loops, and a launch never has more
+// than four blocks per SM: 4.2 rows of Lorenz points, 10,510 steps, 2.99 ms at
+// 56 registers, 2.91 at 80, 2.85 at 128 (unsliced 3.06). The spectrum likewise:
+// 8.2 rows, 3,510 steps, 3.73 ms at 128 registers, 3.65 above (unsliced 4.14).
+template <class F>
+__global__ void __launch_bounds__(kBlock, 4) lle_slice_kernel_f32(LleParams L, SlicePlan plan, long long turn,
+                                                                  float* state, double* out) {
+    run_slice<LlePair<F>, LlePoint<F>>(L, plan, turn, state, out, 1);
+}
+template <class F>
+__global__ void __launch_bounds__(kBlock, 2) spectrum_slice_kernel_f32(LleParams L, SlicePlan plan, long long turn,
+                                                                    float* state, double* out) {
+    run_slice<SpectrumPair<F>, SpectrumPoint<F>>(L, plan, turn, state, out + 3 * L.pBegin, 3);
 }
 
 // Stretch mode of the FP32 LLE maps of the RK4 systems (LleRenorm): 0 the
@@ -250,8 +273,12 @@ __global__ void __launch_bounds__(384, 3) lle_pair_kernel_f32(LleParams L, doubl
 std::atomic<int> g_lle_renorm{0};
 
 template <class F>
-static void launch_twin(const LleParams& L, double* out, cudaStream_t st, int minb, int block) {
+static void launch_twin(const LleParams& L, double* out, cudaStream_t st, int minb, int block, float* state) {
     const int rn = g_lle_renorm.load(std::memory_order_relaxed);
+    if (minb == 0 && rn == kRenormPow2 && state) {
+        const SlicePlan plan = slice_plan(L, kSliceLle);
+        if (plan.jobs > 0) return launch_slices(plan, lle_slice_kernel_f32<F>, L, out, state, st);
+    }
     const unsigned gp = grid_of((L.nPoints + 1) / 2, minb == 2 ? block : kBlock);
     const int bp = minb == 2 ? block : kBlock;
     const unsigned singles = single_blocks(L.nPoints);
@@ -287,19 +314,32 @@ int set_lle_renorm(int v) {
 }
 int get_lle_renorm() { return g_lle_renorm.load(); }
 
-cudaError_t launch_lle_f32(const LleParams& L, double* out, cudaStream_t st) {
+// an explicit variant (chaos_set_tuning / CHAOS_LLE_MINB) wins, then a tuned
+// shape; 0: neither
+static int lle_form(int system, int& block) {
+    block = kBlock;
+    if (lle_variant_forced()) return lle_occupancy_variant(system);
+    const int shape = shape_of(2, system);
+    if (shape / 1024 == 2) block = shape % 1024;
+    return shape / 1024;
+}
+
+size_t lle_f32_state_bytes(const LleParams& L) {
+    int block;
+    if (!system_has_difference_form(L.system) || lle_form(L.system, block) != 0 || get_lle_renorm() != kRenormPow2)
+        return 0;
+    const SlicePlan plan = slice_plan(L, kSliceLle);
+    return plan.words(plan.points == 2 ? LlePair<Lorenz>::kWords : LlePoint<Lorenz>::kWords) * sizeof(float);
+}
+
+cudaError_t launch_lle_f32(const LleParams& L, double* out, cudaStream_t st, float* state) {
     if (L.nPoints <= 0) return cudaSuccess;
-    // an explicit variant (chaos_set_tuning / CHAOS_LLE_MINB) wins, then a tuned shape
-    int minb = lle_variant_forced() ? lle_occupancy_variant(L.system) : 0, block = kBlock;
-    const int shape = shape_of(2, L.system);
-    if (shape && !lle_variant_forced()) {
-        minb = shape / 1024;
-        block = minb == 2 ? shape % 1024 : kBlock;
-    }
+    int block;
+    const int minb = lle_form(L.system, block);
     switch (L.system) {
-        case SYS_LORENZ_RK4: launch_twin<Lorenz>(L, out, st, minb, block); break;
-        case SYS_ROSSLER_RK4: launch_twin<Rossler>(L, out, st, minb, block); break;
-        case SYS_CHEN_RK4: launch_twin<Chen>(L, out, st, minb, block); break;
+        case SYS_LORENZ_RK4: launch_twin<Lorenz>(L, out, st, minb, block, state); break;
+        case SYS_ROSSLER_RK4: launch_twin<Rossler>(L, out, st, minb, block, state); break;
+        case SYS_CHEN_RK4: launch_twin<Chen>(L, out, st, minb, block, state); break;
         case SYS_CHAMELEON:
             lle_chameleon_kernel_f32<<<grid_for(L.nPoints), kBlock, 0, st>>>(L, out);
             note_launch();
@@ -309,21 +349,32 @@ cudaError_t launch_lle_f32(const LleParams& L, double* out, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-template <class F> static void launch_spectrum(const LleParams& L, double* out, cudaStream_t st) {
+template <class F> static void launch_spectrum(const LleParams& L, double* out, cudaStream_t st, float* state) {
+    const SlicePlan plan = state ? slice_plan(L, kSliceSpectrum) : SlicePlan{};
+    if (plan.jobs > 0) return launch_slices(plan, spectrum_slice_kernel_f32<F>, L, out, state, st);
     const unsigned singles = single_blocks(L.nPoints);
     spectrum_pair_kernel_f32<F><<<mixed_grid(L.nPoints, singles), kBlock, 0, st>>>(L, out, singles);
+    note_launch();
 }
 
-cudaError_t launch_spectrum_f32(const LleParams& L, double* out, cudaStream_t st) {
+size_t spectrum_f32_state_bytes(const LleParams& L) {
+    if (!system_has_difference_form(L.system)) return 0;
+    const SlicePlan plan = slice_plan(L, kSliceSpectrum);
+    return plan.words(plan.points == 2 ? SpectrumPair<Lorenz>::kWords : SpectrumPoint<Lorenz>::kWords) * sizeof(float);
+}
+
+cudaError_t launch_spectrum_f32(const LleParams& L, double* out, cudaStream_t st, float* state) {
     if (L.nPoints <= 0) return cudaSuccess;
     switch (L.system) {
-        case SYS_LORENZ_RK4: launch_spectrum<Lorenz>(L, out, st); break;
-        case SYS_ROSSLER_RK4: launch_spectrum<Rossler>(L, out, st); break;
-        case SYS_CHEN_RK4: launch_spectrum<Chen>(L, out, st); break;
-        case SYS_CHAMELEON: spectrum_chameleon_kernel_f32<<<grid_for(L.nPoints), kBlock, 0, st>>>(L, out); break;
+        case SYS_LORENZ_RK4: launch_spectrum<Lorenz>(L, out, st, state); break;
+        case SYS_ROSSLER_RK4: launch_spectrum<Rossler>(L, out, st, state); break;
+        case SYS_CHEN_RK4: launch_spectrum<Chen>(L, out, st, state); break;
+        case SYS_CHAMELEON:
+            spectrum_chameleon_kernel_f32<<<grid_for(L.nPoints), kBlock, 0, st>>>(L, out);
+            note_launch();
+            break;
         default: return cudaErrorNotSupported;
     }
-    note_launch();
     return cudaGetLastError();
 }
 

@@ -21,6 +21,7 @@
 #include "batch.h"
 #include "batch_group.cuh"
 #include "engine.cuh"
+#include "lle_slices.h"
 #include "sweep_launch.h"
 
 namespace chaos {
@@ -33,16 +34,16 @@ __device__ __forceinline__ int exp_of(float v) { return (int)((__float_as_uint(v
 
 __device__ __forceinline__ double finite_or_nan(double v) { return isfinite(v) ? v : __longlong_as_double(0x7ff8000000000000LL); }
 
-// The Benettin blocks of an FF orbit x with the FP32 twin difference e
-// (started where the caller put it), renormalised by powers of two; the
-// stretch of the blocks relative to eps, as the reference measures it.
+// The Benettin blocks b0 to b1 - 1 of an FF orbit x with the FP32 twin
+// difference e (started where the caller put it), renormalised by powers of
+// two; ktot sums the octaves.
 template <class F, bool FUSED = true>
-__device__ __forceinline__ double ff_benettin(const LleParams& L, FF<float>* x, float* e, const FF<float>* a,
-                                              const float* af, const FFH<float>& c, const RK4H<float>& cf) {
+__device__ __forceinline__ void ff_benettin(const LleParams& L, FF<float>* x, float* e, int& ktot, const FF<float>* a,
+                                            const float* af, const FFH<float>& c, const RK4H<float>& cf, int b0,
+                                            int b1) {
     const int eps2Exp = exp_of((float)L.eps * (float)L.eps);
-    int ktot = 0;
     const int nb = L.calcBlocks + 1;
-    for (int b = 0; b < nb; ++b) {
+    for (int b = b0; b < b1; ++b) {
         for (int s = 0; s < L.ntp; ++s) ff_rk4_step<F, true, FUSED>(x, e, a, af, c, cf);
         if (b + 1 < nb) {
             const float n2 = fmaf(e[0], e[0], fmaf(e[1], e[1], e[2] * e[2]));
@@ -54,7 +55,10 @@ __device__ __forceinline__ double ff_benettin(const LleParams& L, FF<float>* x, 
             ktot += k;
         }
     }
-    const double n2 = (double)e[0] * e[0] + (double)e[1] * e[1] + (double)e[2] * e[2];
+}
+// The stretch of the blocks relative to eps, as the reference measures it.
+__device__ __forceinline__ double ff_exponent(const LleParams& L, int ktot, float e0, float e1, float e2) {
+    const double n2 = (double)e0 * e0 + (double)e1 * e1 + (double)e2 * e2;
     return finite_or_nan(pow2_log_stretch(ktot, n2, L.eps) / L.tMax);
 }
 
@@ -66,24 +70,39 @@ __device__ __forceinline__ FFH<float> ff_consts(double h) {
     return c;
 }
 
-template <class F>
-__device__ __forceinline__ double lle_point_ff(const LleParams& L, long long p) {
-    double xd[3], ad[3];
-    lle_load<3, 3>(L, p, xd, ad);
+template <class F> struct FFPoint {
+    static constexpr int kPoints = 1, kWords = 10;
     FF<float> x[3], a[3];
-    float af[3];
+    float af[3], e[3];
+    int k = 0;
+    const FFH<float> c;
+    const RK4H<float> cf;
+    __device__ __forceinline__ FFPoint(const LleParams& L, long long p, long long) : c(ff_consts(L.h)), cf((float)L.h) {
+        double xd[3], ad[3];
+        lle_load<3, 3>(L, p, xd, ad);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        x[k] = ff_from_double(xd[k]);
-        a[k] = ff_from_double(ad[k]);
-        af[k] = (float)ad[k];
+        for (int i = 0; i < 3; ++i) {
+            x[i] = ff_from_double(xd[i]);
+            a[i] = ff_from_double(ad[i]);
+            af[i] = (float)ad[i];
+            e[i] = i == 0 ? (float)L.eps : 0.f;
+        }
     }
-    const FFH<float> c = ff_consts(L.h);
-    const RK4H<float> cf((float)L.h);
-    for (int s = 0; s < L.trans; ++s) ff_rk4_step<F, false>(x, (float*)nullptr, a, af, c, cf);
-    float e[3] = {(float)L.eps, 0.f, 0.f};
-    return ff_benettin<F>(L, x, e, a, af, c, cf);
-}
+    __device__ __forceinline__ void transient(int n) {
+        for (int s = 0; s < n; ++s) ff_rk4_step<F, false>(x, (float*)nullptr, a, af, c, cf);
+    }
+    __device__ __forceinline__ void blocks(const LleParams& L, int b0, int b1) {
+        ff_benettin<F>(L, x, e, k, a, af, c, cf, b0, b1);
+    }
+    template <class IO> __device__ __forceinline__ void words(IO& io) {
+        io.word(x);
+        io.word(e);
+        io.word(k);
+    }
+    __device__ __forceinline__ void result(const LleParams& L, double* outp, double*) const {
+        *outp = ff_exponent(L, k, e[0], e[1], e[2]);
+    }
+};
 
 // From caller-supplied starting states (the reference's semi_result layout:
 // orbit, parameters, twin): the twin difference is q - x, exact in FP64 for
@@ -102,64 +121,76 @@ __global__ void __launch_bounds__(kBlock) lle_ff_states_kernel(LleParams L, cons
         af[i] = (float)r[3 + i];
         e[i] = (float)(r[6 + i] - r[i]);
     }
-    out[k] = ff_benettin<F, false>(L, x, e, a, af, ff_consts(L.h), RK4H<float>((float)L.h));
+    int ktot = 0;
+    ff_benettin<F, false>(L, x, e, ktot, a, af, ff_consts(L.h), RK4H<float>((float)L.h), 0, L.calcBlocks + 1);
+    out[k] = ff_exponent(L, ktot, e[0], e[1], e[2]);
 }
 
 // Two points per thread: FF words are packed pairs (one paired FP32
 // instruction per word operation for both points).
-template <class F>
-__device__ __forceinline__ void lle_pair_ff(const LleParams& L, long long p, long long q, double* outp, double* outq) {
-    double xd[2][3], ad[2][3];
-    lle_load<3, 3>(L, p, xd[0], ad[0]);
-    lle_load<3, 3>(L, q, xd[1], ad[1]);
+template <class F> struct FFPair {
+    static constexpr int kPoints = 2, kWords = 20;
     FF<P2> x[3], a[3];
-    P2 af[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const FF<float> x0 = ff_from_double(xd[0][k]), x1 = ff_from_double(xd[1][k]);
-        const FF<float> a0 = ff_from_double(ad[0][k]), a1 = ff_from_double(ad[1][k]);
-        x[k] = ff_make(P2(x0.hi, x1.hi), P2(x0.lo, x1.lo));
-        a[k] = ff_make(P2(a0.hi, a1.hi), P2(a0.lo, a1.lo));
-        af[k] = P2((float)ad[0][k], (float)ad[1][k]);
-    }
-    FFH<P2> c;
-    {
-        const FF<float> hh = ff_from_double(L.h * 0.5), h = ff_from_double(L.h), h6 = ff_from_double(L.h / 6.0);
-        c.hh = ff_make(P2(hh.hi, hh.hi), P2(hh.lo, hh.lo));
-        c.h = ff_make(P2(h.hi, h.hi), P2(h.lo, h.lo));
-        c.h6 = ff_make(P2(h6.hi, h6.hi), P2(h6.lo, h6.lo));
-    }
-    const RK4H<P2> cf((float)L.h);
-    for (int s = 0; s < L.trans; ++s) ff_rk4_step<F, false>(x, (P2*)nullptr, a, af, c, cf);
-    const float e0 = (float)L.eps;
-    const int eps2Exp = exp_of(e0 * e0);
-    P2 e[3] = {P2(e0, e0), P2(0.f, 0.f), P2(0.f, 0.f)};
+    P2 af[3], e[3];
     int k0 = 0, k1 = 0;
-    const int nb = L.calcBlocks + 1;
-    for (int b = 0; b < nb; ++b) {
-        for (int s = 0; s < L.ntp; ++s) ff_rk4_step<F, true>(x, e, a, af, c, cf);
-        if (b + 1 < nb) {
-            const P2 n2 = fmaT(e[0], e[0], fmaT(e[1], e[1], e[2] * e[2]));
-            const int j0 = pow2_rescale_exponent(n2.v.x, eps2Exp), j1 = pow2_rescale_exponent(n2.v.y, eps2Exp);
-            const P2 sc(pow2_scale(j0), pow2_scale(j1));
-            e[0] *= sc;
-            e[1] *= sc;
-            e[2] *= sc;
-            k0 += j0;
-            k1 += j1;
+    FFH<P2> c;
+    const RK4H<P2> cf;
+    __device__ __forceinline__ FFPair(const LleParams& L, long long p, long long q) : cf((float)L.h) {
+        double xd[2][3], ad[2][3];
+        lle_load<3, 3>(L, p, xd[0], ad[0]);
+        lle_load<3, 3>(L, q, xd[1], ad[1]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const FF<float> x0 = ff_from_double(xd[0][k]), x1 = ff_from_double(xd[1][k]);
+            const FF<float> a0 = ff_from_double(ad[0][k]), a1 = ff_from_double(ad[1][k]);
+            x[k] = ff_make(P2(x0.hi, x1.hi), P2(x0.lo, x1.lo));
+            a[k] = ff_make(P2(a0.hi, a1.hi), P2(a0.lo, a1.lo));
+            af[k] = P2((float)ad[0][k], (float)ad[1][k]);
+            e[k] = k == 0 ? P2((float)L.eps, (float)L.eps) : P2(0.f, 0.f);
+        }
+        const FFH<float> f = ff_consts(L.h);
+        c.hh = ff_make(P2(f.hh.hi, f.hh.hi), P2(f.hh.lo, f.hh.lo));
+        c.h = ff_make(P2(f.h.hi, f.h.hi), P2(f.h.lo, f.h.lo));
+        c.h6 = ff_make(P2(f.h6.hi, f.h6.hi), P2(f.h6.lo, f.h6.lo));
+    }
+    __device__ __forceinline__ void transient(int n) {
+        for (int s = 0; s < n; ++s) ff_rk4_step<F, false>(x, (P2*)nullptr, a, af, c, cf);
+    }
+    __device__ __forceinline__ void blocks(const LleParams& L, int b0, int b1) {
+        const float eps = (float)L.eps;
+        const int eps2Exp = exp_of(eps * eps);
+        const int nb = L.calcBlocks + 1;
+        for (int b = b0; b < b1; ++b) {
+            for (int s = 0; s < L.ntp; ++s) ff_rk4_step<F, true>(x, e, a, af, c, cf);
+            if (b + 1 < nb) {
+                const P2 n2 = fmaT(e[0], e[0], fmaT(e[1], e[1], e[2] * e[2]));
+                const int j0 = pow2_rescale_exponent(n2.v.x, eps2Exp), j1 = pow2_rescale_exponent(n2.v.y, eps2Exp);
+                const P2 sc(pow2_scale(j0), pow2_scale(j1));
+                e[0] *= sc;
+                e[1] *= sc;
+                e[2] *= sc;
+                k0 += j0;
+                k1 += j1;
+            }
         }
     }
-    const double n0 = (double)e[0].v.x * e[0].v.x + (double)e[1].v.x * e[1].v.x + (double)e[2].v.x * e[2].v.x;
-    const double n1 = (double)e[0].v.y * e[0].v.y + (double)e[1].v.y * e[1].v.y + (double)e[2].v.y * e[2].v.y;
-    *outp = finite_or_nan(pow2_log_stretch(k0, n0, L.eps) / L.tMax);
-    if (outq) *outq = finite_or_nan(pow2_log_stretch(k1, n1, L.eps) / L.tMax);
-}
+    template <class IO> __device__ __forceinline__ void words(IO& io) {
+        io.word(x);
+        io.word(e);
+        io.word(k0);
+        io.word(k1);
+    }
+    __device__ __forceinline__ void result(const LleParams& L, double* outp, double* outq) const {
+        *outp = ff_exponent(L, k0, e[0].v.x, e[1].v.x, e[2].v.x);
+        if (outq) *outq = ff_exponent(L, k1, e[0].v.y, e[1].v.y, e[2].v.y);
+    }
+};
 
 template <class F>
 __global__ void __launch_bounds__(kBlock) lle_ff_kernel(LleParams L, double* out) {
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= L.nPoints) return;
-    out[o] = lle_point_ff<F>(L, L.pBegin + o);
+    run_point<FFPoint<F>>(L, L.pBegin + o, L.pBegin + o, out + o, nullptr);
 }
 
 // Two points per thread, the first `singles` blocks one. The FMA pipe bounds
@@ -175,11 +206,19 @@ __global__ void __launch_bounds__(kBlock, 2) lle_ff_pair_kernel(LleParams L, dou
     const long long o = mixed_point(singles, pair);
     if (o >= L.nPoints) return;
     if (!pair) {
-        out[o] = lle_point_ff<F>(L, L.pBegin + o);
+        run_point<FFPoint<F>>(L, L.pBegin + o, L.pBegin + o, out + o, nullptr);
         return;
     }
     const bool two = o + 1 < L.nPoints;
-    lle_pair_ff<F>(L, L.pBegin + o, L.pBegin + (two ? o + 1 : o), out + o, two ? out + o + 1 : nullptr);
+    run_point<FFPair<F>>(L, L.pBegin + o, L.pBegin + (two ? o + 1 : o), out + o, two ? out + o + 1 : nullptr);
+}
+
+// A slice of the jobs whose turn it is (lle_slices.h), with as many registers
+// as the kernel above.
+template <class F>
+__global__ void __launch_bounds__(kBlock, 2) lle_ff_slice_kernel(LleParams L, SlicePlan plan, long long turn, float* state,
+                                                              double* out) {
+    run_slice<FFPair<F>, FFPoint<F>>(L, plan, turn, state, out, 1);
 }
 
 // FF trajectory of an RK4 system: out[t][s][k] = hi + lo of component k after
@@ -213,8 +252,7 @@ __global__ void __launch_bounds__(kBlock) trajectory_kernel_ff(const double* x0,
 
 // Persistent kernel of a batch's float-float LLE jobs of one system
 // (CHAOS_JOB_LLE2D_FF32): pulls chunks of two blocks' worth of points from
-// its counter; every point runs lle_pair_ff, the single-sweep kernel's device
-// function, with the job's parameters staged in shared memory.
+// its counter; every point runs FFPair, as in the single-sweep kernel, with the job's parameters staged in shared memory.
 template <class F>
 __global__ void __launch_bounds__(kBlock) group_ff_kernel(const JobDesc* __restrict__ jobs,
                                                           const Chunk* __restrict__ chunks, int count, int* counter) {
@@ -234,7 +272,7 @@ __global__ void __launch_bounds__(kBlock) group_ff_kernel(const JobDesc* __restr
         for (int t = 2 * threadIdx.x; t < ch.count; t += 2 * blockDim.x) {
             const long long p = ch.begin + t;
             const bool two = t + 1 < ch.count;
-            lle_pair_ff<F>(sL, p, two ? p + 1 : p, J.lle + p, two ? J.lle + p + 1 : nullptr);
+            run_point<FFPair<F>>(sL, p, two ? p + 1 : p, J.lle + p, two ? J.lle + p + 1 : nullptr);
         }
     }
 }
@@ -257,7 +295,18 @@ unsigned blocks_for(long long threads) { return (unsigned)((threads + kBlock - 1
 // the scalar operation does).
 std::atomic<int> g_ff_pairs{1};
 
-template <class F> void launch_ff(const LleParams& L, double* out, cudaStream_t st) {
+bool ff_sliced(const LleParams& L, SlicePlan& plan) {
+    if (!g_ff_pairs.load(std::memory_order_relaxed)) return false;
+    plan = slice_plan(L, kSliceFF);
+    return plan.jobs > 0;
+}
+
+template <class F> void launch_ff(const LleParams& L, double* out, float* state, cudaStream_t st) {
+    SlicePlan plan;
+    if (state && ff_sliced(L, plan)) {
+        launch_slices(plan, lle_ff_slice_kernel<F>, L, out, state, st);
+        return;
+    }
     const unsigned singles = single_blocks(L.nPoints);
     if (g_ff_pairs.load(std::memory_order_relaxed))
         lle_ff_pair_kernel<F><<<mixed_grid(L.nPoints, singles), kBlock, 0, st>>>(L, out, singles);
@@ -273,12 +322,18 @@ int set_ff_pairs(int v) {
 }
 int get_ff_pairs() { return g_ff_pairs.load(); }
 
-cudaError_t launch_lle_ff(const LleParams& L, double* out, cudaStream_t st) {
+size_t lle_ff_state_bytes(const LleParams& L) {
+    SlicePlan plan;
+    if (!system_has_difference_form(L.system) || !ff_sliced(L, plan)) return 0;
+    return plan.words(plan.points == 2 ? FFPair<Lorenz>::kWords : FFPoint<Lorenz>::kWords) * sizeof(float);
+}
+
+cudaError_t launch_lle_ff(const LleParams& L, double* out, cudaStream_t st, float* state) {
     if (L.nPoints <= 0) return cudaSuccess;
     switch (L.system) {
-        case SYS_LORENZ_RK4: launch_ff<Lorenz>(L, out, st); break;
-        case SYS_ROSSLER_RK4: launch_ff<Rossler>(L, out, st); break;
-        case SYS_CHEN_RK4: launch_ff<Chen>(L, out, st); break;
+        case SYS_LORENZ_RK4: launch_ff<Lorenz>(L, out, state, st); break;
+        case SYS_ROSSLER_RK4: launch_ff<Rossler>(L, out, state, st); break;
+        case SYS_CHEN_RK4: launch_ff<Chen>(L, out, state, st); break;
         default: return cudaErrorNotSupported;
     }
     return cudaGetLastError();

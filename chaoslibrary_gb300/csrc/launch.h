@@ -114,9 +114,13 @@ cudaError_t launch_lle_f64(const LleParams& L, double* out, cudaStream_t st);
 // parameter grids (cuRAND), 1 initial-condition grids (sinf), out[p*nx + k];
 // kind 2 the spectrum's, out[(p*nx + j)*nx + i] for component i of twin j
 cudaError_t launch_legacy_draws(int kind, long long n, int nx, double* out, cudaStream_t st);
-cudaError_t launch_lle_f32(const LleParams& L, double* out, cudaStream_t st);
+// state: scratch of lle_f32_state_bytes (0 for a map that runs in one launch);
+// without it every map runs in one launch. The same for the two below.
+size_t lle_f32_state_bytes(const LleParams& L);
+cudaError_t launch_lle_f32(const LleParams& L, double* out, cudaStream_t st, float* state = nullptr);
 // float-float base trajectory, FP32 twin difference (kern_ff.cu; RK4 systems)
-cudaError_t launch_lle_ff(const LleParams& L, double* out, cudaStream_t st);
+size_t lle_ff_state_bytes(const LleParams& L);
+cudaError_t launch_lle_ff(const LleParams& L, double* out, cudaStream_t st, float* state = nullptr);
 // Benettin blocks from caller-supplied states, rows of 2*SIZE_X + SIZE_A (orbit, parameters,
 // twin; kern_f64.cu / kern_ff.cu)
 cudaError_t launch_lle_states_f64(const LleParams& L, const double* states, double* out, cudaStream_t st);
@@ -125,7 +129,8 @@ int set_ff_pairs(int v);  // 1: two points per thread (default), 0: one
 int get_ff_pairs();
 // Lyapunov spectrum, out[p*SIZE_X + j] (FP64: every built-in system; FP32: the RK4 systems)
 cudaError_t launch_spectrum_f64(const LleParams& L, double* out, cudaStream_t st);
-cudaError_t launch_spectrum_f32(const LleParams& L, double* out, cudaStream_t st);
+size_t spectrum_f32_state_bytes(const LleParams& L);
+cudaError_t launch_spectrum_f32(const LleParams& L, double* out, cudaStream_t st, float* state = nullptr);
 // bifurcation points of a list (row k for list[k]); points whose kept-peak
 // count exceeds cap (kern_f64.cu / kern_f32.cu)
 cudaError_t launch_bif_list_f64(const SweepParams& P, const BifOut& O, const int* list, int count, cudaStream_t st);
