@@ -243,19 +243,23 @@ static int check_ff32_lle(const chaos_exec* ex, int system, const LleParams& L) 
 
 // precision / plug-in dispatch of the sweep kernels
 // The legacy per-point loop runs in FP64, the legacy library's arithmetic.
-static cudaError_t run_bif(int prec, const SweepParams& P, const BifOut& O, cudaStream_t st) {
+static cudaError_t run_bif(int prec, const SweepParams& P, const BifOut& O, Call& c) {
+    cudaStream_t st = c.stream;
     if (P.legacyLoop) prec = CHAOS_FP64;
     if (P.system == SYS_USER) return prec == CHAOS_FP32 ? cudaErrorNotSupported : launch_bif_user(P, O, st);
-    return prec == CHAOS_FP32 ? launch_bif_f32(P, O, st) : launch_bif_f64(P, O, st);
+    if (prec == CHAOS_FP32) return launch_bif_f32(P, O, st, (float4*)c.optional(transient_state_bytes(P, false)));
+    return launch_bif_f64(P, O, st);
 }
 static cudaError_t run_bif_list(int prec, const SweepParams& P, const BifOut& O, const int* list, int count,
                                 cudaStream_t st) {
     if (P.legacyLoop) prec = CHAOS_FP64;
     return prec == CHAOS_FP32 ? launch_bif_list_f32(P, O, list, count, st) : launch_bif_list_f64(P, O, list, count, st);
 }
-static cudaError_t run_basins(int prec, const SweepParams& P, const BasinsOut& O, cudaStream_t st) {
+static cudaError_t run_basins(int prec, const SweepParams& P, const BasinsOut& O, Call& c) {
+    cudaStream_t st = c.stream;
     if (P.system == SYS_USER) return prec == CHAOS_FP32 ? cudaErrorNotSupported : launch_basins_user(P, O, st);
-    return prec == CHAOS_FP32 ? launch_basins_f32(P, O, st) : launch_basins_f64(P, O, st);
+    if (prec == CHAOS_FP32) return launch_basins_f32(P, O, st, (float4*)c.optional(transient_state_bytes(P, true)));
+    return launch_basins_f64(P, O, st);
 }
 static cudaError_t run_lle(int prec, const LleParams& L, double* out, Call& c) {
     cudaStream_t st = c.stream;
@@ -538,7 +542,7 @@ static int bif1d_run(const chaos_exec* ex, SweepParams P, int gridMode, const do
     O.peaks = (double*)c.output(peaks, rowBytes);
     O.intervals = (double*)c.output(intervals, rowBytes);
     if (c.failed) return c.finish(CHAOS_E_NOMEM);
-    cudaError_t e = run_bif(c.ex.precision, P, O, c.stream);
+    cudaError_t e = run_bif(c.ex.precision, P, O, c);
     if (e != cudaSuccess) return c.finish(cuda_error(e, "bifurcation kernel"));
     rc = c.to_host(counts, O.counts, n * sizeof(int));
     if (!rc) rc = c.to_host(flags, O.flags, n * sizeof(int));
@@ -608,7 +612,7 @@ static int bif2d_run(const chaos_exec* ex, SweepParams P, int gridMode, const do
         Q.pBegin = b;
         Q.nPoints = std::min(chunk, n - b);
         BifOut O{dCounts + b, dFlags, nullptr, nullptr, dIv, cap};
-        cudaError_t e = run_bif(c.ex.precision, Q, O, c.stream);
+        cudaError_t e = run_bif(c.ex.precision, Q, O, c);
         if (e == cudaSuccess)
             e = launch_point_dbscan(dIv, dCounts + b, Q.nPoints, cap, eps, dLab, dSlot, dLabels + b, c.stream);
         if (e != cudaSuccess) return c.finish(cuda_error(e, "bifurcation 2-D kernels"));
@@ -972,7 +976,7 @@ int chaos_basins_features(const chaos_exec* ex, int system, double tMax, int nPt
     O.counts = (int*)c.output(counts, n * sizeof(int));
     O.last = nullptr;
     if (c.failed) return c.finish(CHAOS_E_NOMEM);
-    cudaError_t e = run_basins(c.ex.precision, P, O, c.stream);
+    cudaError_t e = run_basins(c.ex.precision, P, O, c);
     if (e != cudaSuccess) return c.finish(cuda_error(e, "basins kernel"));
     rc = c.to_host(flags, O.flags, n * sizeof(int));
     if (!rc) rc = c.to_host(avgPeaks, O.avgPeaks, n * sizeof(double));
@@ -1004,7 +1008,7 @@ int chaos_basins(const chaos_exec* ex, int system, double tMax, int nPts, double
     O.last = nullptr;
     int* dLabels = (int*)c.output(labels, n * sizeof(int));
     if (c.failed) return c.finish(CHAOS_E_NOMEM);
-    cudaError_t e = run_basins(c.ex.precision, P, O, c.stream);
+    cudaError_t e = run_basins(c.ex.precision, P, O, c);
     if (e != cudaSuccess) return c.finish(cuda_error(e, "basins kernel"));
     rc = dbscan_compat_device(c, O.avgPeaks, O.avgIntervals, O.flags, n, eps, dLabels);
     if (!rc) rc = c.to_host(labels, dLabels, n * sizeof(int));
@@ -1046,7 +1050,7 @@ int chaos_basins_dbscan(const chaos_exec* ex, int system, double tMax, int nPts,
     cudaError_t e = cudaMemsetAsync(O.mm, 0xff, 3 * kKeyReplicas * sizeof(unsigned long long), c.stream);
     if (e == cudaSuccess)
         e = cudaMemsetAsync(O.mm + 3 * kKeyReplicas, 0, 3 * kKeyReplicas * sizeof(unsigned long long), c.stream);
-    if (e == cudaSuccess) e = run_basins(c.ex.precision, P, O, c.stream);
+    if (e == cudaSuccess) e = run_basins(c.ex.precision, P, O, c);
     unsigned long long hm[6 * kKeyReplicas], keys[6];
     if (e == cudaSuccess) e = cudaMemcpyAsync(hm, O.mm, sizeof hm, cudaMemcpyDeviceToHost, c.stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);

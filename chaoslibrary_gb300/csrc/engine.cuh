@@ -406,9 +406,11 @@ __device__ __forceinline__ void bif_record(const SweepParams& P, const BifOut& O
 // Bifurcation point (reference kernels calculateTransTimeCUDA +
 // calculateDiscreteModelCUDA + peakFinderCUDA, bifurcationCUDA.cu:258-371),
 // fused. Writes flags/counts/first and the first `cap` kept peaks/intervals.
-template <int S, class T, int W>
+// Started: all steps of the transient but the last have been run
+// (transient_slices.cuh), with the state and flag in start[o].
+template <int S, class T, int W, bool Started = false>
 __device__ __forceinline__ void bif_point(const SweepParams& P, const BifOut& O, long long p, long long o,
-                                             Component<W> wc) {
+                                             Component<W> wc, const float4* start = nullptr) {
     constexpr int NX = Traits<S>::NX, NA = Traits<S>::NA;
     T x[NX], a[NA], xp[NX];
     load_point<S, T>(P, p, x, a);
@@ -426,6 +428,14 @@ __device__ __forceinline__ void bif_point(const SweepParams& P, const BifOut& O,
         // the state before the last step is kept for the fixed-point test:
         // the last step is peeled off the loop, so the others copy nothing
         int s = 0;
+        if constexpr (Started) {
+            const float4 v = start[o];
+            x[0] = v.x;
+            x[1] = v.y;
+            x[2] = v.z;
+            flag = v.w != 0.f ? 1 : 0;
+            s = nS - 1;
+        } else
         if constexpr (S != SYS_USER) {
             // blocks of kTransientBlock steps, one divergence branch a block:
             // a point's flags do not depend on the step at which it diverged
@@ -679,14 +689,21 @@ __device__ __forceinline__ void basins_record(const SweepParams& P, const Basins
     write_basins_point(O, o, flag, n > 1 ? n - 1 : 0, sums.peaks(), sums.intervals(P.hInterval), (double)lastT);
 }
 
-template <int S, class T, bool PRE1, int W>
+template <int S, class T, bool PRE1, int W, bool Started = false>
 __device__ __forceinline__ void basins_point(const SweepParams& P, const BasinsOut& O, long long p, long long o,
-                                             Component<W> wc) {
+                                             Component<W> wc, const float4* start = nullptr) {
     constexpr int NX = Traits<S>::NX, NA = Traits<S>::NA;
     T x[NX], a[NA];
     load_point<S, T>(P, p, x, a);
     const StepCtx<T> c((T)P.h);
-    for (int s = 0; s < P.S; ++s) step<S>(x, a, c);
+    if constexpr (Started) {  // the transient has been run (transient_slices.cuh)
+        const float4 v = start[o];
+        x[0] = v.x;
+        x[1] = v.y;
+        x[2] = v.z;
+    } else {
+        for (int s = 0; s < P.S; ++s) step<S>(x, a, c);
+    }
     basins_record<S, T, PRE1>(P, O, x, a, c, o, wc);
 }
 

@@ -8,6 +8,7 @@
 
 #include "engine.cuh"
 #include "lle_slices.h"
+#include "transient_slices.cuh"
 #include "sweep_launch.h"
 
 namespace chaos {
@@ -17,11 +18,11 @@ constexpr int kBlock = kSweepBlock;
 
 // The sweep kernels take Window<trajectories per thread>::bytes(block)
 // of dynamic shared memory.
-template <int S, int W>
-__global__ void __launch_bounds__(kMaxBlock) bif_kernel_f32(SweepParams P, BifOut O) {
+template <int S, int W, bool Started = false>
+__global__ void __launch_bounds__(kMaxBlock) bif_kernel_f32(SweepParams P, BifOut O, const float4* start) {
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= P.nPoints) return;
-    bif_point<S, float>(P, O, P.pBegin + o, o, Component<W>{P.wv});
+    bif_point<S, float, W, Started>(P, O, P.pBegin + o, o, Component<W>{P.wv}, start);
 }
 
 template <int S>
@@ -194,15 +195,28 @@ template <class F> void launch_bif_pairs(const SweepParams& P, const BifOut& O, 
     note_launch();
 }
 
-template <int S> void launch_bif_points(const SweepParams& P, const BifOut& O, int block, cudaStream_t st) {
-    with_component<KnownComponent<S, float>::value>(P.wv, [&](auto wc) {
-        bif_kernel_f32<S, decltype(wc)::kIndex>
-            <<<grid_of(P.nPoints, block), block, Window<1>::bytes(block), st>>>(P, O);
-    });
+template <int S, int W>
+void launch_bif_points_as(const SweepParams& P, const BifOut& O, int block, float4* state, cudaStream_t st) {
+    auto* k = bif_kernel_f32<S, W>;
+    if constexpr (KnownComponent<S, float>::value) {
+        const TransientPlan plan = state ? transient_plan(P, false) : TransientPlan{};
+        if (plan.jobs > 0) {
+            launch_transient<S, W, false>(plan, P, state, st);
+            k = bif_kernel_f32<S, W, true>;
+        }
+    }
+    k<<<grid_of(P.nPoints, block), block, Window<1>::bytes(block), st>>>(P, O, state);
     note_launch();
 }
+template <int S>
+void launch_bif_points(const SweepParams& P, const BifOut& O, int block, float4* state, cudaStream_t st) {
+    with_component<KnownComponent<S, float>::value>(
+        P.wv, [&](auto wc) { launch_bif_points_as<S, decltype(wc)::kIndex>(P, O, block, state, st); });
+}
 
-cudaError_t launch_bif_f32(const SweepParams& P, const BifOut& O, cudaStream_t st) {
+size_t transient_state_bytes(const SweepParams& P, bool basins) { return transient_plan(P, basins).bytes(); }
+
+cudaError_t launch_bif_f32(const SweepParams& P, const BifOut& O, cudaStream_t st, float4* state) {
     if (P.nPoints <= 0) return cudaSuccess;
     const Launch l = sweep_launch(P, false);
     if (l.form == 2) {
@@ -211,7 +225,7 @@ cudaError_t launch_bif_f32(const SweepParams& P, const BifOut& O, cudaStream_t s
         else launch_bif_pairs<Chen>(P, O, l.block, st);
         return cudaGetLastError();
     }
-#define CALL(S) launch_bif_points<S>(P, O, l.block, st)
+#define CALL(S) launch_bif_points<S>(P, O, l.block, state, st)
     CHAOS_SYSTEM_SWITCH(P.system, CALL)
 #undef CALL
     return cudaGetLastError();

@@ -106,9 +106,12 @@ struct LleParams {
 
 // precision-specific launchers (kern_f64.cu / kern_f32.cu)
 cudaError_t launch_bif_f64(const SweepParams& P, const BifOut& O, cudaStream_t st);
-cudaError_t launch_bif_f32(const SweepParams& P, const BifOut& O, cudaStream_t st);
+// state: scratch of transient_state_bytes (0 for a sweep whose transient is not
+// run in slices); without it none is.
+size_t transient_state_bytes(const SweepParams& P, bool basins);
+cudaError_t launch_bif_f32(const SweepParams& P, const BifOut& O, cudaStream_t st, float4* state = nullptr);
 cudaError_t launch_basins_f64(const SweepParams& P, const BasinsOut& O, cudaStream_t st);
-cudaError_t launch_basins_f32(const SweepParams& P, const BasinsOut& O, cudaStream_t st);
+cudaError_t launch_basins_f32(const SweepParams& P, const BasinsOut& O, cudaStream_t st, float4* state = nullptr);
 cudaError_t launch_lle_f64(const LleParams& L, double* out, cudaStream_t st);
 // the legacy LLE kernels' raw twin draws of points [0, n) (kern_f64.cu): kind 0
 // parameter grids (cuRAND), 1 initial-condition grids (sinf), out[p*nx + k];
