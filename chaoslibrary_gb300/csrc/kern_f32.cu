@@ -148,8 +148,9 @@ int set_sweep_pairs(int v) {
 // Launch shapes the self-timing tuner (tune.cu) found, per kind (0 1-D
 // bifurcation, 1 basins, 2 LLE map) and RK4 system: 0 = none (the built-in
 // rules below), else form * 1024 + block with form 1 (one point per thread)
-// or 2 (two points per thread in packed FP32x2 lanes); for the LLE map also form 12 / 16 (one point per thread, registers shaped for
-// 12 / 16 resident blocks per SM, block 128).
+// or 2 (two points per thread in packed FP32x2 lanes); for the LLE map also form
+// 12 / 16 (one point per thread, registers shaped for 12 / 16 resident blocks per
+// SM, block 128).
 std::atomic<int> g_shape[3][3];
 
 int shape_of(int kind, int system) {

@@ -70,6 +70,10 @@ template <class F, int G>
 __global__ void __launch_bounds__(kSweep) lle_team_kernel(LleParams L, double* out) {
     lle_teams<F, G>(L, out);
 }
+template <class F, int G>
+__global__ void __launch_bounds__(kSweep) spectrum_team_kernel(LleParams L, double* out) {
+    spectrum_teams<F, G>(L, out);
+}
 
 // The legacy library's LLE kernels' scheme (L.legacyLoop).
 template <int S>
@@ -420,6 +424,14 @@ bool team_sweep(long long n) {
 }
 bool team_lle(long long n) { return n <= sm_points(80); }
 bool split_lle(long long n) { return n <= sm_points(40); }
+// Spectra (the three twins and the Gram-Schmidt beside the orbit), 500 steps,
+// point per thread / four trajectories a team / a team each, Lorenz: up to 10
+// points per SM 2.99 / 1.62 / 0.58 to 0.64 ms, 16 2.99 / 1.62 / 0.89, 26 2.99 /
+// 1.62 / 1.46, 32 2.99 / 1.69 / 1.74, 60 2.99 / 1.99, 80 2.99 / 2.54, 90 2.99 /
+// 3.00; Rossler 26 2.55 / 1.59 / 1.51, 70 2.55 / 2.32, 80 2.55 / 2.63; Chen 80
+// 3.21 / 3.03, 90 3.22 / 3.56.
+bool team_spectrum(long long n) { return n <= sm_points(76); }
+bool split_spectrum(long long n) { return n <= sm_points(28); }
 inline unsigned team_blocks(long long n, int perWarp) { return (unsigned)((n + perWarp - 1) / perWarp); }
 
 #define CHAOS_RK4_SWITCH(sys, CALL)                  \
@@ -506,6 +518,16 @@ cudaError_t launch_lle_states_f64(const LleParams& L, const double* states, doub
 
 cudaError_t launch_spectrum_f64(const LleParams& L, double* out, cudaStream_t st) {
     if (L.nPoints <= 0) return cudaSuccess;
+    if (!L.legacyLoop && L.system <= SYS_CHEN_RK4 && team_spectrum(L.nPoints)) {
+        const bool split = split_spectrum(L.nPoints);
+#define CALL(F)                                                                                         \
+    (split ? spectrum_team_kernel<F, 4><<<team_blocks(L.nPoints, 2), kSweep, 0, st>>>(L, out)           \
+           : spectrum_team_kernel<F, 1><<<team_blocks(L.nPoints, TeamLane::kTeams), kSweep, 0, st>>>(L, out))
+        CHAOS_RK4_SWITCH(L.system, CALL)
+#undef CALL
+        note_launch();
+        return cudaGetLastError();
+    }
 #define CALL(S)                                                                    \
     {                                                                              \
         if (L.legacyLoop) spectrum_legacy_kernel<S><<<warps_for(L.nPoints), kSweep, 0, st>>>(L, out); \

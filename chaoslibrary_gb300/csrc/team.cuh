@@ -358,4 +358,84 @@ __device__ __forceinline__ void lle_teams(const LleParams& L, double* out) {
     if (writes) out[o] = sum / L.tMax;
 }
 
+// Spectrum points (spectrum_point_full): the orbit and its three twins, all in
+// the lanes of one team (G = 1, ten points a warp) or in a team each (G = 4, two
+// points a warp, teams 8 and 9 idle along). Between blocks every lane holds its
+// component of all four, the dot products are sums over the team's lanes in
+// component order, and with G = 4 a team takes its own twin's norm and logarithm.
+template <class F, int G>
+__device__ __forceinline__ void spectrum_teams(const LleParams& L, double* out) {
+    constexpr int kPoints = G == 1 ? TeamLane::kTeams : 2, M = 4 / G;
+    const TeamLane l;
+    const int point = G == 1 ? l.team : min(l.team / 4, 1);
+    const int traj = G == 1 ? 0 : l.team % 4;  // of this lane: 0 the orbit
+    long long o = (long long)blockIdx.x * kPoints + point;
+    const bool writes = !l.spare() && l.role == 0 && o < L.nPoints && (G == 1 || (traj > 0 && l.team < 8));
+    if (o >= L.nPoints) o = L.nPoints - 1;
+    double xs[3], as[3];
+    lle_load<3, 3>(L, L.pBegin + o, xs, as);
+    const TeamField<F> f(as, l.role);
+    const RK4H<double> c(L.h);
+    double v[M], sum[3] = {0.0, 0.0, 0.0};  // (G = 4: its own twin's in sum[0])
+    v[0] = of_role(xs, l.role);
+#pragma unroll 4
+    for (int s = 0; s < L.trans; ++s) team_step<1>(v, f, c, l);
+    if (G == 1) {
+#pragma unroll
+        for (int j = 1; j < M; ++j) v[j] = l.role == j - 1 ? v[0] + L.eps : v[0];
+    } else if (l.role == traj - 1) {
+        v[0] = v[0] + L.eps;
+    }
+    // sum of the team's products in component order from 0.0: a sum of -0 is +0
+    auto dot = [&](double a, double b) {
+        const double q = a * b, t = (l.from(q, l.base) + l.from(q, l.base + 1)) + l.from(q, l.base + 2);
+        return __double2hiint(t) == (int)0x80000000 && __double2loint(t) == 0 ? 0.0 : t;
+    };
+    for (int b = 0; b <= L.calcBlocks; ++b) {
+#pragma unroll 2
+        for (int s = 0; s < L.ntp; ++s) team_step<M>(v, f, c, l);
+        double x = v[0], d[3], g[3];
+        if (G == 1) {
+#pragma unroll
+            for (int j = 0; j < 3; ++j) d[j] = v[(j + 1) % M] - x;
+        } else {
+            x = l.from(v[0], 12 * point + l.role);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) d[j] = l.from(v[0], 12 * point + 3 * (j + 1) + l.role) - x;
+        }
+        double den[2];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            g[j] = d[j];
+#pragma unroll
+            for (int m = 0; m < j; ++m) {
+                const double num = dot(d[j], g[m]);
+                const double frac = den[m] == 0.0 ? 0.0 : num / den[m];
+                g[j] = g[j] - frac * g[m];
+            }
+            if (j < 2) den[j] = l.sum_squares(g[j]);
+        }
+        auto renorm = [&](double gj, double& s) {
+            const double nrm = sqrt(l.sum_squares(gj));
+            s = s + log(nrm / L.eps);
+            return x + (nrm == 0.0 ? 0.0 : gj / nrm) * L.eps;
+        };
+        if (G == 1) {
+#pragma unroll
+            for (int j = 0; j < 3; ++j) v[(j + 1) % M] = renorm(g[j], sum[j]);
+        } else {
+            const double y = renorm(of_role(g, max(traj - 1, 0)), sum[0]);
+            if (traj > 0) v[0] = y;
+        }
+    }
+    if (!writes) return;
+    double* row = out + (L.pBegin + o) * 3;
+    if (G == 1) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) row[j] = sum[j] / L.tMax;
+    } else {
+        row[traj - 1] = sum[0] / L.tMax;
+    }
+}
+
 }  // namespace chaos
