@@ -150,11 +150,14 @@ void* Call::optional(size_t bytes) {
     if (bytes == 0 || bytes > scratch_budget_bytes()) return nullptr;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     void* p = nullptr;
-    if (cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone &&
-        cudaMallocFromPoolAsync(&p, bytes, pool, stream) == cudaSuccess)
-        owned.push_back(p);
-    else
-        cudaGetLastError();
+    cudaError_t e = cudaStreamIsCapturing(stream, &capture);
+    if (e == cudaSuccess && capture != cudaStreamCaptureStatusNone) return nullptr;
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // the call goes on without
+        return nullptr;
+    }
+    owned.push_back(p);
     return p;
 }
 

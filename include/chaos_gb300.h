@@ -200,7 +200,9 @@ int chaos_compact_peaks(const chaos_exec* ex, const int* counts, const double* p
  * random unit direction with cuRAND). writableVar and maxValue are accepted
  * and unused, as in the reference. CHAOS_FP32 is supported for the three RK4
  * systems and Chameleon (the twin carried as an exact difference, FP64 log
- * sum).
+ * sum). FP32 and float-float maps that fill the GPU unevenly run as several
+ * launches with up to some 20 MB of device scratch; while the stream is being
+ * captured, or without the memory, as one, with the same results.
  */
 int chaos_lle2d(const chaos_exec* ex, int system, double tMax, double NT, int nPts, double h, double eps,
                 const double* initialConditions, int amountOfInitialConditions, const double* ranges,
