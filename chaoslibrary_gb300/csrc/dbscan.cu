@@ -996,37 +996,36 @@ __global__ void __launch_bounds__(256) long_scan_kernel(Sorted Q, Cells K, ScanQ
         const bool allCore = K.dense[c] != 0;
         int found = 0;
         constexpr int kStep = 4;  // points in flight per thread
-        for (int q = q0 + threadIdx.x; q - (int)threadIdx.x < q1; q += kStep * blockDim.x) {
+        const int len = q1 - q0;  // (offsets from q0: a position past the part may not be an int)
+        for (int q = threadIdx.x; q - (int)threadIdx.x < len; q += kStep * blockDim.x) {
             // (the break is uniform over the warp: its lanes read the same word)
             if (labels ? __ldcg(best + p) <= key : __ldcg(acc + p) >= minPts) break;
             float d2[kStep];
 #pragma unroll
             for (int k = 0; k < kStep; ++k) {
                 const int i = q + k * blockDim.x;
-                d2[k] = __int_as_float(0x7f800000);
-                if (i < q1) {
-                    float sum = 0.f;
+                d2[k] = 0.f;
+                if (i < len && range) {
 #pragma unroll
                     for (int d = 0; d < 3; ++d) {
                         if (d >= K.D) continue;
-                        const float df = o[d] - Q.r[d][i];
-                        sum = fmaf(df, df, sum);
+                        const float df = o[d] - Q.r[d][q0 + i];
+                        d2[k] = fmaf(df, df, d2[k]);
                     }
-                    d2[k] = range ? sum : __int_as_float(0x7fc00000);
                 }
             }
             int hits = 0;
 #pragma unroll
             for (int k = 0; k < kStep; ++k) {
-                if (d2[k] > eps2 * kFloatOut) continue;
                 const int i = q + k * blockDim.x;
-                bool in = d2[k] < eps2 * kFloatIn;
+                if (i >= len || (range && d2[k] > eps2 * kFloatOut)) continue;
+                bool in = range && d2[k] < eps2 * kFloatIn;
                 if (!in) {
                     double v[3];
-                    Q.load(i, v);
+                    Q.load(q0 + i, v);
                     in = within_eps(dist2(me, v, K.D), eps);
                 }
-                if (in && labels && !allCore) in = Q.core[i] == 1;
+                if (in && labels && !allCore) in = Q.core[q0 + i] == 1;
                 hits += in ? 1 : 0;
             }
             found = (int)__reduce_add_sync(0xffffffffu, (unsigned)hits);
