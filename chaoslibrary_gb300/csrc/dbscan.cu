@@ -974,7 +974,7 @@ struct ScanQueue {
 __global__ void __launch_bounds__(256) long_scan_kernel(Sorted Q, Cells K, ScanQueue W, double eps, int minPts,
                                                         int labels, int* acc, unsigned long long* best, int* parent,
                                                         const int* compMin) {
-    const int tasks = min(*W.count, W.cap);
+    const int tasks = min(*W.count, W.cap), lane = threadIdx.x & 31;
     const float eps2 = (float)(eps * eps);
     const bool range = eps2 > 1e-30f && eps2 < 1e30f;  // else every distance is taken in FP64
     for (long long w = blockIdx.x; w < (long long)tasks * kScanSplit; w += gridDim.x) {
@@ -998,8 +998,10 @@ __global__ void __launch_bounds__(256) long_scan_kernel(Sorted Q, Cells K, ScanQ
         constexpr int kStep = 4;  // points in flight per thread
         const int len = q1 - q0;  // (offsets from q0: a position past the part may not be an int)
         for (int q = threadIdx.x; q - (int)threadIdx.x < len; q += kStep * blockDim.x) {
-            // (the break is uniform over the warp: its lanes read the same word)
-            if (labels ? __ldcg(best + p) <= key : __ldcg(acc + p) >= minPts) break;
+            // other warps change the word: one lane reads it for its warp
+            bool done = false;
+            if (lane == 0) done = labels ? __ldcg(best + p) <= key : __ldcg(acc + p) >= minPts;
+            if (__shfl_sync(0xffffffffu, done, 0)) break;
             float d2[kStep];
 #pragma unroll
             for (int k = 0; k < kStep; ++k) {
@@ -1030,7 +1032,7 @@ __global__ void __launch_bounds__(256) long_scan_kernel(Sorted Q, Cells K, ScanQ
             }
             found = (int)__reduce_add_sync(0xffffffffu, (unsigned)hits);
             if (found == 0) continue;
-            if ((threadIdx.x & 31) == 0) {
+            if (lane == 0) {
                 if (labels) atomicMin(best + p, key);
                 else atomicAdd(acc + p, found);
             }
@@ -1333,7 +1335,11 @@ __device__ __forceinline__ void cross_cells(Sorted Q, Cells K, const int* nbOwne
         if (lane == 0) deferred[w] = 1;
         return;
     }
-    if (safe && uf_find(parent, ca) == uf_find(parent, cb)) return;
+    if (safe) {  // other warps unite cells meanwhile: one lane looks for its warp
+        bool joined = false;
+        if (lane == 0) joined = uf_find(parent, ca) == uf_find(parent, cb);
+        if (__shfl_sync(0xffffffffu, joined, 0)) return;
+    }
     const double eps2 = eps * eps;
     double gap2, span2;
     pair_boxes(K, ca, cb, gap2, span2);
