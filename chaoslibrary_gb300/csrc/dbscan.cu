@@ -1446,12 +1446,13 @@ __global__ void __launch_bounds__(256) long_pairs_kernel(Sorted Q, Cells K, cons
         const double* lo = K.lo + 3 * (long long)cb;
         const bool coreA = K.dense[ca] != 0, coreB = K.dense[cb] != 0;
         const int endA = Q.se[ca], endB = Q.se[cb];
-        for (int q0 = Q.sb[cb] + (int)(blockIdx.x % team) * 256; q0 < endB; q0 += team * 256) {
+        // (64 bits: a block past the last one may not have an int for its start)
+        for (long long q0 = Q.sb[cb] + (long long)(blockIdx.x % team) * 256; q0 < endB; q0 += team * 256) {
             __syncthreads();
             if (threadIdx.x == 0) apart = uf_find(parent, ca) != uf_find(parent, cb);
             __syncthreads();
             if (!apart) break;
-            const int q = q0 + threadIdx.x;
+            const long long q = q0 + threadIdx.x;
             const bool mine = q < endB && (coreB || Q.core[q] == 1);
             float r[3] = {0.f, 0.f, 0.f};
             if (mine) {
@@ -1460,8 +1461,8 @@ __global__ void __launch_bounds__(256) long_pairs_kernel(Sorted Q, Cells K, cons
                     if (d < K.D) r[d] = Q.r[d][q];
             }
             bool hit = false;
-            for (int p0 = Q.sb[ca]; p0 < endA; p0 += 256) {
-                const int p = p0 + threadIdx.x;
+            for (long long p0 = Q.sb[ca]; p0 < endA; p0 += 256) {
+                const long long p = p0 + threadIdx.x;
                 __syncthreads();
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
@@ -1470,7 +1471,7 @@ __global__ void __launch_bounds__(256) long_pairs_kernel(Sorted Q, Cells K, cons
                                                                               : __int_as_float(0x7f800000);
                 }
                 __syncthreads();
-                const int m = min(256, endA - p0);
+                const int m = (int)min(256LL, endA - p0);
                 for (int k = 0; k < m && mine && !hit; ++k) {
                     float sum = 0.f;
 #pragma unroll
@@ -1485,8 +1486,8 @@ __global__ void __launch_bounds__(256) long_pairs_kernel(Sorted Q, Cells K, cons
                         continue;
                     }
                     double a[3] = {0, 0, 0}, b[3] = {0, 0, 0};
-                    Q.load(p0 + k, a);
-                    Q.load(q, b);
+                    Q.load((int)p0 + k, a);
+                    Q.load((int)q, b);
                     hit = (coreA || Q.core[p0 + k] == 1) && within_eps(dist2(a, b, K.D), eps);
                 }
                 if (__syncthreads_or(hit)) break;
