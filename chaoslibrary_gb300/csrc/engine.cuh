@@ -1452,14 +1452,14 @@ __device__ __forceinline__ void record_pair_windows(int B, P2* x, P2* xp, Compon
         if (rec[0] && dv0) {
             rec[0] = false;
             flag[0] = 0;
-            open &= ~1u;
         }
         if (rec[1] && dv1) {
             rec[1] = false;
             flag[1] = 0;
-            open &= ~2u;
         }
         if (!rec[0] && !rec[1]) return;
+        // a lane that diverged on a plateau leaves it there: nothing of it is judged any more
+        open &= (rec[0] ? 1u : 0u) | (rec[1] ? 2u : 0u);
         up0 = mask0 & 1u;
         up1 = mask1 & 1u;
         w.put(-2, make_float2(w.at(0, K - 2), w.at(1, K - 2)));
