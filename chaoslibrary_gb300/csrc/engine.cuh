@@ -274,9 +274,15 @@ template <int L> struct Window {
 // a sample) sent nearly every block of a chaotic sweep through the
 // transitions sample by sample, since one of 32 orbits always had a peak in
 // it. Measured against that, 20,000 steps: 1,000 Lorenz points (then with the
-// detector as selects) 1.83 -> 0.88 ms, 700,001 Rossler points 19.9 -> 18.1 ms;
-// 1024^2 Lorenz basins 37.4 -> 33.9 ms.
-template <int NX, int W, class Advance, class Diverged, class OnPeak>
+// detector as selects) 1.83 -> 0.88 ms, 700,001 Rossler points 19.9 -> 18.1 ms.
+//
+// Stop: a window ends after the four samples among which the orbit diverged. In
+// maps with many such points the rest of the window is time lost (basins of 40
+// time units, 5 steps a sample: rossler_cd 400^2 0.370 -> 0.303 ms, memristor
+// 900^2 12.9 -> 11.7); the basins of the RK4 systems and of Chameleon with one
+// step a sample go without, where the test costs up to 5 % (Rossler 400^2 0.757
+// -> 0.799 ms) and a window at most some 2 us.
+template <int NX, bool Stop, int W, class Advance, class Diverged, class OnPeak>
 __device__ __forceinline__ int record_windows(int B, float* x, float* xp, Component<W> wc, const Window<1>& w, float& last,
                                               int& n, Advance&& advance, Diverged&& diverged, OnPeak&& on_peak) {
     constexpr int K = Window<1>::K;
@@ -291,8 +297,9 @@ __device__ __forceinline__ int record_windows(int B, float* x, float* xp, Compon
     bool dv = false;
     for (; i + K < B; i += K) {
         unsigned mask = 0;
+        int q = 0;
 #pragma unroll 1
-        for (int q = 0; q < K; q += 4) {
+        for (; q < K && !(Stop && dv); q += 4) {
             mask <<= 4;
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
@@ -306,8 +313,8 @@ __device__ __forceinline__ int record_windows(int B, float* x, float* xp, Compon
         }
         int m = K;
         if (__builtin_expect(dv, 0)) {  // the samples up to the one before the divergent one count
-            for (m = 1; m < K && !diverged(w.at(0, m));) ++m;
-            mask >>= K - m;
+            for (m = 1; m < q && !diverged(w.at(0, m));) ++m;
+            mask >>= q - m;
             p = w.at(0, m - 1);
         }
         const unsigned cand = PeakWindow::candidates(mask, up, m);
@@ -371,7 +378,7 @@ __device__ __forceinline__ void bif_record(const SweepParams& P, const BifOut& O
     for (int j = 0; j < NX; ++j) xp[j] = x[j];
     if constexpr (std::is_same<T, float>::value) {
         float last;
-        flag = record_windows<NX>(
+        flag = record_windows<NX, KnownComponent<S, T>::value>(
             nB, x, xp, wc, Window<1>(), last, n, [&] { step<S>(x, a, c); },
             [&](float v) { return bif_diverged(v, P); },
             [&](int, const PeakWindow& d, float val, int t) { write_peak(d.n, d.tprev, val, t); });
@@ -658,7 +665,7 @@ __device__ __forceinline__ void basins_record(const SweepParams& P, const Basins
     if constexpr (std::is_same<T, float>::value) {  // as bif_record; the sums in shared memory
         const Window<1> w;
         sums.store(w.sum);
-        flag = record_windows<NX>(
+        flag = record_windows<NX, !(KnownComponent<S, T>::value && PRE1)>(
             P.B, x, xp, wc, w, lastT, n, advance, [&](float v) { return basins_diverged(v, P); },
             [&](int, const PeakWindow& d, float val, int t) {
                 if (d.n >= 1) PeakSums<float>::add_stored(w.sum, val, t - d.tprev);
@@ -1398,7 +1405,13 @@ __device__ __forceinline__ void bif_pair_transient(const SweepParams& P, P2* x, 
 // record_windows: rec[l] says whether lane l records, flag[l] becomes 0 when
 // it diverges (the pair goes on while the other lane records), xp the state
 // before the last advance (of a lane that did not diverge).
-template <int W, class Advance, class Diverged, class OnPeak>
+// Tested: the first four samples are tested one by one. A basins transient has
+// no test, and where it left both orbits of a pair beyond the bound a window
+// run past the first sample would be most of the pair's time: 700^2 Lorenz
+// points, all of them beyond, 5 steps a sample, 0.116 -> 0.042 ms. (A test after
+// every four samples of a window costs the other maps 2 %; the bifurcation's
+// pairs, whose transient has a test, lose up to 5 % to this form.)
+template <bool Tested, int W, class Advance, class Diverged, class OnPeak>
 __device__ __forceinline__ void record_pair_windows(int B, P2* x, P2* xp, Component<W> wc, const Window<2>& w, bool* rec,
                                                     int* flag, float* last, Advance&& advance, Diverged&& diverged,
                                                     OnPeak&& on_peak) {
@@ -1412,84 +1425,103 @@ __device__ __forceinline__ void record_pair_windows(int B, P2* x, P2* xp, Compon
     P2 v = wc.template of<3>(x), p(0.0);
     unsigned up0 = 0, up1 = 0, open = 0;
     int i = 0;
-    for (; i + K < B; i += K) {
-        unsigned mask0 = 0, mask1 = 0;
-        bool dv0 = false, dv1 = false;
-#pragma unroll 1
-        for (int q = 0; q < K; q += 4) {
-            mask0 <<= 4;
-            mask1 <<= 4;
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                if (v.v.x > p.v.x) mask0 |= 8u >> r;
-                if (v.v.y > p.v.y) mask1 |= 8u >> r;
-                p = v;
-                w.put(q + r, v.v);
-                advance();
-                v = wc.template of<3>(x);
-                dv0 |= diverged(v.v.x);
-                dv1 |= diverged(v.v.y);
-            }
-        }
-        int m0 = K, m1 = K;
-        if (__builtin_expect(rec[0] && dv0, 0)) {
-            for (m0 = 1; m0 < K && !diverged(w.at(0, m0));) ++m0;
-            mask0 >>= K - m0;
-        }
-        if (__builtin_expect(rec[1] && dv1, 0)) {
-            for (m1 = 1; m1 < K && !diverged(w.at(1, m1));) ++m1;
-            mask1 >>= K - m1;
-        }
-        const unsigned c0 = rec[0] ? PeakWindow::candidates(mask0, up0, m0) : 0u;
-        const unsigned c1 = rec[1] ? PeakWindow::candidates(mask1, up1, m1) : 0u;
-        unsigned moved = 0;
-        if (open != 0u)
-            moved = open & ((mask0 != 0u || w.at(0, m0 - 1) != w.at(0, -1) ? 1u : 0u) |
-                            (mask1 != 0u || w.at(1, m1 - 1) != w.at(1, -1) ? 2u : 0u));
-        if ((c0 | c1 | moved) != 0u) w.judge(i, c0, c1, m0, m1, moved, open, on_peak);
-        if (rec[0]) last[0] = w.at(0, m0 - 1);
-        if (rec[1]) last[1] = w.at(1, m1 - 1);
-        if (rec[0] && dv0) {
-            rec[0] = false;
-            flag[0] = 0;
-        }
-        if (rec[1] && dv1) {
-            rec[1] = false;
-            flag[1] = 0;
-        }
-        if (!rec[0] && !rec[1]) return;
+    auto carry = [&](unsigned mask0, unsigned mask1, int n) {
         // a lane that diverged on a plateau leaves it there: nothing of it is judged any more
         open &= (rec[0] ? 1u : 0u) | (rec[1] ? 2u : 0u);
         up0 = mask0 & 1u;
         up1 = mask1 & 1u;
-        w.put(-2, make_float2(w.at(0, K - 2), w.at(1, K - 2)));
+        w.put(-2, make_float2(w.at(0, n - 2), w.at(1, n - 2)));
         w.put(-1, p.v);
-    }
-    unsigned mask0 = 0, mask1 = 0;
-    int m0 = 0, m1 = 0, m = 0;  // samples each lane judges, and those of the tail
-    for (; i + m < B && (rec[0] || rec[1]);) {
+    };
+    // full windows, their steps without a test; whether a lane still records
+    auto windows = [&]() -> bool {
+        for (; i + K < B; i += K) {
+            unsigned mask0 = 0, mask1 = 0;
+            bool dv0 = false, dv1 = false;
+#pragma unroll 1
+            for (int q = 0; q < K; q += 4) {
+                mask0 <<= 4;
+                mask1 <<= 4;
 #pragma unroll
-        for (int j = 0; j < 3; ++j) xp[j] = x[j];
-        if (rec[0]) {
-            mask0 = (mask0 << 1) | (v.v.x > p.v.x ? 1u : 0u);
-            ++m0;
-            last[0] = v.v.x;
+                for (int r = 0; r < 4; ++r) {
+                    if (v.v.x > p.v.x) mask0 |= 8u >> r;
+                    if (v.v.y > p.v.y) mask1 |= 8u >> r;
+                    p = v;
+                    w.put(q + r, v.v);
+                    advance();
+                    v = wc.template of<3>(x);
+                    dv0 |= diverged(v.v.x);
+                    dv1 |= diverged(v.v.y);
+                }
+            }
+            int m0 = K, m1 = K;
+            if (__builtin_expect(rec[0] && dv0, 0)) {
+                for (m0 = 1; m0 < K && !diverged(w.at(0, m0));) ++m0;
+                mask0 >>= K - m0;
+            }
+            if (__builtin_expect(rec[1] && dv1, 0)) {
+                for (m1 = 1; m1 < K && !diverged(w.at(1, m1));) ++m1;
+                mask1 >>= K - m1;
+            }
+            const unsigned c0 = rec[0] ? PeakWindow::candidates(mask0, up0, m0) : 0u;
+            const unsigned c1 = rec[1] ? PeakWindow::candidates(mask1, up1, m1) : 0u;
+            unsigned moved = 0;
+            if (open != 0u)
+                moved = open & ((mask0 != 0u || w.at(0, m0 - 1) != w.at(0, -1) ? 1u : 0u) |
+                                (mask1 != 0u || w.at(1, m1 - 1) != w.at(1, -1) ? 2u : 0u));
+            if ((c0 | c1 | moved) != 0u) w.judge(i, c0, c1, m0, m1, moved, open, on_peak);
+            if (rec[0]) last[0] = w.at(0, m0 - 1);
+            if (rec[1]) last[1] = w.at(1, m1 - 1);
+            if (rec[0] && dv0) {
+                rec[0] = false;
+                flag[0] = 0;
+            }
+            if (rec[1] && dv1) {
+                rec[1] = false;
+                flag[1] = 0;
+            }
+            if (!rec[0] && !rec[1]) return false;
+            carry(mask0, mask1, K);
         }
-        if (rec[1]) {
-            mask1 = (mask1 << 1) | (v.v.y > p.v.y ? 1u : 0u);
-            ++m1;
-            last[1] = v.v.y;
+        return true;
+    };
+    // a window of at most `most` samples, a test after each; whether samples and a lane that records are left
+    auto tested = [&](int most) -> bool {
+        unsigned mask0 = 0, mask1 = 0;
+        int m0 = 0, m1 = 0, m = 0;  // samples each lane judges, and those of the window
+        for (; m < most && i + m < B && (rec[0] || rec[1]);) {
+#pragma unroll
+            for (int j = 0; j < 3; ++j) xp[j] = x[j];
+            if (rec[0]) {
+                mask0 = (mask0 << 1) | (v.v.x > p.v.x ? 1u : 0u);
+                ++m0;
+                last[0] = v.v.x;
+            }
+            if (rec[1]) {
+                mask1 = (mask1 << 1) | (v.v.y > p.v.y ? 1u : 0u);
+                ++m1;
+                last[1] = v.v.y;
+            }
+            p = v;
+            w.put(m++, v.v);
+            advance();
+            v = wc.template of<3>(x);
+            if (rec[0] && diverged(v.v.x)) { rec[0] = false; flag[0] = 0; }
+            if (rec[1] && diverged(v.v.y)) { rec[1] = false; flag[1] = 0; }
         }
-        p = v;
-        w.put(m++, v.v);
-        advance();
-        v = wc.template of<3>(x);
-        if (rec[0] && diverged(v.v.x)) { rec[0] = false; flag[0] = 0; }
-        if (rec[1] && diverged(v.v.y)) { rec[1] = false; flag[1] = 0; }
+        const unsigned c0 = m0 > 0 ? PeakWindow::candidates(mask0, up0, m0) : 0u;
+        const unsigned c1 = m1 > 0 ? PeakWindow::candidates(mask1, up1, m1) : 0u;
+        if ((c0 | c1 | open) != 0u) w.judge(i, c0, c1, m0, m1, open, open, on_peak);
+        i += m;
+        if (i >= B || (!rec[0] && !rec[1])) return false;
+        carry(mask0, mask1, m);
+        return true;
+    };
+    if constexpr (Tested) {
+        for (int most = 4; tested(most) && windows(); most = K) {}
+    } else if (windows()) {
+        tested(K);
     }
-    const unsigned c0 = m0 > 0 ? PeakWindow::candidates(mask0, up0, m0) : 0u;
-    const unsigned c1 = m1 > 0 ? PeakWindow::candidates(mask1, up1, m1) : 0u;
-    if ((c0 | c1 | open) != 0u) w.judge(i, c0, c1, m0, m1, open, open, on_peak);
 }
 
 template <class F, int W>
@@ -1517,7 +1549,7 @@ __device__ __forceinline__ void bif_pair_point(const SweepParams& P, const BifOu
         }
         const Window<2> w;
         float last[2];
-        record_pair_windows(P.B, x, xp, wc, w, rec, flag, last, [&] { rk4_step<F>(x, a, c); },
+        record_pair_windows<false>(P.B, x, xp, wc, w, rec, flag, last, [&] { rk4_step<F>(x, a, c); },
                             [&](float v) { return bif_diverged(v, P); },
                             [&](int l, const PeakWindow& d, float val, int t) {
                                 const int q = d.n - 1;
@@ -1559,7 +1591,7 @@ __device__ __forceinline__ void basins_pair_point(const SweepParams& P, const Ba
     const Window<2> w;
     sums[0].store(w.sum);
     sums[1].store(w.sum + blockDim.x);
-    record_pair_windows(
+    record_pair_windows<true>(
         P.B, x, xp, wc, w, rec, flag, lastF,
         [&] {
             if (PRE1) rk4_step<F>(x, a, c);
