@@ -178,6 +178,20 @@ template <int NX, class T> __device__ __forceinline__ bool basins_fixed(const T*
 // Steps per block of the bifurcation transients' block form.
 constexpr int kTransientBlock = 8;
 
+// Steps laid out one after the other in the FP32 loops: transient steps before a
+// test, and samples of a window in a row. sin3 and the memristor have long steps
+// with branches of their own (the slow ranges of the sines and exponentials), and
+// copies of them fetch and wait: sin3, 40 time units, 1,000 points 2.4 -> 1.7 ms,
+// 400,000 14.7 -> 12.4; its basins 30^2 0.97 -> 0.86; memristor 1,000 points 2.79 ->
+// 2.76 ms, 400,000 21.0 -> 18.4 (one sample in a row 2.98 and 17.7: left at four).
+// sin2 basins of 400^2 points, several steps a sample, 1.14 -> 1.12 ms with two in
+// a row, but 1.08 -> 1.13 with one step a sample.
+template <int S> struct Straight {
+    static constexpr int kTransient = S == SYS_SIN3 || S == SYS_MEMRISTOR ? 1 : kTransientBlock;
+    static constexpr int kSamples = S == SYS_SIN3 ? 1 : 4;  // of one step each
+    static constexpr int kLongSamples = S == SYS_SIN2 ? 2 : kSamples;
+};
+
 // The FP32 recorded loops judge their samples in windows (PeakWindow,
 // peaks.h). A thread runs L trajectories (1, or 2 in packed lanes); what it
 // needs once a window lives in shared memory, so that the step loop keeps its
@@ -281,8 +295,8 @@ template <int L> struct Window {
 // time units, 5 steps a sample: rossler_cd 400^2 0.370 -> 0.303 ms, memristor
 // 900^2 12.9 -> 11.7); the basins of the RK4 systems and of Chameleon with one
 // step a sample go without, where the test costs up to 5 % (Rossler 400^2 0.757
-// -> 0.799 ms) and a window at most some 2 us.
-template <int NX, bool Stop, int W, class Advance, class Diverged, class OnPeak>
+// -> 0.799 ms) and a window at most some 2 us. Samples: of a window in a row.
+template <int NX, bool Stop, int Samples, int W, class Advance, class Diverged, class OnPeak>
 __device__ __forceinline__ int record_windows(int B, float* x, float* xp, Component<W> wc, const Window<1>& w, float& last,
                                               int& n, Advance&& advance, Diverged&& diverged, OnPeak&& on_peak) {
     constexpr int K = Window<1>::K;
@@ -301,7 +315,7 @@ __device__ __forceinline__ int record_windows(int B, float* x, float* xp, Compon
 #pragma unroll 1
         for (; q < K && !(Stop && dv); q += 4) {
             mask <<= 4;
-#pragma unroll
+#pragma unroll (Samples)
             for (int r = 0; r < 4; ++r) {
                 if (v > p) mask |= 8u >> r;
                 p = v;
@@ -378,7 +392,7 @@ __device__ __forceinline__ void bif_record(const SweepParams& P, const BifOut& O
     for (int j = 0; j < NX; ++j) xp[j] = x[j];
     if constexpr (std::is_same<T, float>::value) {
         float last;
-        flag = record_windows<NX, KnownComponent<S, T>::value>(
+        flag = record_windows<NX, KnownComponent<S, T>::value, Straight<S>::kSamples>(
             nB, x, xp, wc, Window<1>(), last, n, [&] { step<S>(x, a, c); },
             [&](float v) { return bif_diverged(v, P); },
             [&](int, const PeakWindow& d, float val, int t) { write_peak(d.n, d.tprev, val, t); });
@@ -449,7 +463,7 @@ __device__ __forceinline__ void bif_point(const SweepParams& P, const BifOut& O,
             // (the steps after it on an unbounded state report nothing).
             // Lorenz in FP32, one warp per scheduler: 69 cycles a step
             // against 91 with a branch after every step.
-            constexpr int K = kTransientBlock;
+            constexpr int K = std::is_same<T, float>::value ? Straight<S>::kTransient : kTransientBlock;
             for (; s + K <= nS - 1; s += K) {
                 bool dv = false;
 #pragma unroll
@@ -665,7 +679,9 @@ __device__ __forceinline__ void basins_record(const SweepParams& P, const Basins
     if constexpr (std::is_same<T, float>::value) {  // as bif_record; the sums in shared memory
         const Window<1> w;
         sums.store(w.sum);
-        flag = record_windows<NX, !(KnownComponent<S, T>::value && PRE1)>(
+        constexpr bool stop = !(KnownComponent<S, T>::value && PRE1);
+        constexpr int samples = PRE1 ? Straight<S>::kSamples : Straight<S>::kLongSamples;
+        flag = record_windows<NX, stop, samples>(
             P.B, x, xp, wc, w, lastT, n, advance, [&](float v) { return basins_diverged(v, P); },
             [&](int, const PeakWindow& d, float val, int t) {
                 if (d.n >= 1) PeakSums<float>::add_stored(w.sum, val, t - d.tprev);
