@@ -246,12 +246,14 @@ static int check_ff32_lle(const chaos_exec* ex, int system, const LleParams& L) 
 
 // precision / plug-in dispatch of the sweep kernels
 // The legacy per-point loop runs in FP64, the legacy library's arithmetic.
-static cudaError_t run_bif(int prec, const SweepParams& P, const BifOut& O, Call& c) {
-    cudaStream_t st = c.stream;
+// state: scratch of bif_state_bytes, or null.
+static size_t bif_state_bytes(int prec, const SweepParams& P) {
+    return prec == CHAOS_FP32 && !P.legacyLoop ? transient_state_bytes(P, false) : 0;
+}
+static cudaError_t run_bif(int prec, const SweepParams& P, const BifOut& O, float4* state, cudaStream_t st) {
     if (P.legacyLoop) prec = CHAOS_FP64;
     if (P.system == SYS_USER) return prec == CHAOS_FP32 ? cudaErrorNotSupported : launch_bif_user(P, O, st);
-    if (prec == CHAOS_FP32) return launch_bif_f32(P, O, st, (float4*)c.optional(transient_state_bytes(P, false)));
-    return launch_bif_f64(P, O, st);
+    return prec == CHAOS_FP32 ? launch_bif_f32(P, O, st, state) : launch_bif_f64(P, O, st);
 }
 static cudaError_t run_bif_list(int prec, const SweepParams& P, const BifOut& O, const int* list, int count,
                                 cudaStream_t st) {
@@ -545,7 +547,8 @@ static int bif1d_run(const chaos_exec* ex, SweepParams P, int gridMode, const do
     O.peaks = (double*)c.output(peaks, rowBytes);
     O.intervals = (double*)c.output(intervals, rowBytes);
     if (c.failed) return c.finish(CHAOS_E_NOMEM);
-    cudaError_t e = run_bif(c.ex.precision, P, O, c);
+    float4* state = (float4*)c.optional(bif_state_bytes(c.ex.precision, P));
+    cudaError_t e = run_bif(c.ex.precision, P, O, state, c.stream);
     if (e != cudaSuccess) return c.finish(cuda_error(e, "bifurcation kernel"));
     rc = c.to_host(counts, O.counts, n * sizeof(int));
     if (!rc) rc = c.to_host(flags, O.flags, n * sizeof(int));
@@ -578,7 +581,10 @@ static int bif2d_run(const chaos_exec* ex, SweepParams P, int gridMode, const do
     int cap = capFull;
     const int capKnob = g_bif2d_cap.load(std::memory_order_relaxed);
     const bool adapt = capKnob >= 0 && P.system != SYS_USER && n <= 0x7fffffffLL && capFull > 64;
-    const long long capBudget = (long long)(scratch_budget_bytes() / ((size_t)n * (sizeof(double) + 2 * sizeof(int))));
+    const size_t rowBytes = sizeof(double) + 2 * sizeof(int);
+    const size_t fixedBytes = c.ex.precision == CHAOS_FP32 ? sizeof(float4) : 0;  // a sliced transient's state
+    const size_t pointBudget = scratch_budget_bytes() / (size_t)n;
+    const long long capBudget = pointBudget > fixedBytes ? (long long)((pointBudget - fixedBytes) / rowBytes) : 0;
     if (adapt && capKnob > 0) {
         cap = std::min(capKnob, capFull);
     } else if (adapt && capBudget >= 512) {
@@ -600,7 +606,7 @@ static int bif2d_run(const chaos_exec* ex, SweepParams P, int gridMode, const do
         const int mx = std::max(0, *std::max_element(hc.begin(), hc.end()));
         cap = (int)std::min<long long>(capFull, (long long)mx + mx / 4 + 16);
     }
-    const size_t perPoint = (size_t)cap * (sizeof(double) + 2 * sizeof(int));
+    const size_t perPoint = cap * rowBytes + fixedBytes;
     long long chunk = (long long)std::max<size_t>(scratch_budget_bytes() / perPoint, 1);
     chunk = std::min(chunk, n);
     int* dLabels = (int*)c.output(labels, n * sizeof(int));
@@ -610,12 +616,18 @@ static int bif2d_run(const chaos_exec* ex, SweepParams P, int gridMode, const do
     int* dLab = (int*)c.alloc((size_t)chunk * cap * sizeof(int));
     int* dSlot = (int*)c.alloc((size_t)chunk * cap * sizeof(int));
     if (c.failed) return c.finish(CHAOS_E_NOMEM);
+    SweepParams Q = P;
+    size_t stateBytes = 0;  // one state for all chunks: they follow each other on the stream
+    for (long long m : {chunk, n % chunk}) {
+        Q.nPoints = m;
+        stateBytes = std::max(stateBytes, bif_state_bytes(c.ex.precision, Q));
+    }
+    float4* state = (float4*)c.optional(stateBytes);
     for (long long b = 0; b < n; b += chunk) {
-        SweepParams Q = P;
         Q.pBegin = b;
         Q.nPoints = std::min(chunk, n - b);
         BifOut O{dCounts + b, dFlags, nullptr, nullptr, dIv, cap};
-        cudaError_t e = run_bif(c.ex.precision, Q, O, c);
+        cudaError_t e = run_bif(c.ex.precision, Q, O, state, c.stream);
         if (e == cudaSuccess)
             e = launch_point_dbscan(dIv, dCounts + b, Q.nPoints, cap, eps, dLab, dSlot, dLabels + b, c.stream);
         if (e != cudaSuccess) return c.finish(cuda_error(e, "bifurcation 2-D kernels"));
