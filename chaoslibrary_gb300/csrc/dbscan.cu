@@ -879,7 +879,7 @@ struct Sorted {
 
 template <class Src>
 __global__ void sort_kernel(Src S, long long n, const int* slot, const int* slotCell, const int* begin, int* cursor,
-                            Sorted Q, const unsigned char* dense, const double* boxLo, int compat, const int* total) {
+                            Sorted Q, const unsigned char* dense, int compat, const int* total) {
     if (*total == 0) return;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
@@ -900,10 +900,7 @@ __global__ void sort_kernel(Src S, long long n, const int* slot, const int* slot
     S.load(i, v);
 #pragma unroll
     for (int d = 0; d < 3; ++d)
-        if (d < Q.D) {
-            Q.s[d][pos] = v[d];
-            Q.r[d][pos] = (float)(v[d] - boxLo[3 * (long long)c + d]);
-        }
+        if (d < Q.D) Q.s[d][pos] = v[d];
     Q.core[pos] = compat || dense[c] ? 1 : 0;
     if (Q.fix) Q.fix[pos] = S.fix(i) ? 1 : 0;
 }
@@ -1504,13 +1501,19 @@ __global__ void iota_kernel(int* p, long long n) {
 }
 
 // The nodes of the final union-find: the cells' components so far, then the
-// sorted points.
-__global__ void nodes_kernel(int C, const int* parentC, int* parent, int* compMin, int* compFix, const int* counts) {
-    const long long n = (long long)C + sorted_points(counts);
+// sorted points (and their offsets from their cells' boxes).
+__global__ void nodes_kernel(Sorted Q, Cells K, const int* parentC, int* parent, int* compMin, int* compFix,
+                             const int* counts) {
+    const long long n = (long long)K.C + sorted_points(counts);
     for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
-        parent[v] = v < C ? parentC[v] : (int)v;
+        parent[v] = v < K.C ? parentC[v] : (int)v;
         compMin[v] = INT_MAX;
         compFix[v] = INT_MAX;
+        if (v < K.C) continue;
+        const long long p = v - K.C, c = Q.cell[p];
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+            if (d < Q.D) Q.r[d][p] = (float)(Q.s[d][p] - K.lo[3 * c + d]);
     }
 }
 
@@ -1768,6 +1771,7 @@ struct Arena {
 // 10,000 points take 256 instead of 445 us, 1,000,000 505 instead of 690. Fout
 // (basin maps) receives the normalised features.
 constexpr long long kSmallSet = 65536;
+constexpr long long kRoomySet = 1 << 22;  // beyond it, 36 B of scratch a point are worth a wait
 
 template <class Src>
 int cell_cluster(Call& c, const Src& S, long long n, double eps, int minPts, bool compat, double bound, double* Fout,
@@ -1931,25 +1935,16 @@ int cell_cluster(Call& c, const Src& S, long long n, double eps, int minPts, boo
     Q.fix = compat ? A.take<unsigned char>(n1) : nullptr;
     for (int d = 0; d < 3; ++d) {
         Q.s[d] = d < D ? A.take<double>(n1) : nullptr;
-        Q.r[d] = d < D ? A.take<float>(n1) : nullptr;
+        Q.r[d] = nullptr;
     }
     Q.sb = K.sb;
     Q.se = K.se;
     Q.D = D;
-    // what the long scans find per sorted point (a count, later the best
-    // component's key), and their queue
-    unsigned long long* found = A.take<unsigned long long>(n1);
     ScanQueue W;
     W.cap = (int)std::min<long long>(std::max<long long>(4096, n), 1 << 20);
     W.point = A.take<int>(W.cap);
     W.cell = A.take<int>(W.cap);
     W.count = counts + kScanA;
-    // nodes: the cells, then the sorted points
-    const size_t N = (size_t)C + (size_t)n + 1;
-    int* parent = A.take<int>(N);
-    int* compMin = A.take<int>(N);
-    int* compFix = A.take<int>(N);
-    int* compLabel = A.take<int>(N);
     const long long words = (n + 31) / 32;
     unsigned* bits = A.take<unsigned>(2 * words);
     int* ranks = A.take<int>(2 * words);
@@ -1959,7 +1954,7 @@ int cell_cluster(Call& c, const Src& S, long long n, double eps, int minPts, boo
         if (r) return r;
         phase_begin_kernel<<<blocks(C), kTPB, 0, st>>>(C, cursor, take, before, begin, K.sb, K.se, K.cnt);
         note_launch();
-        sort_kernel<Src><<<blocks(n), kTPB, 0, st>>>(S, n, slot, slotCell, begin, cursor, Q, K.dense, K.lo,
+        sort_kernel<Src><<<blocks(n), kTPB, 0, st>>>(S, n, slot, slotCell, begin, cursor, Q, K.dense,
                                                      compat ? 1 : 0, total);
         note_launch();
         CKL();
@@ -1984,7 +1979,25 @@ int cell_cluster(Call& c, const Src& S, long long n, double eps, int minPts, boo
     take_needed_kernel<<<blocks(C), kTPB, 0, st>>>(K, take);
     note_launch();
     if ((rc = sort_phase(counts + kSparse, counts + kNeeded))) return rc;
-    nodes_kernel<<<loop, kTPB, 0, st>>>(C, parentC, parent, compMin, compFix, counts);
+    // what is kept per sorted point: its offsets, what the long scans find (a
+    // count, later the best component's key) and its nodes. By the points while
+    // there are few, otherwise by the number that was sorted, which takes a wait.
+    long long M = n;
+    if (n > kRoomySet) {
+        int hm[kNeeded + 1];
+        CK(cudaMemcpyAsync(hm, counts, sizeof hm, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        M = (long long)hm[kSparse] + hm[kNeeded];
+    }
+    const size_t M1 = (size_t)M + 1, N = (size_t)C + M1;  // nodes: the cells, then the sorted points
+    for (int d = 0; d < D; ++d) Q.r[d] = A.take<float>(M1);
+    unsigned long long* found = A.take<unsigned long long>(M1);
+    int* parent = A.take<int>(N);
+    int* compMin = A.take<int>(N);
+    int* compFix = A.take<int>(N);
+    int* compLabel = A.take<int>(N);
+    NEED(!c.failed);
+    nodes_kernel<<<loop, kTPB, 0, st>>>(Q, K, parentC, parent, compMin, compFix, counts);
     note_launch();
     if (!compat) {  // the undecided counts, exactly (their neighbours are sorted now)
         core_kernel<<<loop, kTPB, 0, st>>>(Q, K, nbStart, nbList, eps, minPts, 1, W, (int*)found, counts);
