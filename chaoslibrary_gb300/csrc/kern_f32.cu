@@ -107,14 +107,11 @@ int lle_env_variant() {
     return forced;
 }
 
-int lle_occupancy_variant(int system) {
-    (void)system;
+// 0: none is forced
+int lle_forced_variant() {
     const int set = g_lle_variant.load(std::memory_order_relaxed);
-    if (set) return set;
-    return lle_env_variant() ? lle_env_variant() : 2;
+    return set ? set : lle_env_variant();
 }
-
-bool lle_variant_forced() { return g_lle_variant.load(std::memory_order_relaxed) != 0 || lle_env_variant() != 0; }
 
 }  // namespace
 
@@ -178,11 +175,8 @@ Launch sweep_launch(const SweepParams& P, bool basins) {
     const bool big = P.nPoints >= pair_threshold();
     if (mode == 0) return {1, block};
     if (mode >= 2) return {2, block};
-    if (shape) {
-        const int form = shape / 1024;
-        return {big ? form : 1, block};
-    }
-    return {big ? 2 : 1, kBlock};
+    if (!big) return {1, kBlock};  // (the tuner times 8192 points per SM)
+    return {shape ? shape / 1024 : 2, block};
 }
 
 template <class F> void launch_bif_pairs(const SweepParams& P, const BifOut& O, int block, cudaStream_t st) {
@@ -320,7 +314,7 @@ int set_lle_variant(int v) {
     g_lle_variant.store(v);
     return 0;
 }
-int get_lle_variant() { return lle_occupancy_variant(0); }
+int get_lle_variant() { return lle_forced_variant(); }
 
 int set_lle_renorm(int v) {
     if (v < kRenormPow2 || v > kRenormF64) return -1;
@@ -330,18 +324,20 @@ int set_lle_renorm(int v) {
 int get_lle_renorm() { return g_lle_renorm.load(); }
 
 // an explicit variant (chaos_set_tuning / CHAOS_LLE_MINB) wins, then a tuned
-// shape; 0: neither
-static int lle_form(int system, int& block) {
+// shape, for maps of more rows than those that run in slices or in mixed blocks:
+// the tuner times 64 rows per SM; 0: neither
+static int lle_form(const LleParams& L, int& block) {
     block = kBlock;
-    if (lle_variant_forced()) return lle_occupancy_variant(system);
-    const int shape = shape_of(2, system);
+    if (const int forced = lle_forced_variant()) return forced;
+    if (L.nPoints <= kSliceLle.mostRows() * kBlock * sm_count()) return 0;
+    const int shape = shape_of(2, L.system);
     if (shape / 1024 == 2) block = shape % 1024;
     return shape / 1024;
 }
 
 size_t lle_f32_state_bytes(const LleParams& L) {
     int block;
-    if (!system_has_difference_form(L.system) || lle_form(L.system, block) != 0 || get_lle_renorm() != kRenormPow2)
+    if (!system_has_difference_form(L.system) || lle_form(L, block) != 0 || get_lle_renorm() != kRenormPow2)
         return 0;
     const SlicePlan plan = slice_plan(L, kSliceLle);
     return plan.words(plan.points == 2 ? LlePair<Lorenz>::kWords : LlePoint<Lorenz>::kWords) * sizeof(float);
@@ -350,7 +346,7 @@ size_t lle_f32_state_bytes(const LleParams& L) {
 cudaError_t launch_lle_f32(const LleParams& L, double* out, cudaStream_t st, float* state) {
     if (L.nPoints <= 0) return cudaSuccess;
     int block;
-    const int minb = lle_form(L.system, block);
+    const int minb = lle_form(L, block);
     switch (L.system) {
         case SYS_LORENZ_RK4: launch_twin<Lorenz>(L, out, st, minb, block, state); break;
         case SYS_ROSSLER_RK4: launch_twin<Rossler>(L, out, st, minb, block, state); break;

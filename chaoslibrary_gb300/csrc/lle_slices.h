@@ -20,6 +20,8 @@
 
 namespace chaos {
 
+constexpr int kRowsBeyond = 14;
+
 // What a map's time is made of, in units of what a further row costs the
 // kernel that runs it at once.
 struct SliceCost {
@@ -30,6 +32,7 @@ struct SliceCost {
     int blocks;         // Benettin blocks a slice has a multiple of
     double ns;          // the unit, for one transient step
     int residentRows;   // rows of pairs an SM holds
+    constexpr int mostRows() const { return residentRows + kRowsBeyond; }  // of a map that may run in slices
 };
 // From runs of 1 to 20 rows of the three RK4 systems. At once a row more takes
 // 0.287 ms (FP32 Lorenz, 5,500 steps), 0.334 (float-float Rossler, 1,510 steps),
@@ -41,7 +44,6 @@ constexpr SliceCost kSliceFF{0.08, 1.0, 0.08, 1.36, 1.1, 1, 208.0, 4};
 constexpr SliceCost kSliceSpectrum{0.33, 0.99, 0.29, 1.34, 4.0, kLleGroup, 31.8, 6};
 constexpr double kLaunchNs = 8000;  // a launch's start and end, about
 constexpr int kMaxSlices = 64;
-constexpr int kRowsBeyond = 14;
 
 // jobs == 0: the map runs in one launch. The horizon is counted in units of
 // unit transient steps or of the Benettin blocks that cost as much, so that the
@@ -56,7 +58,7 @@ struct SlicePlan {
 inline SlicePlan slice_plan(const LleParams& L, const SliceCost& k) {
     SlicePlan best{};
     const double rows = (double)L.nPoints / (double)(kSweepBlock * sm_count());
-    if (rows <= 1.0 || rows > k.residentRows + kRowsBeyond) return best;
+    if (rows <= 1.0 || rows > k.mostRows()) return best;
     const long long unit = (long long)(k.twin * L.ntp * k.blocks + 0.5);
     if (unit > 1000000) return best;
     const long long transient = (L.trans + unit - 1) / unit;

@@ -545,7 +545,9 @@ int chaos_trajectory(const chaos_exec* ex, int system, long long nTraj, const do
  * Kernel-shape knobs (no reference counterpart). CHAOS_TUNE_LLE_F32_VARIANT:
  * 2 = two grid points per thread in packed FP32x2 instructions, 12 / 16 = one
  * point per thread with registers shaped for 12 / 16 resident blocks per SM,
- * 0 = the library default. Process-wide; results do not depend on it.
+ * 0 = the library default, which picks by the size of the map.
+ * chaos_get_tuning gives the variant set here or in the environment
+ * (CHAOS_LLE_MINB), else 0. Process-wide; results do not depend on it.
  */
 #define CHAOS_TUNE_LLE_F32_VARIANT 1
 /* CHAOS_TUNE_SWEEP_PAIRS: FP32 bifurcation / basins sweeps of the RK4 systems
@@ -602,8 +604,10 @@ int chaos_get_tuning(int knob);
  * FP32 sweeps of the three RK4 systems -- one or two trajectories per thread,
  * the LLE map's register shapes, blocks of 64 / 128 / 256 threads -- on probe
  * sweeps that fill the GPU of ex (about 2-3 s in all), and installs the
- * fastest per (kind, system) for every later call in the process; a shape
- * replaces the built-in rule only when at least 1 % faster. Results do not
+ * fastest per (kind, system) for every later call in the process that is as
+ * large as the built-in rules' own large form (2048 points per SM; an LLE map
+ * of more than 2816); a shape replaces the built-in rule only when at least
+ * 1 % faster. Results do not
  * depend on shapes. An explicit CHAOS_TUNE_SWEEP_PAIRS (0 / 2 / 3) or
  * CHAOS_TUNE_LLE_F32_VARIANT still wins. table (may be NULL) receives nTable
  * rows (9 fill all) of 6 doubles: kind (0 1-D bifurcation, 1 basins, 2 LLE
