@@ -363,7 +363,11 @@ cudaError_t launch_lle_f32(const LleParams& L, double* out, cudaStream_t st, flo
 template <class F> static void launch_spectrum(const LleParams& L, double* out, cudaStream_t st, float* state) {
     const SlicePlan plan = state ? slice_plan(L, kSliceSpectrum) : SlicePlan{};
     if (plan.jobs > 0) return launch_slices(plan, spectrum_slice_kernel_f32<F>, L, out, state, st);
-    const unsigned singles = single_blocks(L.nPoints);
+    // up to three rows all of them single: their time goes with the rows, 2 rows of
+    // Lorenz points (2,510 steps) 0.626 ms, in pairs 0.647, 3 rows 0.914, one single
+    // and one of pairs 0.935 (Rossler 0.495 / 0.523 and 0.719 / 0.744)
+    const unsigned singles = L.nPoints <= kSliceSpectrum.singleRows * kBlock * sm_count()
+                                 ? grid_of(L.nPoints, kBlock) : single_blocks(L.nPoints);
     spectrum_pair_kernel_f32<F><<<mixed_grid(L.nPoints, singles), kBlock, 0, st>>>(L, out, singles);
     note_launch();
 }

@@ -32,16 +32,20 @@ struct SliceCost {
     int blocks;         // Benettin blocks a slice has a multiple of
     double ns;          // the unit, for one transient step
     int residentRows;   // rows of pairs an SM holds
+    int singleRows;     // up to so many rows a map at once runs one point per thread
     constexpr int mostRows() const { return residentRows + kRowsBeyond; }  // of a map that may run in slices
 };
 // From runs of 1 to 20 rows of the three RK4 systems. At once a row more takes
 // 0.287 ms (FP32 Lorenz, 5,500 steps), 0.334 (float-float Rossler, 1,510 steps),
 // 0.271 (spectrum, 2,510 steps); a slice kernel's row of FP32 costs more than the
-// 56-register kernel's. residentRows are those of the registers they take, and a
+// 56-register kernel's. Slices against one launch, each of the three systems in each
+// of the three kernels, 31 sizes from 1.05 to 20.1 rows: 0.71 to 0.99 of the time
+// where slices run, but for 1.00 and 1.01 (FP32 at 3.4 rows), 1.01 (spectrum of
+// Rossler at 11) -- Chen, whose kernels take other registers, 0.71 to 0.99. residentRows are those of the registers they take, and a
 // map of kRowsBeyond more has enough rows not to feel the last one.
-constexpr SliceCost kSliceLle{0.36, 1.06, 0.22, 1.48, 2.0, 1, 27.0, 8};
-constexpr SliceCost kSliceFF{0.08, 1.0, 0.08, 1.36, 1.1, 1, 208.0, 4};
-constexpr SliceCost kSliceSpectrum{0.33, 0.99, 0.29, 1.34, 4.0, kLleGroup, 31.8, 6};
+constexpr SliceCost kSliceLle{0.36, 1.06, 0.22, 1.48, 2.0, 1, 27.0, 8, 0};
+constexpr SliceCost kSliceFF{0.08, 1.0, 0.08, 1.36, 1.1, 1, 208.0, 4, 0};
+constexpr SliceCost kSliceSpectrum{0.33, 0.99, 0.29, 1.34, 4.0, kLleGroup, 31.8, 6, 3};
 constexpr double kLaunchNs = 8000;  // a launch's start and end, about
 constexpr int kMaxSlices = 64;
 
@@ -63,9 +67,10 @@ inline SlicePlan slice_plan(const LleParams& L, const SliceCost& k) {
     if (unit > 1000000) return best;
     const long long transient = (L.trans + unit - 1) / unit;
     const long long total = transient + ((long long)L.calcBlocks + k.blocks) / k.blocks;
-    // one launch: whole pair rows, or an odd number of rows up to kMixedRows (single_blocks)
+    // one launch: rows of single points, whole pair rows, or an odd number of rows (single_blocks)
     const double whole = std::ceil(rows), even = 2.0 * std::ceil(whole / 2.0) + k.once;
-    const double once = single_blocks(L.nPoints) ? std::min(even, whole + k.once + 0.16) : even;
+    const double once = whole <= k.singleRows ? whole + 0.27
+                        : single_blocks(L.nPoints) ? std::min(even, whole + k.once + 0.16) : even;
     // slices have to promise 3 %: what the model is off by
     double least = 0.97 * once * (double)total * (double)unit * k.ns;
     const int rowsMost = std::min((int)rows, k.residentRows);

@@ -34,11 +34,18 @@ inline long long sm_count() {
 // waited until they were done. FP32 Lorenz map, all single / all pairs / this
 // rule: one row 0.21 / 0.31 / 0.20 ms, three 0.50 / 0.56 / 0.46, five 0.80 /
 // 0.81 / 0.71, seven 1.10 / 1.06 / 0.96 (float-float 1.92 / 2.11 / 1.88), nine
-// 1.40 / 1.30 / 1.30.
+// 1.40 / 1.30 / 1.30. Not where the pairs behind the singles all but fill their
+// rows: then some SM gets one more of them than its share, and the map takes as
+// long as in pairs alone (three rows: 151 of 152 pair blocks 0.91 ms, spectrum of
+// Lorenz, 152 1.16; five: 292 of 304 1.45, 294 1.70; seven: 444 of 456 1.99, 446
+// 2.24; the LLE maps alike).
 constexpr long long kMixedRows = 7;
 inline unsigned single_blocks(long long n) {
     const long long row = kSweepBlock * sm_count(), rows = (n + row - 1) / row;
     if (rows % 2 == 0 || rows > kMixedRows) return 0;
+    const long long pairs = n > row ? grid_of((n - row + 1) / 2, kSweepBlock) : 0;
+    const long long spare = rows / 2 * sm_count() - pairs;
+    if (rows > 1 && spare < (rows == 3 ? 1 : sm_count() / 12)) return 0;
     return grid_of(std::min(n, row), kSweepBlock);
 }
 // Grid of such a kernel.
