@@ -241,18 +241,22 @@ cudaError_t launch_bif_list_f32(const SweepParams& P, const BifOut& O, const int
 // outside the step loop; the 1024^2 Rössler map went from 133.7 to 128.6 ms
 // (from 3.37 waves of resident blocks to 2.99) and the Lorenz map from 39.1
 // to 36.2 ms, results unchanged. Blocks of 64, 128 and 256 (the tuner's
-// choices) all launch under the bound. Chen's step keeps more and is the faster
-// for 128 registers: 4 rows of 128 points per SM (5,510 steps) 1.42 -> 1.38 ms, 60
-// rows 20.2 -> 19.9 (Lorenz at 128 1.23 -> 1.30).
-// singles: the first blocks, which run one point per thread (single_blocks),
-// with the default renormalisation only.
-template <class F, int RN = kRenormPow2>
-__global__ void __launch_bounds__(std::is_same<F, Chen>::value ? kMaxBlock : 384, std::is_same<F, Chen>::value ? 2 : 3)
+// choices) all launch under the bound.
+// Mixed: the first `singles` blocks run one point per thread (single_blocks).
+// Chen's step keeps more than Lorenz's and Rossler's: its mixed form takes 80
+// registers (three rows of 128 points per SM, 5,510 steps, 1.14 ms at 56, 1.11 at
+// 80), and where it has more than two rows and no singles it runs in a form of
+// pairs alone at 56 (mixed / pairs alone: 2 rows 0.741 / 0.747 ms, 4 rows 1.40 /
+// 1.37, 30 rows 9.99 / 9.60; the others' mixed form runs pairs as fast as one of
+// pairs alone, or faster).
+template <class F> constexpr bool is_chen() { return std::is_same<F, Chen>::value; }
+template <class F, int RN = kRenormPow2, bool Mixed = RN == kRenormPow2>
+__global__ void __launch_bounds__(is_chen<F>() && Mixed ? kMaxBlock : 384, is_chen<F>() && Mixed ? 2 : 3)
 lle_pair_kernel_f32(LleParams L, double* out, unsigned singles) {
     bool pair;
     const long long o = mixed_point(singles, pair);
     if (o >= L.nPoints) return;
-    if (RN == kRenormPow2 && !pair) {
+    if (Mixed && !pair) {
         out[o] = lle_point_twin<F>(L, L.pBegin + o);
         return;
     }
@@ -291,10 +295,11 @@ static void launch_twin(const LleParams& L, double* out, cudaStream_t st, int mi
     const unsigned gp = grid_of((L.nPoints + 1) / 2, minb == 2 ? block : kBlock);
     const int bp = minb == 2 ? block : kBlock;
     const unsigned singles = single_blocks(L.nPoints);
+    const bool mixed = minb == 0 && (!is_chen<F>() || singles || L.nPoints <= 2 * kBlock * sm_count());
     if (rn == kRenormF32Log) lle_pair_kernel_f32<F, kRenormF32Log><<<gp, bp, 0, st>>>(L, out, 0u);
     else if (rn == kRenormF64) lle_pair_kernel_f32<F, kRenormF64><<<gp, bp, 0, st>>>(L, out, 0u);
-    else if (minb == 0) lle_pair_kernel_f32<F><<<mixed_grid(L.nPoints, singles), kBlock, 0, st>>>(L, out, singles);
-    else if (minb == 2) lle_pair_kernel_f32<F><<<gp, bp, 0, st>>>(L, out, 0u);
+    else if (mixed) lle_pair_kernel_f32<F><<<mixed_grid(L.nPoints, singles), kBlock, 0, st>>>(L, out, singles);
+    else if (minb == 0 || minb == 2) lle_pair_kernel_f32<F, kRenormPow2, !is_chen<F>()><<<gp, bp, 0, st>>>(L, out, 0u);
     else if (minb >= 16) lle_twin_kernel_f32<F, 16><<<grid_for(L.nPoints), kBlock, 0, st>>>(L, out);
     else lle_twin_kernel_f32<F, 12><<<grid_for(L.nPoints), kBlock, 0, st>>>(L, out);
     note_launch();
