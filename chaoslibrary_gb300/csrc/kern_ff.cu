@@ -253,11 +253,14 @@ __global__ void __launch_bounds__(kBlock) trajectory_kernel_ff(const double* x0,
 // Persistent kernel of a batch's float-float LLE jobs of one system
 // (CHAOS_JOB_LLE2D_FF32): pulls chunks of two blocks' worth of points from
 // its counter; every point runs FFPair, as in the single-sweep kernel, with the
-// job's parameters staged in shared memory. Asked for two blocks per SM like
-// that kernel: a 600^2 Rossler map (6,010 steps) 26.9 -> 26.6 ms, maps
-// of 500^2, 400^2 and 500^2 points 50.5 -> 50.1.
+// job's parameters staged in shared memory. The compiler takes 126 registers,
+// four blocks per SM, and not more are asked for: the chunks of a batch of small
+// maps wait for a free block where fewer are resident. 3,010 steps, with this /
+// with up to 168 registers / up to 255: 600^2 Rossler points 13.25 / 13.14 /
+// 13.11 ms, 12 maps of 244^2 27.74 / 27.78 / 27.55, maps of 200^2, 300^2, 100^2
+// and 50^2 5.75 / 5.88 / 6.75, 99 of 54^2 11.8 / 11.8 / 13.0.
 template <class F>
-__global__ void __launch_bounds__(kBlock, 2) group_ff_kernel(const JobDesc* __restrict__ jobs,
+__global__ void __launch_bounds__(kBlock) group_ff_kernel(const JobDesc* __restrict__ jobs,
                                                           const Chunk* __restrict__ chunks, int count, int* counter) {
     __shared__ int slot;
     __shared__ LleParams sL;
