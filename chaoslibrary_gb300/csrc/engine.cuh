@@ -1659,10 +1659,19 @@ __device__ __forceinline__ void trajectory_point(const double* x0, const double*
     double* o = out + t * (long long)(nSteps + 1) * NX;
 #pragma unroll
     for (int j = 0; j < NX; ++j) o[j] = (double)x[j];
-    for (int s = 1; s <= nSteps; ++s) {
+    auto record = [&](int s) {
         step<S>(x, a, c);
 #pragma unroll
         for (int j = 0; j < NX; ++j) o[(long long)s * NX + j] = (double)x[j];
+    };
+    if constexpr (std::is_same<T, float>::value && S <= SYS_CHEN_RK4) {
+        // one step at a time: several in a row are scheduled for a longer chain (64
+        // trajectories, 4,000 steps: Lorenz 0.73 -> 0.64 ms, Rossler 0.69 -> 0.63, Chen
+        // 0.72 -> 0.63)
+#pragma unroll 1
+        for (int s = 1; s <= nSteps; ++s) record(s);
+    } else {
+        for (int s = 1; s <= nSteps; ++s) record(s);
     }
 }
 
