@@ -35,9 +35,14 @@ template <> struct FieldOf<SYS_CHEN_RK4> { using F = Chen; };
 // the group's range from its counter until none is left. One kernel per
 // group keeps each code path's register allocation as small as the
 // single-sweep kernel's (a kernel that switched over every kind and system
-// would be sized for the largest of them).
+// would be sized for the largest of them). The RK4 systems' take at most what
+// leaves room for five blocks per SM: the bifurcation pairs of Lorenz and Chen
+// take 106 and 108 registers unasked, and four blocks of those leave no room for
+// one of another group. Nine jobs of 60,000 to 600 points 6.04 -> 5.14 ms, six of
+// 100,000 to 1,000 5.27 -> 4.66, twelve of 70,000 to 700 7.29 -> 7.02, fifteen of
+// 100,000 to 1,000 9.95 -> 10.02.
 template <template <int> class Work, int S>
-__global__ void __launch_bounds__(kBatchBlock) group_kernel(const JobDesc* __restrict__ jobs,
+__global__ void __launch_bounds__(kBatchBlock, S <= SYS_CHEN_RK4 ? 5 : 0) group_kernel(const JobDesc* __restrict__ jobs,
                                                             const Chunk* __restrict__ chunks, int count,
                                                             int* counter) {
     __shared__ int slot;
