@@ -211,10 +211,11 @@ __device__ __forceinline__ void box_dist2(const double* v, const double* lo, con
 
 // ---- counts the pipeline keeps on the device ---------------------------------------
 // The sizes of the later steps stay in device memory: their kernels read them
-// (a fixed grid loops over the work), and the host waits once, for the number
-// of cells.
+// (a fixed grid loops over the work). The host waits for the number of cells,
+// and in large sets for a bound on it, for the neighbour entries and for the
+// sorted points (cell_cluster).
 enum Count {
-    kCells, kErr, kEntries, kOpen, kJoinedCount, kSparse, kNeeded, kRoots, kActive, kLong, kScanA, kScanB, kCounts
+    kCells, kErr, kEntries, kOpen, kJoinedCount, kSparse, kNeeded, kActive, kLong, kScanA, kScanB, kCounts
 };
 constexpr int kLoopBlocksPerSm = 8;  // blocks of kTPB threads of a looping kernel
 
@@ -472,7 +473,8 @@ __device__ __forceinline__ long long table_slot(unsigned long long* tab, unsigne
 // lane finds (or claims) the cell's entry, adds the group's count and keeps
 // its smallest and largest index; a lane whose point lies outside the box it
 // reads widens it. A group that finds no room goes to the cell table itself.
-// Bound by the read of the points. Folding every run of equal cells straight
+// Bound by the FP64 pipe, which takes the points to their cells (81 % busy; 8
+// million points in 3-D 0.31 ms, 0.68 TB/s). Folding every run of equal cells straight
 // into the cell table, with an atomic per quantity, spent its time on the
 // addresses of the few cells that hold most points: 1,000,000 points in
 // random order 480 -> 55 us, a 2048^2 basin map 284 -> 273 us; reading a cell's
@@ -1314,8 +1316,9 @@ __constant__ int kPassChunks[kCrossPasses] = {2, 8, 0x7fffffff};
 
 constexpr long long kLongPair = 1 << 16;  // point pairs of two cells that one warp takes on in the last pass
 
-__device__ __forceinline__ void cross_cells(Sorted Q, Cells K, const int* nbOwner, const int* nbList,                                   double eps, int* parent, int pass, unsigned char* deferred,
-                                  int* longPairs, int* nLong, long long w) {
+__device__ __forceinline__ void cross_cells(Sorted Q, Cells K, const int* nbOwner, const int* nbList, double eps,
+                                            int* parent, int pass, unsigned char* deferred, int* longPairs, int* nLong,
+                                            long long w) {
     const int lane = threadIdx.x & 31;
     int ca = nbOwner[w], cb = nbList[w];
     if (!sorted_cell(Q, ca) || !sorted_cell(Q, cb)) return;
@@ -1410,8 +1413,9 @@ __device__ __forceinline__ void cross_cells(Sorted Q, Cells K, const int* nbOwne
     if (cut && lane == 0) deferred[w] = 1;
 }
 
-__global__ void cross_cell_kernel(Sorted Q, Cells K, const int* nbOwner, const int* nbList,                                   double eps, int* parent, int pass, unsigned char* deferred,
-                                  int* longPairs, int* nLong, const int* active, const int* counts) {
+__global__ void cross_cell_kernel(Sorted Q, Cells K, const int* nbOwner, const int* nbList, double eps, int* parent,
+                                  int pass, unsigned char* deferred, int* longPairs, int* nLong, const int* active,
+                                  const int* counts) {
     const int n = counts[kActive];
     for (long long k = first_warp(); k < n; k += warp_stride())
         cross_cells(Q, K, nbOwner, nbList, eps, parent, pass, deferred, longPairs, nLong, active[k]);
@@ -1767,9 +1771,12 @@ struct Arena {
 // a small set's table is sized by its points (measuring their extent takes a
 // pass and a wait, more than the larger table costs), a large one's by the
 // extent of its cells. Every wait for a count costs the host's round trip and
-// an idle GPU: with one left of seven, and the scratch in few allocations,
-// 10,000 points take 256 instead of 445 us, 1,000,000 505 instead of 690. Fout
-// (basin maps) receives the normalised features.
+// an idle GPU. Of seven, small sets keep one (the cells), sets above kSmallSet
+// one more (the extent; a basin map brings its bound), more than 8,456 cells in
+// 3-D (43,690 in 2-D) one more (their neighbour entries) and sets above
+// kRoomySet one more (the sorted points): with that, and the scratch in few
+// allocations, 10,000 points take 256 instead of 445 us, 1,000,000 505 instead of
+// 690. Fout (basin maps) receives the normalised features.
 constexpr long long kSmallSet = 65536;
 constexpr long long kRoomySet = 1 << 22;  // beyond it, 36 B of scratch a point are worth a wait
 

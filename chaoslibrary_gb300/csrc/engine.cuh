@@ -4,10 +4,13 @@
 // and the FP32 kernel translation units, which instantiate the templates for
 // their arithmetic type.
 //
-// Layout rule for every kernel here: one CUDA thread owns one trajectory; its
-// full state, its parameters and its peak detector live in registers; the
-// trajectory itself never reaches HBM. What a point writes to HBM is its
-// result row (a few scalars, plus its peak list for the bifurcation sweeps).
+// Layout rule for every kernel here: one CUDA thread owns one trajectory (two in
+// the packed FP32 forms; in small FP64 sweeps three lanes share one, team.cuh).
+// State and parameters live in registers, with the FP64 peak detector; the FP32
+// sweeps keep a window of samples and their detectors in shared memory. The
+// trajectory itself never reaches HBM, but for the state of points whose
+// horizon runs in slices. What a point writes to HBM is its result row (a few
+// scalars, plus its peak list for the bifurcation sweeps).
 #pragma once
 
 #include <cuda_runtime.h>

@@ -120,12 +120,14 @@ std::atomic<int> g_sweep_pairs{-1};
 // Paired (two points per thread, packed FP32x2 lanes) FP32 sweeps for the RK4
 // systems. Mode 1 (default): sweeps of at least 2048 points per SM run as
 // pairs, smaller ones one point per thread: pairs issue half the instructions
-// but halve the warps that hide each other's latency. Measured on GB300, one
-// point per thread against pairs: 1-D Rossler, 20,000 steps, 240,000 points
-// 7.38 / 7.42 ms, 320,000 9.56 / 9.40 ms, 700,001 20.0 / 18.1 ms; Lorenz
-// basins, 25,000 steps, 500^2 9.09 / 9.18 ms, 600^2 13.2 / 12.9 ms, 1024^2
-// 35.4 / 33.9 ms. 2 (or 3): always pairs; 0: never. Set with
-// chaos_set_tuning or CHAOS_SWEEP_PAIRS.
+// but halve the warps that hide each other's latency, and up to those 16 rows
+// of 128 the transient of single points runs in slices. Measured on GB300, one
+// point per thread against pairs: 1-D Rossler, 20,000 steps, 160,000 points
+// 4.97 / 5.16 ms, 240,000 7.24 / 7.10, 320,000 9.41 / 9.06, 700,001 19.7 / 17.8;
+// Lorenz basins, 25,000 steps, 400^2 5.73 / 5.95 ms, 500^2 8.48 / 8.23, 600^2
+// 12.3 / 11.7, 1024^2 34.6 / 31.2 (so full maps of 1,400 to 2,048 points per SM
+// would be up to 10 % faster in pairs). 2 (or 3): always pairs; 0: never. Set
+// with chaos_set_tuning or CHAOS_SWEEP_PAIRS.
 int sweep_pairs() {
     const int v = g_sweep_pairs.load(std::memory_order_relaxed);
     if (v >= 0) return v;
@@ -154,15 +156,7 @@ int shape_of(int kind, int system) {
     return system >= 0 && system <= SYS_CHEN_RK4 ? g_shape[kind][system].load(std::memory_order_relaxed) : 0;
 }
 
-long long pair_threshold() {
-    static long long threshold = [] {
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        return 2048LL * std::max(sms, 1);
-    }();
-    return threshold;
-}
+long long pair_threshold() { return 2048 * sm_count(); }
 
 // Pairs halve the threads: worth it when the sweep fills the GPU several
 // times over, not for small (latency-bound) sweeps. An explicit sweep-pairs

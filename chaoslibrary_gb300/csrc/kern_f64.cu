@@ -9,6 +9,7 @@
 
 #include "engine.cuh"
 #include "legacy_lle.cuh"
+#include "sweep_launch.h"
 #include "team.cuh"
 
 namespace chaos {
@@ -201,19 +202,6 @@ __global__ void __launch_bounds__(kBlock) trajectory_kernel(const double* x0, co
 inline unsigned grid_for(long long n) { return (unsigned)((n + kBlock - 1) / kBlock); }
 inline unsigned warps_for(long long n) { return (unsigned)((n + kSweep - 1) / kSweep); }
 
-#define CHAOS_SYSTEM_SWITCH(sys, CALL) \
-    switch (sys) {                     \
-        case SYS_LORENZ_RK4: CALL(SYS_LORENZ_RK4); break; \
-        case SYS_ROSSLER_RK4: CALL(SYS_ROSSLER_RK4); break; \
-        case SYS_CHEN_RK4: CALL(SYS_CHEN_RK4); break; \
-        case SYS_CHAMELEON: CALL(SYS_CHAMELEON); break; \
-        case SYS_ROSSLER_CD: CALL(SYS_ROSSLER_CD); break; \
-        case SYS_SIN3: CALL(SYS_SIN3); break; \
-        case SYS_SIN2: CALL(SYS_SIN2); break; \
-        case SYS_MEMRISTOR: CALL(SYS_MEMRISTOR); break; \
-        default: return cudaErrorInvalidValue; \
-    }
-
 // Peak finder over caller series (the reference's peakFinderCUDA semantics on
 // identical input arrays): one thread streams one series.
 __global__ void peak_array_kernel(const double* __restrict__ data, long long nSeries, int len, double h, int cap,
@@ -255,10 +243,10 @@ __global__ void peak_array_kernel(const double* __restrict__ data, long long nSe
 // is skipped too, as entry 0 was expanded first and the unlabelled entries
 // only get fewer. The distances go by a float copy of the row in shared memory
 // unless the error bound of the float difference leaves the limit open: with
-// an FP64 subtraction and conversion per pair the FP64 pipe was 84 % busy.
-// 300^2 points of the Chameleon with 60 intervals each: 2.40 ms with labels
-// and slots in scratch, 0.98 ms with the bits, 0.32 ms with the float copy
-// (issue slots 82 % busy).
+// an FP64 subtraction and conversion per pair the FP64 pipe bounded it. 300^2
+// points of the Chameleon with 60 intervals each: 2.40 ms with labels and slots
+// in scratch, 0.98 ms with the bits, 0.32 ms with the float copy; then issue
+// slots bound it (89 % busy, 90,000 rows of 60 intervals 0.14 to 0.33 ms).
 constexpr int kDbscanBits = 1024;
 
 // distance < eps of two intervals: the distance is 0 for equal ones (also
@@ -420,15 +408,7 @@ int launch_block_size() { return kBlock; }
 // 40^2 7.12 / 4.24 ms, 100^2 7.12 / 6.10, 110^2 (80 per SM) 7.12 / 6.95, 116^2
 // 7.12 / 8.23; orbit and twin in a team each 40^2 2.62 ms, 77^2 (39 per SM)
 // 4.33 against 4.41 in one team, 90^2 5.95 against 5.32.
-long long sm_points(long long perSm) {
-    static long long sms = [] {
-        int dev = 0, n = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        return (long long)(n > 1 ? n : 1);
-    }();
-    return perSm * sms;
-}
+long long sm_points(long long perSm) { return perSm * sm_count(); }
 bool team_sweep(long long n) {
     return n <= sm_points(120) || (n > sm_points(128) && n <= sm_points(160));
 }

@@ -57,6 +57,10 @@ CHAOS_HD DiffTest diff_test(float v, float p1) {
 //
 // One subtraction per sample (diff_test): the next sample's rise test
 // "d[k] - d[k-1] > 1e-13" is taken when d[k] arrives and kept as a flag.
+//
+// The FP64 kernels run the branching double form. The float forms (Gate, and
+// the selects of Sel) have no kernel: the FP32 loops judge windows (PeakWindow),
+// which the host tests check against them.
 template <class T, bool Sel = false> struct PeakStream {
     // Gate (float, branching form): the common sample -- no plateau open and
     // no candidate to judge -- costs one subtraction, one compare against a

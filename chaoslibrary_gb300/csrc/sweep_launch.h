@@ -15,6 +15,7 @@ constexpr int kMaxBlock = 256;    // largest block a tuned launch may use
 
 inline unsigned grid_of(long long threads, int block) { return (unsigned)((threads + block - 1) / block); }
 
+// SMs of the process's first device.
 inline long long sm_count() {
     static const long long sms = [] {
         int dev = 0, n = 0;
